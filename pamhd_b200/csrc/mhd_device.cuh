@@ -34,15 +34,25 @@ namespace pamhd_b200 {
 constexpr double DBL_EPS = 2.220446049250313080847e-16;  // numeric_limits<double>::epsilon()
 constexpr double DBL_MIN_NORMAL = 2.2250738585072013831e-308;
 
+/*
+Checks on the high word (sign, exponent, top of the mantissa): one or two
+integer instructions, where comparisons of doubles would take the FP64
+pipe that bounds these kernels.
+*/
 __device__ __forceinline__ bool is_normal(const double x)
 {
-	const double a = fabs(x);
-	return a >= DBL_MIN_NORMAL and a <= 1.7976931348623157e308;
+	return ((unsigned int)__double2hiint(x) & 0x7fffffffu) - 0x00100000u < 0x7fe00000u;
+}
+
+// x > 0 and normal
+__device__ __forceinline__ bool is_positive_normal(const double x)
+{
+	return (unsigned int)__double2hiint(x) - 0x00100000u < 0x7fe00000u;
 }
 
 __device__ __forceinline__ bool is_finite(const double x)
 {
-	return fabs(x) <= 1.7976931348623157e308;
+	return ((unsigned int)__double2hiint(x) & 0x7fffffffu) < 0x7ff00000u;
 }
 
 // physical constants of one run
@@ -63,60 +73,72 @@ reference would raise for any face touching this cell, in its order of
 checks: density, then pressure, then wave speed.
 */
 struct Derived {
-	double rinv, vx, vy, vz, p, cf[3];
+	double rinv, vx, vy, vz, p, pt, cf[3];  // pt: thermal plus magnetic pressure
 	uint32_t bad;
 };
 
 /*
-Reciprocal of a non-zero normal double by Newton-Raphson iteration
-(r <- r + r (1 - x r), quadratic convergence) from the hardware estimate of
-PTX rcp.approx.ftz.f64; two iterations bring the estimate's relative error
-below 2^-52, so the result is within one unit in the last place of 1/x.
+Reciprocal of a non-zero normal double: one third-order step of the
+Householder family for f(r) = 1/r - x, r <- r (1 + e + e^2) with
+e = 1 - x r, from the hardware estimate of PTX rcp.approx.ftz.f64.  The
+step cubes the estimate's relative error (at most 2^-19.9, measured over
+2^26 mantissas), so the result is within one unit in the last place of
+1/x, with three dependent operations where two Newton steps take four.
 Used where the operand is a normal, non-zero number by construction.
 */
 __device__ __forceinline__ double recip(const double x)
 {
 	double r;
 	asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(x));
-	double e = __fma_rn(-x, r, 1.0);
-	r = __fma_rn(r, e, r);
-	e = __fma_rn(-x, r, 1.0);
-	return __fma_rn(r, e, r);
+	const double e = __fma_rn(-x, r, 1.0);
+	return __fma_rn(r, __fma_rn(e, e, e), r);
 }
 
 /*
-Reciprocal square root of a positive normal double: Newton-Raphson
-iteration for f(r) = 1/r^2 - x, r <- r + (r/2)(1 - x r^2) (quadratic
-convergence), from the hardware estimate of PTX rsqrt.approx.ftz.f64; two
-iterations.  sqrt(x) is then x * rsqrt(x), within a few units in the last
-place, which the 1e-12 parity bar leaves ample room for.
+One third-order step for f(r) = 1/r^2 - x from an estimate r:
+r <- r (1 + e/2 + 3 e^2 / 8) with e = 1 - x r^2.
+*/
+__device__ __forceinline__ double rsqrt_step(const double x, const double r)
+{
+	const double e = __fma_rn(__dmul_rn(-x, r), r, 1.0);
+	return __fma_rn(__dmul_rn(r, e), __fma_rn(0.375, e, 0.5), r);
+}
+
+/*
+Reciprocal square root of a positive normal double, from the hardware
+estimate of PTX rsqrt.approx.ftz.f64.
 */
 __device__ __forceinline__ double rsqrt_nr(const double x)
 {
 	double r;
 	asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(x));
-	double e = __fma_rn(__dmul_rn(-x, r), r, 1.0);
-	r = __fma_rn(__dmul_rn(0.5, r), e, r);
-	e = __fma_rn(__dmul_rn(-x, r), r, 1.0);
-	return __fma_rn(__dmul_rn(0.5, r), e, r);
+	return rsqrt_step(x, r);
 }
 
 /*
-Square root of a non-negative double as x * rsqrt_nr(x) (0, +inf and NaN
-pass through as themselves).
+Square root of a non-negative finite double as x rsqrt(x): the estimate is
+taken of x raised to the smallest normal number (an integer maximum of the
+high word), so that 0 gives 0.
 */
 __device__ __forceinline__ double sqrt_nr(const double x)
 {
-	return (x > 0.0 and x <= 1.7976931348623157e308) ? __dmul_rn(x, rsqrt_nr(x)) : x;
+	const double c = __hiloint2double(max(__double2hiint(x), 0x00100000), __double2loint(x));
+	double r;
+	asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(c));
+	return __dmul_rn(x, rsqrt_step(x, r));
 }
-
 
 /*
 Every operation below is an explicitly rounded intrinsic, so that every
 inlined copy of this function computes the same bits for the same cell
 (the halo of one tile is the interior of the next).
+
+The fast speed: c_f^2 = (a^2 + v_A^2 + root) / 2 with
+root^2 = (a^2 + v_A^2)^2 - 4 a^2 v_A,n^2, written as
+(a^2 - v_A^2)^2 + 4 a^2 v_A,t^2 (v_A,t from the field across the axis):
+no division by B^2 and no cancellation.
 */
-template <bool NEED_X, bool NEED_Y, bool NEED_Z, bool NR_SQRT = false>
+template <bool NEED_X, bool NEED_Y, bool NEED_Z>
 __device__ __forceinline__ Derived derive(
 	const double rho, const double mx, const double my, const double mz,
 	const double E, const double bx, const double by, const double bz, const Gas& g
@@ -126,53 +148,54 @@ __device__ __forceinline__ Derived derive(
 	d.vx = __dmul_rn(mx, d.rinv);
 	d.vy = __dmul_rn(my, d.rinv);
 	d.vz = __dmul_rn(mz, d.rinv);
-	const double b2 = __fma_rn(bz, bz, __fma_rn(by, by, __dmul_rn(bx, bx)));
+	const double bb[3] = {__dmul_rn(bx, bx), __dmul_rn(by, by), __dmul_rn(bz, bz)};
+	const double b2 = __dadd_rn(__dadd_rn(bb[0], bb[1]), bb[2]);
 	const double m2 = __fma_rn(mz, mz, __fma_rn(my, my, __dmul_rn(mx, mx)));
 	const double kinetic = __dmul_rn(__dmul_rn(0.5, d.rinv), m2);
 	const double magnetic = __dmul_rn(__dmul_rn(0.5, g.inv_mu0), b2);
 	d.p = __dmul_rn(__dsub_rn(__dsub_rn(E, kinetic), magnetic), g.gamma - 1.0);
+	d.pt = __dadd_rn(d.p, magnetic);
 	d.bad = 0;
-	if (not (rho > 0.0 and is_normal(rho))) {
+	if (not is_positive_normal(rho)) {
 		d.bad = PAMHD_FLAG_DENSITY;
-	} else if (not (d.p > 0.0 and is_normal(d.p))) {
+	} else if (not is_positive_normal(d.p)) {
 		d.bad = PAMHD_FLAG_PRESSURE;
 	}
 	const double cs2 = __dmul_rn(__dmul_rn(g.gamma, d.p), d.rinv);
+	const bool need[3] = {NEED_X, NEED_Y, NEED_Z};
 	if (b2 > 0.0) {
-		const double va2 = __dmul_rn(__dmul_rn(b2, g.inv_mu0), d.rinv);
-		const double sum2 = __dadd_rn(cs2, va2);
-		const double inv_b2 = recip(b2);
-		const double prod = __dmul_rn(__dmul_rn(2.0, cs2), va2);
-		const double base = __fma_rn(va2, va2, __dmul_rn(cs2, cs2));
-		const double comp[3] = {bx, by, bz};
-		const bool need[3] = {NEED_X, NEED_Y, NEED_Z};
-		bool wave_ok = is_normal(sum2) and is_finite(b2);
+		const double im = __dmul_rn(g.inv_mu0, d.rinv);
+		const double va2 = __dmul_rn(b2, im);
+		const double sum2 = __dadd_rn(cs2, va2), diff2 = __dsub_rn(cs2, va2);
+		const double base = __dmul_rn(diff2, diff2);
+		const double cross = __dmul_rn(__dmul_rn(4.0, cs2), im);
+		bool wave_ok = is_positive_normal(sum2) and is_finite(b2);
 		#pragma unroll
 		for (int a = 0; a < 3; a++) {
 			if (not need[a]) {
 				d.cf[a] = 0.0;
 				continue;
 			}
-			const double cos2 = __dmul_rn(__dmul_rn(comp[a], comp[a]), inv_b2);
-			const double to_sqrt = __fma_rn(prod, __fma_rn(-2.0, cos2, 1.0), base);
-			wave_ok = wave_ok and to_sqrt > 0.0 and is_normal(to_sqrt);
-			d.cf[a] = NR_SQRT
-				? sqrt_nr(__dmul_rn(0.5, __dadd_rn(sum2, sqrt_nr(fmax(to_sqrt, 0.0)))))
-				: __dsqrt_rn(__dmul_rn(0.5, __dadd_rn(sum2, __dsqrt_rn(fmax(to_sqrt, 0.0)))));
+			const double to_sqrt = __fma_rn(cross, __dadd_rn(bb[(a + 1) % 3], bb[(a + 2) % 3]), base);
+			wave_ok = wave_ok and is_positive_normal(to_sqrt);
+			d.cf[a] = sqrt_nr(__dmul_rn(0.5, __dadd_rn(sum2, sqrt_nr(to_sqrt))));
 		}
 		if (d.bad == 0 and not wave_ok) d.bad = PAMHD_FLAG_WAVE_SPEED;
 	} else {
-		const double cs = NR_SQRT ? sqrt_nr(fmax(cs2, 0.0)) : __dsqrt_rn(fmax(cs2, 0.0));
-		d.cf[0] = d.cf[1] = d.cf[2] = cs;
+		d.cf[0] = d.cf[1] = d.cf[2] = sqrt_nr(cs2);
 		if (d.bad == 0 and not is_finite(b2)) d.bad = PAMHD_FLAG_WAVE_SPEED;
 	}
+	// a refused cell: no face of it counts, its speeds stay numbers
+	if (d.bad != 0) d.cf[0] = d.cf[1] = d.cf[2] = 0.0;
 	return d;
 }
 
 // one cell seen from a face, rotated into the face frame
 struct Side {
 	double rho, m0, m1, m2, E, b0, b1, b2;
-	double rinv, v0, v1, v2, p, cf;
+	double rinv, v0, v1, v2, cf;
+	double pt;   // thermal plus magnetic pressure
+	double p;    // thermal pressure, for the fluxes with a background field only
 	uint32_t bad;
 };
 
@@ -210,6 +233,7 @@ __device__ __forceinline__ Side side_of(const double U[8], const Derived& d)
 	s.E = U[4];
 	rotate<A>(U[5], U[6], U[7], s.b0, s.b1, s.b2);
 	s.rinv = d.rinv;
+	s.pt = d.pt;
 	s.p = d.p;
 	s.cf = d.cf[A];
 	s.v0 = s.m0 * s.rinv;
@@ -220,55 +244,39 @@ __device__ __forceinline__ Side side_of(const double U[8], const Derived& d)
 }
 
 /*
-Arithmetic of the face solvers (Rusanov, HLL, HLLD).  Ar<false>: plain expressions, as written
-(the files built with -fmad=false round every operation on its own).
-Ar<true>: every operation an explicitly rounded intrinsic, a fused
-multiply-add where the formula has a product added, so that every kernel
-of the cell-centred step (single grid, batched, persistent) computes the
-same bits for the same face, whatever other code it is inlined beside.
-In both, fma(a, b, c) is a b + c and x - y z is written fma(-y, z, x),
-which negates exactly, so Ar<false> keeps the written operation order.
+Arithmetic of the face solvers (Rusanov, HLL, HLLD): every operation an
+explicitly rounded intrinsic, a fused multiply-add where the formula has a
+product added, so that every kernel computes the same bits for the same
+face, whatever other code it is inlined beside and whichever flags its
+file is compiled with.
 */
-template <bool X> struct Ar {
-	static __device__ __forceinline__ double mul(const double a, const double b) { return X ? __dmul_rn(a, b) : a * b; }
-	static __device__ __forceinline__ double add(const double a, const double b) { return X ? __dadd_rn(a, b) : a + b; }
-	static __device__ __forceinline__ double sub(const double a, const double b) { return X ? __dsub_rn(a, b) : a - b; }
+struct Ar {
+	static __device__ __forceinline__ double mul(const double a, const double b) { return __dmul_rn(a, b); }
+	static __device__ __forceinline__ double add(const double a, const double b) { return __dadd_rn(a, b); }
+	static __device__ __forceinline__ double sub(const double a, const double b) { return __dsub_rn(a, b); }
 	static __device__ __forceinline__ double fma(const double a, const double b, const double c)
 	{
-		return X ? __fma_rn(a, b, c) : a * b + c;
+		return __fma_rn(a, b, c);
 	}
 };
 
 /*
 Ideal-MHD flux along the face normal, mhd/common.hpp:146-244, with the
-background field zero (every configuration of the fused step).  pb is the
-magnetic pressure B^2 / (2 mu0).
+background field zero (every configuration of the fused step).
 */
-template <bool X = false>
-__device__ __forceinline__ void physical_flux(const Side& s, const double pb, const Gas& g, double F[8])
+__device__ __forceinline__ void physical_flux(const Side& s, const Gas& g, double F[8])
 {
-	if constexpr (X) {
-		using A = Ar<true>;
-		F[0] = s.m0;
-		F[1] = A::add(A::fma(s.m0, s.v0, -A::mul(g.inv_mu0, A::mul(s.b0, s.b0))), A::add(s.p, pb));
-		F[2] = A::fma(s.m1, s.v0, -A::mul(g.inv_mu0, A::mul(s.b0, s.b1)));
-		F[3] = A::fma(s.m2, s.v0, -A::mul(g.inv_mu0, A::mul(s.b0, s.b2)));
-		const double vb = A::fma(s.v2, s.b2, A::fma(s.v1, s.b1, A::mul(s.v0, s.b0)));
-		F[4] = A::fma(s.v0, A::add(A::add(s.E, s.p), pb), -A::mul(A::mul(s.b0, vb), g.inv_mu0));
-		F[5] = 0.0;
-		F[6] = A::fma(s.v0, s.b1, -A::mul(s.b0, s.v1));
-		F[7] = A::fma(s.v0, s.b2, -A::mul(s.b0, s.v2));
-		return;
-	}
+	using A = Ar;
+	const double b0m = A::mul(s.b0, g.inv_mu0);
 	F[0] = s.m0;
-	F[1] = s.m0 * s.v0 - g.inv_mu0 * (s.b0 * s.b0) + (s.p + pb);
-	F[2] = s.m1 * s.v0 - g.inv_mu0 * (s.b0 * s.b1);
-	F[3] = s.m2 * s.v0 - g.inv_mu0 * (s.b0 * s.b2);
-	const double vb = s.v0 * s.b0 + s.v1 * s.b1 + s.v2 * s.b2;
-	F[4] = s.v0 * (s.E + s.p + pb) - s.b0 * vb * g.inv_mu0;
+	F[1] = A::fma(s.m0, s.v0, A::fma(-b0m, s.b0, s.pt));
+	F[2] = A::fma(s.m1, s.v0, -A::mul(b0m, s.b1));
+	F[3] = A::fma(s.m2, s.v0, -A::mul(b0m, s.b2));
+	const double vb = A::fma(s.v2, s.b2, A::fma(s.v1, s.b1, A::mul(s.v0, s.b0)));
+	F[4] = A::fma(s.v0, A::add(s.E, s.pt), -A::mul(b0m, vb));
 	F[5] = 0.0;
-	F[6] = s.v0 * s.b1 - s.b0 * s.v1;
-	F[7] = s.v0 * s.b2 - s.b0 * s.v2;
+	F[6] = A::fma(s.v0, s.b1, -A::mul(s.b0, s.v1));
+	F[7] = A::fma(s.v0, s.b2, -A::mul(s.b0, s.v2));
 }
 
 /*
@@ -295,27 +303,17 @@ __device__ __forceinline__ void physical_flux_bg(
 	F[7] = s.v0 * t2 - t0 * s.v2;
 }
 
-template <bool X = false>
-__device__ __forceinline__ double magnetic_pressure(const Side& s, const Gas& g)
-{
-	if constexpr (X) {
-		using A = Ar<true>;
-		return A::mul(A::mul(0.5, g.inv_mu0), A::fma(s.b2, s.b2, A::fma(s.b1, s.b1, A::mul(s.b0, s.b0))));
-	}
-	return 0.5 * g.inv_mu0 * (s.b0 * s.b0 + s.b1 * s.b1 + s.b2 * s.b2);
-}
-
 /*
 Rusanov (local Lax-Friedrichs), mhd/rusanov.hpp:67-179:
 F = (F_L + F_R)/2 - s/2 (U_R - U_L), s = max(|u_L|, |u_R|) + max(c_f,L, c_f,R).
 The field's normal component is diffused like the rest (the reference
 does not zero it).
 */
-template <bool BG, bool EX = false>
+template <bool BG>
 __device__ __forceinline__ double flux_rusanov(const Side& L, const Side& R, const Gas& g, double F[8],
                                                uint32_t& flag, const double* bg = nullptr)
 {
-	using A = Ar<EX and not BG>;
+	using A = Ar;
 	const double fast = fmax(L.cf, R.cf);
 	const double s = A::add(fmax(fabs(L.v0), fabs(R.v0)), fast);
 	double FL[8], FR[8];
@@ -323,8 +321,8 @@ __device__ __forceinline__ double flux_rusanov(const Side& L, const Side& R, con
 		physical_flux_bg(L, bg[0], bg[1], bg[2], g, FL);
 		physical_flux_bg(R, bg[0], bg[1], bg[2], g, FR);
 	} else {
-		physical_flux<EX>(L, magnetic_pressure<EX>(L, g), g, FL);
-		physical_flux<EX>(R, magnetic_pressure<EX>(R, g), g, FR);
+		physical_flux(L, g, FL);
+		physical_flux(R, g, FR);
 	}
 	const double h = A::mul(0.5, s);
 	const double UL[8] = {L.rho, L.m0, L.m1, L.m2, L.E, L.b0, L.b1, L.b2};
@@ -341,20 +339,21 @@ __device__ __forceinline__ double flux_rusanov(const Side& L, const Side& R, con
 HLL with Davis wave-speed estimates, mhd/hll_athena.hpp:65-275:
 S_L = min(u_L, u_R) - max c_f, S_R = max(u_L, u_R) + max c_f,
 bm = min(S_L, 0), bp = max(S_R, 0); a degenerate fan (bp - bm not a
-positive normal number) gives zero flux and zero speed.
+positive normal number) gives zero flux and zero speed.  The flux as
+bp / (bp - bm) (F_L - bm U_L) - bm / (bp - bm) (F_R - bp U_R).
 */
-template <bool BG, bool EX = false>
+template <bool BG>
 __device__ __forceinline__ double flux_hll(const Side& L, const Side& R, const Gas& g, double F[8],
                                            uint32_t& /*flag*/, const double* bg = nullptr)
 {
-	using A = Ar<EX and not BG>;
+	using A = Ar;
 	const double fast = fmax(L.cf, R.cf);
 	const bool order = L.v0 <= R.v0;
 	const double s_neg = A::sub(order ? L.v0 : R.v0, fast);
 	const double s_pos = A::add(order ? R.v0 : L.v0, fast);
 	const double bm = fmin(s_neg, 0.0), bp = fmax(s_pos, 0.0);
 	const double width = A::sub(bp, bm);
-	if (not (is_normal(width) and width > 0.0)) {
+	if (not is_positive_normal(width)) {
 		#pragma unroll
 		for (int v = 0; v < 8; v++) F[v] = 0.0;
 		return 0.0;
@@ -364,58 +363,47 @@ __device__ __forceinline__ double flux_hll(const Side& L, const Side& R, const G
 		physical_flux_bg(L, bg[0], bg[1], bg[2], g, FL);
 		physical_flux_bg(R, bg[0], bg[1], bg[2], g, FR);
 	} else {
-		physical_flux<EX>(L, magnetic_pressure<EX>(L, g), g, FL);
-		physical_flux<EX>(R, magnetic_pressure<EX>(R, g), g, FR);
+		physical_flux(L, g, FL);
+		physical_flux(R, g, FR);
 	}
 	const double UL[8] = {L.rho, L.m0, L.m1, L.m2, L.E, L.b0, L.b1, L.b2};
 	const double UR[8] = {R.rho, R.m0, R.m1, R.m2, R.E, R.b0, R.b1, R.b2};
-	const double w = A::mul(A::mul(0.5, A::add(bp, bm)), recip(width));
+	const double iw = recip(width);
+	const double wl = A::mul(bp, iw), wr = A::mul(-bm, iw);
 	#pragma unroll
 	for (int v = 0; v < 8; v++) {
-		const double a = (v == 5) ? 0.0 : A::fma(-bm, UL[v], FL[v]);
-		const double b = (v == 5) ? 0.0 : A::fma(-bp, UR[v], FR[v]);
-		F[v] = A::fma(A::sub(a, b), w, A::mul(0.5, A::add(a, b)));
+		F[v] = v == 5 ? 0.0 : A::fma(wl, A::fma(-bm, UL[v], FL[v]), A::mul(wr, A::fma(-bp, UR[v], FR[v])));
 	}
-	return fmax(fabs(bp), fabs(bm));
+	return fmax(bp, -bm);
 }
 
-// transverse velocity and field of one side's star state (Miyoshi & Kusano eqns 44-47); the
-// degeneracy test is a select, so the function is one basic block
+// transverse velocity and field of one side's star state (Miyoshi & Kusano eqns 44-47): v - b t1
+// and b t2, with t1 = 0 and t2 = 1 in the degenerate case (keep)
 struct Star_T {
 	double w1, w2, b1, b2;
+	bool keep;
 };
 
-template <bool EX>
 __device__ __forceinline__ Star_T star_transverse(const Side& X, const double rho_sd, const double sd,
-                                                  const double sm, const double s_mid, const double bx,
-                                                  const double bx2_mu, const double thr, const Gas& g)
+                                                  const double sm, const double s_mid, const double bxm,
+                                                  const double bx2_mu, const double thr)
 {
-	using A = Ar<EX>;
+	using A = Ar;
 	const double tmp = A::fma(rho_sd, sm, -bx2_mu);
 	const double it = recip(tmp);
-	const bool keep = fabs(tmp) < thr;
-	const double t1 = A::mul(A::mul(A::mul(bx, A::sub(s_mid, X.v0)), g.inv_mu0), it);
-	const double t2 = A::mul(A::fma(rho_sd, sd, -bx2_mu), it);
 	Star_T t;
-	t.w1 = keep ? X.v1 : A::fma(-X.b1, t1, X.v1);
-	t.w2 = keep ? X.v2 : A::fma(-X.b2, t1, X.v2);
-	t.b1 = keep ? X.b1 : A::mul(X.b1, t2);
-	t.b2 = keep ? X.b2 : A::mul(X.b2, t2);
+	t.keep = fabs(tmp) < thr;
+	const double t1 = t.keep ? 0.0 : A::mul(A::mul(bxm, A::sub(s_mid, X.v0)), it);
+	const double t2 = t.keep ? 1.0 : A::mul(A::fma(rho_sd, sd, -bx2_mu), it);
+	t.w1 = A::fma(-X.b1, t1, X.v1);
+	t.w2 = A::fma(-X.b2, t1, X.v2);
+	t.b1 = A::mul(X.b1, t2);
+	t.b2 = A::mul(X.b2, t2);
 	return t;
 }
 
 /*
-HLLD of Miyoshi & Kusano (J. Comput. Phys. 208, 2005), as
-mhd/hlld_athena.hpp:62-559; the background field is ignored there (:77)
-and here.  Past the supersonic cases every region's ingredients are
-computed in one straight run (both sides' transverse star states, the
-double-star state) and the reference's region choice (:475-552) selects
-among them, so that the compiler can overlap the two sides' dependency
-chains; values of regions not taken are discarded by selects, never
-multiplied in.
-The side the flux is taken from comes from pick(left): a caller that holds
-the sides' records in shared memory reads that side again instead of
-selecting all of its fields between the two sides held in registers.
+The two sides a face is solved between, when both are held in registers.
 */
 struct Held_Sides {
 	const Side& L;
@@ -423,34 +411,63 @@ struct Held_Sides {
 	__device__ __forceinline__ Side operator()(const bool left) const { return left ? L : R; }
 };
 
-template <bool EX, class PICK>
+/*
+HLLD of Miyoshi & Kusano (J. Comput. Phys. 208, 2005), as
+mhd/hlld_athena.hpp:62-559; the background field is ignored there (:77)
+and here.  Past the supersonic cases every region's ingredients are
+computed in one straight run (both sides' transverse star states, the
+step across the Alfven wave) and the reference's region choice (:475-552)
+selects among them, so that the compiler can overlap the two sides'
+dependency chains; values of regions not taken are discarded by selects,
+never multiplied in.
+
+The reference sums the flux up from the outer state, F + S_out (U* - U) +
+S_in (U** - U*).  The jump conditions that define the star states make
+that sum, in exact arithmetic, the flux of the intermediate state itself
+with the star total pressure,
+  rho* S_M,  rho* S_M^2 + p_t*,  rho* S_M v_t - B_x B_t / mu0,
+  (E + p_t*) S_M - B_x (v . B) / mu0,  S_M B_t - B_x v_t,
+plus what the reference's use of the side's own normal field B_n in F (and
+in v . B of the outer state), where the star states have the mean B_x,
+leaves over:
+  -B_n^2 / mu0 in the normal momentum (the formula has no B_x^2 there),
+  -(B_n - B_x) B_t / mu0, -(B_n - B_x) (v . B) / mu0, -(B_n - B_x) v_t
+of the outer state in the others; in the degenerate case, where the star
+state keeps the outer B_t and v_t, also (v_n - S_M) B_t in the field.
+That is some 60 operations less per face, and the double-star state needs
+only the velocity step across its Alfven wave: v** = v* + dv,
+B** = B* +- sqrt(mu0 rho*) sign(B_x) dv, dv = 0 where there is no such
+wave.  The step is bound by the latency of these FP64 chains: with this
+form, the third-order reciprocals and the fast speed of derive() a 256^3
+step went from 2.14 to 1.73 ms, a 150 x 99 x 67 step from 180 to 148 us.
+
+The side the flux is taken from comes from pick(left): a caller that holds
+the sides' records in shared memory reads that side again instead of
+selecting all of its fields between the two sides held in registers.
+*/
+template <class PICK>
 __device__ __forceinline__ double flux_hlld(const Side& L, const Side& R, const Gas& g, double F[8],
-                                            uint32_t& /*flag*/, const PICK& pick)
+                                            const PICK& pick)
 {
-	using A = Ar<EX>;
+	using A = Ar;
 	const double fast = fmax(L.cf, R.cf);
 	const bool order = L.v0 <= R.v0;
 	const double s_neg = A::sub(order ? L.v0 : R.v0, fast);  // eqn 67
 	const double s_pos = A::add(order ? R.v0 : L.v0, fast);
-	const double pbL = magnetic_pressure<EX>(L, g), pbR = magnetic_pressure<EX>(R, g);
 
-	if (s_neg >= 0.0) {
-		physical_flux<EX>(L, pbL, g, F);
-		return fabs(s_pos);
+	if (s_neg >= 0.0 or s_pos <= 0.0) {
+		const bool from_left = s_neg >= 0.0;
+		physical_flux(pick(from_left), g, F);
+		return from_left ? fabs(s_pos) : fabs(s_neg);
 	}
-	if (s_pos <= 0.0) {
-		physical_flux<EX>(R, pbR, g, F);
-		return fabs(s_neg);
-	}
-	const double speed = fmax(fabs(s_neg), fabs(s_pos));
+	const double speed = fmax(-s_neg, s_pos);
 
 	const double bx = A::mul(0.5, A::add(L.b0, R.b0));
-	const double bx2_mu = A::mul(A::mul(bx, bx), g.inv_mu0);
+	const double bxm = A::mul(bx, g.inv_mu0), bx2_mu = A::mul(bx, bxm);
 	const double sdL = A::sub(s_neg, L.v0), sdR = A::sub(s_pos, R.v0);       // < 0 and > 0 here
-	const double ptL = A::add(L.p, pbL), ptR = A::add(R.p, pbR);
 	const double rsdL = A::mul(L.rho, sdL), rsdR = A::mul(R.rho, sdR);
 	// eqn 38; the denominator is sdR rho_R - sdL rho_L > 0
-	const double s_mid = A::mul(A::add(A::sub(A::fma(sdR, R.m0, -A::mul(sdL, L.m0)), ptR), ptL),
+	const double s_mid = A::mul(A::add(A::sub(A::fma(sdR, R.m0, -A::mul(sdL, L.m0)), R.pt), L.pt),
 	                            recip(A::sub(rsdR, rsdL)));
 	const double smL = A::sub(s_neg, s_mid), smR = A::sub(s_pos, s_mid);     // < 0 and > 0 for physical states
 	const double ismL = recip(smL), ismR = recip(smR);
@@ -461,71 +478,61 @@ __device__ __forceinline__ double flux_hlld(const Side& L, const Side& R, const 
 	// eqn 51
 	const double abx = A::mul(fabs(bx), g.inv_sqrt_mu0);
 	const double ssL = A::fma(-abx, irL, s_mid), ssR = A::fma(abx, irR, s_mid);
-	const double ptst = A::fma(rsdL, A::sub(s_mid, L.v0), ptL);
+	const double ptst = A::fma(rsdL, A::sub(s_mid, L.v0), L.pt);
 	const double thr = A::mul(DBL_EPS, ptst);
 	// transverse star velocity and field of both sides, eqns 44-47
-	const Star_T tl = star_transverse<EX>(L, rsdL, sdL, smL, s_mid, bx, bx2_mu, thr, g);
-	const Star_T tr = star_transverse<EX>(R, rsdR, sdR, smR, s_mid, bx, bx2_mu, thr, g);
+	const Star_T tl = star_transverse(L, rsdL, sdL, smL, s_mid, bxm, bx2_mu, thr);
+	const Star_T tr = star_transverse(R, rsdR, sdR, smR, s_mid, bxm, bx2_mu, thr);
 
 	// region order of hlld_athena.hpp:475-552: S*_L >= 0, S_M >= 0, S*_R > 0, else
 	const bool left = s_mid >= 0.0;
 	const bool star_l = ssL >= 0.0;
 	const bool star_r = not star_l and not left and not (ssR > 0.0);
-	const bool dbl = not star_l and not star_r;
-	const bool useL = star_l or (dbl and left);   // the side the flux is taken from
+	const bool useL = star_l or (not star_r and left);   // the side the flux is taken from
+	// the double-star region (the star state itself when Bx ~ 0)
+	const bool two = not star_l and not star_r and not (A::mul(A::mul(0.5, bx), bx) < thr);
 	const Side S = pick(useL);
-	const Star_T& ts = useL ? tl : tr;
-	const double sd = useL ? sdL : sdR, ism = useL ? ismL : ismR, rs = useL ? rsL : rsR;
-	const double pt = useL ? ptL : ptR, s_out = useL ? s_neg : s_pos;
+	const Star_T ts = useL ? tl : tr;
+	const double ism = useL ? ismL : ismR, rs = useL ? rsL : rsR;
 
-	// that side's full star state, eqn 48 for the energy
-	const double vb_star = A::fma(ts.w2, ts.b2, A::fma(ts.w1, ts.b1, A::mul(s_mid, bx)));
-	const double vb = A::fma(S.v2, S.b2, A::fma(S.v1, S.b1, A::mul(S.v0, S.b0)));
-	double us[8];
-	us[0] = rs; us[1] = A::mul(rs, s_mid); us[2] = A::mul(rs, ts.w1); us[3] = A::mul(rs, ts.w2);
-	{
-		double e = A::fma(sd, S.E, -A::mul(pt, S.v0));
-		e = A::fma(ptst, s_mid, e);
-		e = A::fma(A::mul(bx, g.inv_mu0), A::sub(vb, vb_star), e);
-		us[4] = A::mul(e, ism);
-	}
-	us[5] = bx; us[6] = ts.b1; us[7] = ts.b2;
-	const double U0[8] = {S.rho, S.m0, S.m1, S.m2, S.E, S.b0, S.b1, S.b2};
-	physical_flux<EX>(S, useL ? pbL : pbR, g, F);
-
-	// double-star state, eqns 59-63 (the star state itself when Bx ~ 0)
+	// the step across that side's Alfven wave, eqns 59-62 less the star state
 	const double inv_sum = recip(A::add(sqL, sqR));
 	const double sgn = (bx > 0.0) ? 1.0 : -1.0;
 	const double cv = A::mul(sgn, g.inv_sqrt_mu0);
-	const double v1 = A::mul(inv_sum, A::fma(cv, A::sub(tr.b1, tl.b1), A::fma(sqR, tr.w1, A::mul(sqL, tl.w1))));
-	const double v2 = A::mul(inv_sum, A::fma(cv, A::sub(tr.b2, tl.b2), A::fma(sqR, tr.w2, A::mul(sqL, tl.w2))));
-	const double wb = A::mul(A::mul(A::mul(sgn, sqL), sqR), g.sqrt_mu0);
-	const double b1 = A::mul(inv_sum, A::fma(wb, A::sub(tr.w1, tl.w1), A::fma(sqR, tl.b1, A::mul(sqL, tr.b1))));
-	const double b2 = A::mul(inv_sum, A::fma(wb, A::sub(tr.w2, tl.w2), A::fma(sqR, tl.b2, A::mul(sqL, tr.b2))));
-	const double vb2 = A::fma(v2, b2, A::fma(v1, b1, A::mul(s_mid, bx)));
-	const double e2 = left
-		? A::sub(us[4], A::mul(A::mul(A::mul(sqL, sgn), A::sub(vb_star, vb2)), g.inv_sqrt_mu0))
-		: A::add(us[4], A::mul(A::mul(A::mul(sqR, sgn), A::sub(vb_star, vb2)), g.inv_sqrt_mu0));
-	const bool two = dbl and not (A::mul(A::mul(0.5, bx), bx) < thr);
-	double u2[8];
-	u2[0] = us[0]; u2[1] = us[1];
-	u2[2] = two ? A::mul(rs, v1) : us[2];
-	u2[3] = two ? A::mul(rs, v2) : us[3];
-	u2[4] = two ? e2 : us[4];
-	u2[5] = us[5];
-	u2[6] = two ? b1 : us[6];
-	u2[7] = two ? b2 : us[7];
+	const double near = useL ? sqL : -sqR, far = useL ? sqR : -sqL;
+	const double d1 = A::mul(inv_sum, A::fma(cv, A::sub(tr.b1, tl.b1), A::mul(far, A::sub(tr.w1, tl.w1))));
+	const double d2 = A::mul(inv_sum, A::fma(cv, A::sub(tr.b2, tl.b2), A::mul(far, A::sub(tr.w2, tl.w2))));
+	const double dv1 = two ? d1 : 0.0, dv2 = two ? d2 : 0.0;
+	const double db = A::mul(A::mul(sgn, g.sqrt_mu0), near);
+	const double w1 = A::add(ts.w1, dv1), w2 = A::add(ts.w2, dv2);
+	const double b1 = A::fma(db, dv1, ts.b1), b2 = A::fma(db, dv2, ts.b2);
 
-	// single star: F + s_out (U* - U); double star: F + s_in U** - (s_in - s_out) U* - s_out U
-	const double s_in = left ? ssL : ssR;
-	const double c2 = dbl ? s_in : 0.0;
-	const double c1 = dbl ? A::sub(s_in, s_out) : -s_out;
-	#pragma unroll
-	for (int v = 0; v < 8; v++) {
-		if (v == 5) continue;
-		F[v] = A::fma(-U0[v], s_out, A::fma(-us[v], c1, A::fma(u2[v], c2, F[v])));
-	}
+	// energy of the star state, eqn 48, and of the double-star state, eqn 63
+	const double vb = A::fma(S.v2, S.b2, A::fma(S.v1, S.b1, A::mul(S.v0, S.b0)));
+	const double smb = A::mul(s_mid, bx);
+	const double vb_star = A::fma(ts.w2, ts.b2, A::fma(ts.w1, ts.b1, smb));
+	const double vb2 = A::fma(w2, b2, A::fma(w1, b1, smb));
+	double e = A::fma(A::sub(useL ? s_neg : s_pos, S.v0), S.E, -A::mul(S.pt, S.v0));
+	e = A::fma(ptst, s_mid, e);
+	e = A::fma(bxm, A::sub(vb, vb_star), e);
+	e = A::fma(A::mul(cv, near), A::sub(vb2, vb_star), A::mul(e, ism));
+
+	// the flux
+	const double b0m = A::mul(S.b0, g.inv_mu0);
+	const double over = A::sub(S.b0, bx), overm = A::sub(b0m, bxm);
+	F[0] = A::mul(rs, s_mid);
+	F[1] = A::fma(F[0], s_mid, A::fma(-b0m, S.b0, ptst));
+	F[2] = A::fma(F[0], w1, A::fma(-bxm, b1, -A::mul(overm, S.b1)));
+	F[3] = A::fma(F[0], w2, A::fma(-bxm, b2, -A::mul(overm, S.b2)));
+	F[4] = A::fma(A::add(e, ptst), s_mid, A::fma(-bxm, vb2, -A::mul(overm, vb)));
 	F[5] = 0.0;
+	F[6] = A::fma(s_mid, b1, A::fma(-bx, w1, -A::mul(over, S.v1)));
+	F[7] = A::fma(s_mid, b2, A::fma(-bx, w2, -A::mul(over, S.v2)));
+	if (ts.keep) {
+		const double kv = A::sub(S.v0, s_mid);
+		F[6] = A::fma(kv, S.b1, F[6]);
+		F[7] = A::fma(kv, S.b2, F[7]);
+	}
 	return speed;
 }
 
@@ -777,32 +784,25 @@ __device__ __forceinline__ double flux_roe(const Side& L, const Side& R, const G
 	return fmax(fabs(s_neg), fabs(s_pos));
 }
 
-template <bool EX = false>
-__device__ __forceinline__ double flux_hlld(const Side& L, const Side& R, const Gas& g, double F[8],
-                                            uint32_t& flag)
-{
-	return flux_hlld<EX>(L, R, g, F, flag, Held_Sides{L, R});
-}
-
-// pick: see flux_hlld (the other solvers use the sides held); EX: Ar<true> arithmetic for HLLD
-template <int SOLVER, bool EX = false, class PICK>
+// pick: see flux_hlld (the other solvers use the sides held)
+template <int SOLVER, class PICK>
 __device__ __forceinline__ double solve_face(const Side& L, const Side& R, const Gas& g, double F[8],
                                              uint32_t& flag, const PICK& pick)
 {
 	flag = L.bad | R.bad;
 	if (flag & PAMHD_FLAG_DENSITY) flag = PAMHD_FLAG_DENSITY;
 	else if (flag & PAMHD_FLAG_PRESSURE) flag = PAMHD_FLAG_PRESSURE;
-	if (SOLVER == PAMHD_RUSANOV) return flux_rusanov<false, EX>(L, R, g, F, flag);
-	if (SOLVER == PAMHD_HLL_ATHENA) return flux_hll<false, EX>(L, R, g, F, flag);
-	if (SOLVER == PAMHD_HLLD_ATHENA) return flux_hlld<EX>(L, R, g, F, flag, pick);
+	if (SOLVER == PAMHD_RUSANOV) return flux_rusanov<false>(L, R, g, F, flag);
+	if (SOLVER == PAMHD_HLL_ATHENA) return flux_hll<false>(L, R, g, F, flag);
+	if (SOLVER == PAMHD_HLLD_ATHENA) return flux_hlld(L, R, g, F, pick);
 	return flux_roe(L, R, g, F, flag);
 }
 
-template <int SOLVER, bool EX = false>
+template <int SOLVER>
 __device__ __forceinline__ double solve_face(const Side& L, const Side& R, const Gas& g, double F[8],
                                              uint32_t& flag)
 {
-	return solve_face<SOLVER, EX>(L, R, g, F, flag, Held_Sides{L, R});
+	return solve_face<SOLVER>(L, R, g, F, flag, Held_Sides{L, R});
 }
 
 } // namespace pamhd_b200

@@ -142,7 +142,7 @@ plane's stores apart from the reads of the plane two before it.
 constexpr int STX = 32, STY = 8;            // 256 threads, two blocks per SM (one for Roe)
 constexpr int SW = STX + 1;                 // a record row: the -x halo at column 0
 constexpr int SCELLS = SW * (STY + 1);      // record rows: the -y halo at row 0
-constexpr int SREC = 13;                    // rho, mom xyz, E, B xyz, 1/rho, p, c_f xyz
+constexpr int SREC = 13;                    // rho, mom xyz, E, B xyz, 1/rho, pressure, c_f xyz
 constexpr int SSLOT = SREC * SCELLS;        // doubles of one slot
 constexpr int SSLOTS = 3;
 constexpr size_t SMEM_FACES = SSLOTS * (SSLOT * sizeof(double) + SCELLS * sizeof(uint32_t));
@@ -152,7 +152,7 @@ Read cell c from HBM and derive its record into slot position r, with the
 fast speeds along the axes its faces in the tile need (a halo cell only
 along the axis of the face it shares with the tile).
 */
-template <bool CX, bool CY, bool CZ>
+template <bool CX, bool CY, bool CZ, bool BG>
 __device__ __forceinline__ void stage_cell(const Stag_Params& P, double* rec, uint32_t* bad, const int r,
                                            const long long c)
 {
@@ -163,7 +163,7 @@ __device__ __forceinline__ void stage_cell(const Stag_Params& P, double* rec, ui
 	#pragma unroll
 	for (int v = 0; v < 8; v++) rec[v * SCELLS + r] = U[v];
 	rec[8 * SCELLS + r] = d.rinv;
-	rec[9 * SCELLS + r] = d.p;
+	rec[9 * SCELLS + r] = BG ? d.p : d.pt;
 	if (CX) rec[10 * SCELLS + r] = d.cf[0];
 	if (CY) rec[11 * SCELLS + r] = d.cf[1];
 	if (CZ) rec[12 * SCELLS + r] = d.cf[2];
@@ -180,7 +180,7 @@ __device__ __forceinline__ void stage_cell(const Stag_Params& P, double* rec, ui
 }
 
 // the cell at slot position r seen from a face normal to axis A (as side_of<A>)
-template <int A>
+template <int A, bool BG>
 __device__ __forceinline__ Side side_rec(const double* rec, const uint32_t* bad, const int r)
 {
 	Side s;
@@ -189,7 +189,8 @@ __device__ __forceinline__ Side side_rec(const double* rec, const uint32_t* bad,
 	s.E = rec[4 * SCELLS + r];
 	rotate<A>(rec[5 * SCELLS + r], rec[6 * SCELLS + r], rec[7 * SCELLS + r], s.b0, s.b1, s.b2);
 	s.rinv = rec[8 * SCELLS + r];
-	s.p = rec[9 * SCELLS + r];
+	// with a background field the record holds the thermal pressure, else thermal plus magnetic
+	s.p = s.pt = rec[9 * SCELLS + r];
 	s.cf = rec[(10 + A) * SCELLS + r];
 	s.v0 = s.m0 * s.rinv;
 	s.v1 = s.m1 * s.rinv;
@@ -219,9 +220,7 @@ __device__ __forceinline__ void solve_minus_face(const Stag_Params& P, Side L, S
 		s = SOLVER == PAMHD_RUSANOV ? flux_rusanov<true>(L, R, P.gas, G, flag, b)
 		                            : flux_hll<true>(L, R, P.gas, G, flag, b);
 	} else {
-		// HLLD in explicitly rounded arithmetic (fused multiply-adds: fewer instructions under
-		// -fmad=false); the other solvers as written, in the oracle's operation order
-		s = solve_face<SOLVER, SOLVER == PAMHD_HLLD_ATHENA>(L, R, P.gas, G, flag);
+		s = solve_face<SOLVER>(L, R, P.gas, G, flag);
 	}
 	if (flag != 0) record_failure(P, flag, m, A);
 	smax = fmax(smax, s);
@@ -278,7 +277,7 @@ __global__ void __launch_bounds__(STX * STY, SOLVER == PAMHD_ROE_ATHENA ? 1 : 2)
 	double s0 = 0.0, s1 = 0.0, s2 = 0.0;
 	bool zero = false;
 	// the plane before the chunk, own cells only: the left sides of the first plane's -z faces
-	if (own) stage_cell<false, false, true>(P, smem, bad_base, ri, col + plane * (kb == 0 ? nz - 1 : kb - 1));
+	if (own) stage_cell<false, false, true, BG>(P, smem, bad_base, ri, col + plane * (kb == 0 ? nz - 1 : kb - 1));
 	for (int k = kb; k < ke; k++) {
 		const int t = k - kb + 1;
 		double* const rec = smem + (t % SSLOTS) * SSLOT;
@@ -286,26 +285,26 @@ __global__ void __launch_bounds__(STX * STY, SOLVER == PAMHD_ROE_ATHENA ? 1 : 2)
 		const double* const prv = smem + ((t - 1) % SSLOTS) * SSLOT;
 		const uint32_t* const pbad = bad_base + ((t - 1) % SSLOTS) * SCELLS;
 		const long long kofs = plane * k;
-		if (own) stage_cell<true, true, true>(P, rec, bad, ri, col + kofs);
+		if (own) stage_cell<true, true, true, BG>(P, rec, bad, ri, col + kofs);
 		if (ty == 0) {
-			if (hr >= 0) stage_cell<false, true, false>(P, rec, bad, hr, hcol + kofs);
+			if (hr >= 0) stage_cell<false, true, false, BG>(P, rec, bad, hr, hcol + kofs);
 		} else if (hr >= 0) {
-			stage_cell<true, false, false>(P, rec, bad, hr, hcol + kofs);
+			stage_cell<true, false, false, BG>(P, rec, bad, hr, hcol + kofs);
 		}
 		__syncthreads();
 		if (own) {
 			const long long c = col + kofs;
 			const long long mz = col + plane * (k == 0 ? nz - 1 : k - 1);
 			if (has_x) {
-				solve_minus_face<SOLVER, 0, BG>(P, side_rec<0>(rec, bad, ri - 1), side_rec<0>(rec, bad, ri), c,
+				solve_minus_face<SOLVER, 0, BG>(P, side_rec<0, BG>(rec, bad, ri - 1), side_rec<0, BG>(rec, bad, ri), c,
 				                                col_mx + kofs, s0, zero);
 			}
 			if (has_y) {
-				solve_minus_face<SOLVER, 1, BG>(P, side_rec<1>(rec, bad, ri - SW), side_rec<1>(rec, bad, ri), c,
+				solve_minus_face<SOLVER, 1, BG>(P, side_rec<1, BG>(rec, bad, ri - SW), side_rec<1, BG>(rec, bad, ri), c,
 				                                col_my + kofs, s1, zero);
 			}
 			if (not (P.ext[2] and k == 0)) {
-				solve_minus_face<SOLVER, 2, BG>(P, side_rec<2>(prv, pbad, ri), side_rec<2>(rec, bad, ri), c, mz,
+				solve_minus_face<SOLVER, 2, BG>(P, side_rec<2, BG>(prv, pbad, ri), side_rec<2, BG>(rec, bad, ri), c, mz,
 				                                s2, zero);
 			}
 		}

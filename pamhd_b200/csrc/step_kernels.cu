@@ -46,10 +46,11 @@ constexpr int TX = 32;
 constexpr int TY_3D = PAMHD_TY;     // tile rows of the batched step on 2-D and 3-D grids
 constexpr int MINB = PAMHD_MINB;    // resident blocks per SM asked of the register allocator
 constexpr int TY_STEP = PAMHD_STEP_TY;  // tile rows of the single-grid step (Roe aside)
-// record of a cell in shared memory: rho, mom xyz, E, B xyz, 1/rho, p, cf x, cf y (the fast
+// record of a cell in shared memory: rho, mom xyz, E, B xyz, 1/rho, thermal plus magnetic
+// pressure, cf x, cf y (the fast
 // speed along z is needed by the column's owner only, which keeps it in a register)
 constexpr int NV = 12;
-enum { R_RINV = 8, R_P = 9, R_CF = 10 };
+enum { R_RINV = 8, R_PT = 9, R_CF = 10 };
 
 /*
 Rows of a face flux kept in shared memory, in the face frame: rho, the
@@ -336,11 +337,11 @@ __device__ __forceinline__ double load_record(const Step_Params& P, double* rec,
 	double U[8];
 	#pragma unroll
 	for (int v = 0; v < 8; v++) U[v] = CO ? __ldcg(P.in + v * P.L.var + off) : __ldg(P.in + v * P.L.var + off);
-	const Derived d = derive<CX, CY, CZ, true>(U[0], U[1], U[2], U[3], U[4], U[5], U[6], U[7], P.gas);
+	const Derived d = derive<CX, CY, CZ>(U[0], U[1], U[2], U[3], U[4], U[5], U[6], U[7], P.gas);
 	#pragma unroll
 	for (int v = 0; v < 8; v++) rec[v * cells + ri] = U[v];
 	rec[R_RINV * cells + ri] = d.rinv;
-	rec[R_P * cells + ri] = d.p;
+	rec[R_PT * cells + ri] = d.pt;
 	if (CX) rec[(R_CF + 0) * cells + ri] = d.cf[0];
 	if (CY) rec[(R_CF + 1) * cells + ri] = d.cf[1];
 	bad[ri] = uint8_t(d.bad);
@@ -360,7 +361,8 @@ __device__ __forceinline__ Side side_at(const double* rec, const uint8_t* bad, c
 	s.E = rec[4 * cells + ri];
 	rotate<A>(rec[5 * cells + ri], rec[6 * cells + ri], rec[7 * cells + ri], s.b0, s.b1, s.b2);
 	s.rinv = rec[R_RINV * cells + ri];
-	s.p = rec[R_P * cells + ri];
+	s.pt = rec[R_PT * cells + ri];
+	s.p = 0.0;  // not read without a background field
 	s.cf = cf;
 	s.v0 = s.m0 * s.rinv;
 	s.v1 = s.m1 * s.rinv;
@@ -389,7 +391,7 @@ __device__ __forceinline__ void solve_z(const Step_Params& P, const double* rec_
 	const auto pick = [&](const bool left) {
 		return side_at<2>(left ? rec_l : rec_r, left ? bad_l : bad_r, CELLS, ri, left ? cf_l : cf_r);
 	};
-	const double s = solve_face<SOLVER, true>(L, R, P.gas, F, flag, pick);
+	const double s = solve_face<SOLVER>(L, R, P.gas, F, flag, pick);
 	if (flag != 0) record_failure(P, flag, i, j, k, 3);
 	smax = fmax(smax, s);
 	zero = zero or not (s > 0.0);
@@ -425,7 +427,8 @@ __device__ __forceinline__ void solve_xy(const Step_Params& P, const double* rec
 		s.b1 = rec[(5 + a1) * CELLS + r];
 		s.b2 = rec[(5 + a2) * CELLS + r];
 		s.rinv = rec[R_RINV * CELLS + r];
-		s.p = rec[R_P * CELLS + r];
+		s.pt = rec[R_PT * CELLS + r];
+		s.p = 0.0;  // not read without a background field
 		s.cf = rec[(R_CF + a) * CELLS + r];
 		s.v0 = s.m0 * s.rinv;
 		s.v1 = s.m1 * s.rinv;
@@ -438,7 +441,7 @@ __device__ __forceinline__ void solve_xy(const Step_Params& P, const double* rec
 	double F[8];
 	uint32_t flag = 0;
 	const auto pick = [&](const bool left) { return side(left ? rl : rr); };
-	const double sp = solve_face<SOLVER, true>(L, R, P.gas, F, flag, pick);
+	const double sp = solve_face<SOLVER>(L, R, P.gas, F, flag, pick);
 	if (flag != 0) record_failure(P, flag, i, j, k, a + 1);
 	if (a == 0) s0 = fmax(s0, sp); else s1 = fmax(s1, sp);
 	zero = zero or not (sp > 0.0);
@@ -785,6 +788,7 @@ __device__ __forceinline__ void boundary_face(const Step_Params& P, const int d,
 		s.rinv = dd.rinv;
 		s.v0 = s.m0 * s.rinv; s.v1 = s.m1 * s.rinv; s.v2 = s.m2 * s.rinv;
 		s.p = dd.p;
+		s.pt = dd.pt;
 		s.cf = dd.cf[e];
 		s.bad = dd.bad;
 	};
@@ -792,7 +796,7 @@ __device__ __forceinline__ void boundary_face(const Step_Params& P, const int d,
 	fill(R, UB, db);
 	double F[8];
 	uint32_t flag = 0;
-	const double sp = solve_face<SOLVER, true>(L, R, P.gas, F, flag);
+	const double sp = solve_face<SOLVER>(L, R, P.gas, F, flag);
 	if (flag != 0) record_failure(P, flag, a[0], a[1], a[2], e + 1);
 	smax[e] = fmax(smax[e], sp);
 	zero = zero or not (sp > 0.0);
@@ -1042,6 +1046,7 @@ __device__ __forceinline__ Side face_side(const double* s, const double* bg, con
 	out.rinv = d.rinv;
 	out.v0 = d.vx; out.v1 = d.vy; out.v2 = d.vz;
 	out.p = d.p;
+	out.pt = d.pt;
 	out.cf = d.cf[0];
 	out.bad = d.bad;
 	if (use_bg) {
@@ -1080,9 +1085,9 @@ __global__ void face_flux_kernel(long long n, const double* __restrict__ neg, co
 		if (flag & PAMHD_FLAG_DENSITY) flag = PAMHD_FLAG_DENSITY;
 		else if (flag & PAMHD_FLAG_PRESSURE) flag = PAMHD_FLAG_PRESSURE;
 		double s;
-		if (SOLVER == PAMHD_RUSANOV) s = use_bg ? flux_rusanov<true>(L, R, g, F, flag, b) : flux_rusanov<false, true>(L, R, g, F, flag);
-		else if (SOLVER == PAMHD_HLL_ATHENA) s = use_bg ? flux_hll<true>(L, R, g, F, flag, b) : flux_hll<false, true>(L, R, g, F, flag);
-		else if (SOLVER == PAMHD_HLLD_ATHENA) s = flux_hlld<true>(L, R, g, F, flag);
+		if (SOLVER == PAMHD_RUSANOV) s = use_bg ? flux_rusanov<true>(L, R, g, F, flag, b) : flux_rusanov<false>(L, R, g, F, flag);
+		else if (SOLVER == PAMHD_HLL_ATHENA) s = use_bg ? flux_hll<true>(L, R, g, F, flag, b) : flux_hll<false>(L, R, g, F, flag);
+		else if (SOLVER == PAMHD_HLLD_ATHENA) s = flux_hlld(L, R, g, F, Held_Sides{L, R});
 		else s = flux_roe(L, R, g, F, flag);
 		for (int v = 0; v < 8; v++) flux[8 * t + v] = flag ? 0.0 : F[v];
 		speed[t] = flag ? 0.0 : s;
