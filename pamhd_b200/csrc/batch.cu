@@ -38,7 +38,8 @@ struct pamhd_batch {
 	cudaStream_t stream = nullptr;
 	int nboxes = 0;
 	int solver = 0;
-	bool yact = true;
+	bool yact = true, zact = true;   // every box has the same active dimensions
+	Tile_Kind kind(const int rows) const { return Tile_Kind{solver, rows, zact}; }
 	std::vector<pamhd_cfg> cfg;
 	std::vector<Layout> L;
 	std::vector<long long> off;      // doubles from the start of a state buffer to each box
@@ -249,7 +250,7 @@ int issue_step(pamhd_batch& b)
 		PAMHD_TRY(launch_batch_boundary_speeds(b.d_params[b.cur], b.nboxes, b.largest_plane, phase, b.solver,
 		                                       b.stream));
 	}
-	PAMHD_TRY(launch_batch_step(b.d_params[b.cur], b.d_items, b.nitems, phase, b.grid, b.solver, b.ty, b.stream));
+	PAMHD_TRY(launch_batch_step(b.d_params[b.cur], b.d_items, b.nitems, phase, b.grid, b.kind(b.ty), b.stream));
 	b.cur ^= 1;
 	b.steps++;
 	return PAMHD_OK;
@@ -310,7 +311,7 @@ int run_steps(pamhd_batch& b, int left)
 int set_run_grid(pamhd_batch& b)
 {
 	int per_sm = 0, sms = 0;
-	PAMHD_TRY(batch_run_blocks_per_sm(b.solver, b.ty, &per_sm));
+	PAMHD_TRY(batch_run_blocks_per_sm(b.kind(b.ty), &per_sm));
 	PAMHD_TRY(check(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, b.device)));
 	if (per_sm < 1) return PAMHD_ERR_CUDA;
 	b.run_grid = std::max(1, std::min(b.nitems_run, sms * per_sm));
@@ -323,7 +324,7 @@ int issue_run(pamhd_batch& b, const int nsteps)
 	PAMHD_TRY(check(cudaMemsetAsync(b.sync, 0, sizeof(Run_Sync), b.stream)));
 	PAMHD_TRY(check(cudaMemsetAsync(b.d_done, 0, b.nboxes * sizeof(unsigned int), b.stream)));
 	return launch_batch_run(b.d_params[b.cur], b.d_params[b.cur ^ 1], b.d_items, b.nitems_run, b.d_box_items,
-	                        b.d_done, b.nboxes, b.steps, nsteps, b.sync, b.wait_limit, b.run_grid, b.solver, b.ty,
+	                        b.d_done, b.nboxes, b.steps, nsteps, b.sync, b.wait_limit, b.run_grid, b.kind(b.ty),
 	                        b.stream);
 }
 
@@ -408,6 +409,7 @@ int pamhd_gpu_batch_create(const int32_t device, const int32_t nboxes, const pam
 	b->nboxes = nboxes;
 	b->solver = cfgs[0].solver;
 	b->yact = cfgs[0].n[1] > 1;
+	b->zact = cfgs[0].n[2] > 1;
 	b->cfg.assign(cfgs, cfgs + nboxes);
 	long long largest_cells = 0;
 	for (int i = 0; i < nboxes; i++) {
@@ -439,11 +441,11 @@ int pamhd_gpu_batch_create(const int32_t device, const int32_t nboxes, const pam
 	}
 	b->ty = b->yact ? batch_tile_rows() : 1;
 	for (const int ty: tile_choices(*b)) {
-		if (prepare_batch_kernels(b->solver, ty) != PAMHD_OK) return fail(PAMHD_ERR_CUDA);
-		if (prepare_batch_run_kernels(b->solver, ty) != PAMHD_OK) return fail(PAMHD_ERR_CUDA);
+		if (prepare_batch_kernels(b->kind(ty)) != PAMHD_OK) return fail(PAMHD_ERR_CUDA);
+		if (prepare_batch_run_kernels(b->kind(ty)) != PAMHD_OK) return fail(PAMHD_ERR_CUDA);
 	}
 	int per_sm = 0;
-	if (batch_blocks_per_sm(b->solver, b->ty, &per_sm) != PAMHD_OK or per_sm < 1) return fail(PAMHD_ERR_CUDA);
+	if (batch_blocks_per_sm(b->kind(b->ty), &per_sm) != PAMHD_OK or per_sm < 1) return fail(PAMHD_ERR_CUDA);
 	int sms = 0;
 	cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
 	if (build_work(*b, 32) != PAMHD_OK) return fail(PAMHD_ERR_CUDA);
@@ -659,7 +661,7 @@ int pamhd_gpu_batch_tune(pamhd_batch* b, const int32_t trial_steps, int32_t* pla
 		if (rc != PAMHD_OK) break;
 		b->ty = ty;
 		int per_sm = 0;
-		rc = batch_blocks_per_sm(b->solver, ty, &per_sm);
+		rc = batch_blocks_per_sm(b->kind(ty), &per_sm);
 		if (rc == PAMHD_OK) rc = build_work(*b, planes);
 		for (const int waves: {1, 2, 0}) {
 			if (rc != PAMHD_OK) break;

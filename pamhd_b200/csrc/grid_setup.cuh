@@ -151,7 +151,7 @@ inline bool grid_params(const pamhd_cfg& c, const Layout& L, Step_Params& P, con
 		if (P.active[d] and not P.periodic[d] and own_side and active_count > 1) needs_boundary_speeds = true;
 	}
 	// z planes per block: enough blocks for several waves on 148 SMs, few redundant z faces
-	const int ty = P.active[1] ? step_tile_rows(c.solver) : 1;
+	const int ty = step_tile(c.solver, P.active[1], P.active[2]).rows;
 	const long long tiles = (long long)((c.n[0] + 31) / 32) * ((c.n[1] + ty - 1) / ty);
 	long long chunks = (PAMHD_CHUNK_BLOCKS + tiles - 1) / tiles;
 	chunks = std::max(1LL, std::min(chunks, (long long)std::max(1, c.n[2] / 16)));

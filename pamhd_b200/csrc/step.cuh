@@ -110,6 +110,13 @@ struct Step_Params {
 	const Inflow_Table* inflow;  // [3][2] by dimension and side (lo, hi) in device memory, or nullptr
 };
 
+// the kernel instance a grid or batch runs: solver, tile rows (1: y inactive), whether there are z faces
+struct Tile_Kind {
+	int solver;
+	int rows;
+	bool zact;
+};
+
 // launchers (step_kernels.cu)
 int launch_step(const Step_Params& P, int solver, cudaStream_t stream);
 int launch_boundary_speeds(const Step_Params& P, int solver, cudaStream_t stream);
@@ -117,25 +124,26 @@ int launch_scatter(const double* packed, double* var_base, const Layout& L, cuda
 int launch_gather(const double* var_base, double* packed, const Layout& L, cudaStream_t stream);
 int launch_fill_ghosts_values(const Step_Params& P, double* state, const double lo[3][8], const double hi[3][8],
                               cudaStream_t stream);
-int prepare_step_kernels(int solver, bool y_active);
+int prepare_step_kernels(const Tile_Kind& kind);
 int launch_face_flux(int solver, long long n, const double* neg, const double* pos, const double* bg,
                      const Gas& gas, double* flux, double* speed, uint32_t* flags, cudaStream_t stream);
 int launch_totals(const double* state, const Layout& L, double volume, double* partial, int nblocks,
                   cudaStream_t stream);
-int step_tile_rows(int solver);
+Tile_Kind step_tile(int solver, bool yact, bool zact);
 int batch_tile_rows();
-int prepare_batch_kernels(int solver, int tile_rows);
-int batch_blocks_per_sm(int solver, int tile_rows, int* blocks);
-int launch_batch_step(const Step_Params* boxes, const int4* items, int nitems, int phase, int grid, int solver,
-                      int tile_rows, cudaStream_t stream);
+int prepare_batch_kernels(const Tile_Kind& kind);
+int batch_blocks_per_sm(const Tile_Kind& kind, int* blocks);
+int launch_batch_step(const Step_Params* boxes, const int4* items, int nitems, int phase, int grid,
+                      const Tile_Kind& kind, cudaStream_t stream);
 int launch_batch_boundary_speeds(const Step_Params* boxes, int nboxes, int largest, int phase, int solver,
                                  cudaStream_t stream);
 // the persistent batched run: nsteps steps of every box in one cooperative launch (see batch_run_kernel)
-int prepare_batch_run_kernels(int solver, int tile_rows);
-int batch_run_blocks_per_sm(int solver, int tile_rows, int* blocks);
+int prepare_batch_run_kernels(const Tile_Kind& kind);
+int batch_run_blocks_per_sm(const Tile_Kind& kind, int* blocks);
 int launch_batch_run(const Step_Params* boxes_even, const Step_Params* boxes_odd, const int4* items, int nitems,
                      const int* box_items, unsigned int* done, int nboxes, long long step0, int nsteps,
-                     Run_Sync* sync, long long wait_limit, int grid, int solver, int tile_rows, cudaStream_t stream);
+                     Run_Sync* sync, long long wait_limit, int grid, const Tile_Kind& kind,
+                     cudaStream_t stream);
 constexpr int BOUNDARY_CHUNK = 4096;  // ghost-ghost faces per boundary work item of the persistent run
 
 } // namespace pamhd_b200

@@ -1,7 +1,7 @@
 /*
 Kernels of the fused finite-volume MHD step (sm_100a, FP64 CUDA cores).
 
-step_kernel<SOLVER, TY, MINB> - one launch = one whole step (the reference's
+step_kernel<SOLVER, TY, ZACT> - one launch = one whole step (the reference's
   get_all_fluxes + update_mhd_state + minimize_timestep, mhd/solve.hpp:
   1702-1811, :1518-1614, :1933-2014, in their cell-centred form):
   * a block owns a 32 x TY column tile and marches along z through a chunk
@@ -26,26 +26,20 @@ and one z plane per chunk are solved twice.
 */
 #include <cuda_runtime.h>
 
+#include <type_traits>
+
 #include "step.cuh"
 
 namespace pamhd_b200 {
 
 constexpr int TX = 32;
-#ifndef PAMHD_TY
-#define PAMHD_TY 4
-#endif
-#ifndef PAMHD_MINB
-#define PAMHD_MINB 3
-#endif
-#ifndef PAMHD_STEP_TY
-#define PAMHD_STEP_TY 8
-#endif
-#ifndef PAMHD_STEP_MINB
-#define PAMHD_STEP_MINB 2
-#endif
-constexpr int TY_3D = PAMHD_TY;     // tile rows of the batched step on 2-D and 3-D grids
-constexpr int MINB = PAMHD_MINB;    // resident blocks per SM asked of the register allocator
-constexpr int TY_STEP = PAMHD_STEP_TY;  // tile rows of the single-grid step (Roe aside)
+constexpr int TY_3D = 4;     // the smaller tile: 32 x 4
+constexpr int TY_WIDE = 8;   // the larger: 32 x 8
+
+// resident blocks per SM asked of the register allocator: 16 warps of at most 128 registers with
+// 32 x 8 tiles, 12 warps of at most 168 with 32 x 4 (and one-row) tiles
+template <int TY, bool ZACT> struct Resident { static constexpr int blocks = TY == TY_WIDE ? 2 : 3; };
+
 // record of a cell in shared memory: rho, mom xyz, E, B xyz, 1/rho, thermal plus magnetic
 // pressure, cf x, cf y (the fast
 // speed along z is needed by the column's owner only, which keeps it in a register)
@@ -60,7 +54,7 @@ solver whose flux of it is not zero (mhd/rusanov.hpp diffuses it).
 */
 template <int SOLVER> struct Flux_Rows { static constexpr int N = SOLVER == PAMHD_RUSANOV ? 8 : 7; };
 
-template <int TY, int NF = 8> struct Tile {
+template <int TY, bool ZACT, int NF = 8> struct Tile {
 	static constexpr int JO = (TY > 1) ? 1 : 0;            // halo rows exist when y is active
 	static constexpr int W = TX + 2;                       // record row width (halo columns)
 	static constexpr int H = TY + 2 * JO;                  // record rows
@@ -68,31 +62,14 @@ template <int TY, int NF = 8> struct Tile {
 	static constexpr int REC = NV * CELLS;                 // doubles per plane slot
 	static constexpr int FXN = TY * (TX + 1);              // x faces of a plane
 	static constexpr int FYN = (TY > 1) ? (TY + 1) * TX : 0;
-	// two record slots, the x and y face fluxes, one validity byte per cell and slot
-	static constexpr size_t BYTES = size_t(2 * REC + NF * FXN + NF * FYN) * 8 + size_t(2 * CELLS);
+	static constexpr int SLOTS = ZACT ? 2 : 1;             // planes whose records are held
+	// the record slots, the x and y face fluxes, one validity byte per cell and slot
+	static constexpr size_t BYTES = size_t(SLOTS * REC + NF * FXN + NF * FYN) * 8 + size_t(SLOTS * CELLS);
 };
 
-template <int SOLVER, int TY> constexpr size_t tile_bytes() { return Tile<TY, Flux_Rows<SOLVER>::N>::BYTES; }
-
-/*
-Tile rows of the single-grid step on 2-D and 3-D grids and the resident
-blocks per SM it is built for: 32 x 8 tiles, two blocks of 256 threads per
-SM at 128 registers (16 warps per SM; a taller tile solves fewer halo
-faces and records per cell); Roe's solver needs more registers than that,
-so it keeps 32 x 4 tiles at three blocks per SM.
-*/
-template <int SOLVER> struct Step_Shape {
-	static constexpr int rows = SOLVER == PAMHD_ROE_ATHENA ? TY_3D : TY_STEP;
-	static constexpr int blocks = SOLVER == PAMHD_ROE_ATHENA ? MINB : PAMHD_STEP_MINB;
-};
-
-template <int SOLVER, int TY> struct Step_Minb {
-	static constexpr int value = (TY > 1 and TY == Step_Shape<SOLVER>::rows) ? Step_Shape<SOLVER>::blocks : MINB;
-};
-
-int step_tile_rows(const int solver)
+template <int SOLVER, int TY, bool ZACT> constexpr size_t tile_bytes()
 {
-	return solver == PAMHD_ROE_ATHENA ? Step_Shape<PAMHD_ROE_ATHENA>::rows : TY_STEP;
+	return Tile<TY, ZACT, Flux_Rows<SOLVER>::N>::BYTES;
 }
 
 int batch_tile_rows()
@@ -150,6 +127,52 @@ __device__ __forceinline__ bool stopped_before(const Step_Params& P)
 {
 	const unsigned int at = __ldcg(&P.status->fail_step);
 	return at != 0u and (long long)(at - 1u) < __ldcg(&P.clock[P.phase].steps);
+}
+
+/*
+A block barrier in two halves (an mbarrier in shared memory, one arrival
+per warp): what a warp does between its arrival and its wait overlaps the
+other warps' way to theirs.  phase counts the block's uses, from 0.
+*/
+struct Split_Barrier {
+	uint32_t addr;   // shared-memory address
+	uint32_t phase;
+
+	// by one thread, before a __syncthreads()
+	__device__ __forceinline__ void init(const uint32_t warps) const
+	{
+		asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" :: "r"(addr), "r"(warps) : "memory");
+	}
+
+	__device__ __forceinline__ void arrive() const
+	{
+		__syncwarp();
+		if ((threadIdx.x & 31) == 0) {
+			asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" :: "r"(addr) : "memory");
+		}
+	}
+
+	// false (with PAMHD_FLAG_TIMEOUT raised) when the other warps did not arrive within the poll limit
+	__device__ __forceinline__ bool wait(Status* status)
+	{
+		const uint32_t parity = phase & 1u;
+		phase++;
+		#pragma unroll 1
+		for (int poll = 0; poll < (1 << 20); poll++) {
+			uint32_t done;
+			asm volatile("{\n\t.reg .pred p;\n\t"
+			             "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+			             "selp.u32 %0, 1, 0, p;\n\t}" : "=r"(done) : "r"(addr), "r"(parity) : "memory");
+			if (done) return true;
+		}
+		atomicOr(&status->flags, (unsigned int)PAMHD_FLAG_TIMEOUT);
+		return false;
+	}
+};
+
+__device__ __forceinline__ Split_Barrier split_barrier(unsigned long long* const word)
+{
+	return Split_Barrier{uint32_t(__cvta_generic_to_shared(word)), 0u};
 }
 
 // block-wide start of a step: every block computes dt; block 0 advances the clock ring.  *s_stop:
@@ -494,27 +517,36 @@ chunk bz, marched plane by plane; the face speeds are folded into
 s0, s1, s2 and zero (flushed by the caller).  Shared by the single-grid
 and the batched kernels, so that both compute the same bits.
 
-Per plane k: (a) stage the plane's records (two slots alternate, so the
-z face between planes k - 1 and k can read both); (b) every x and y face
-of the plane into shared memory, and the z face below each own cell in
-registers, which completes the cell below: its new state is written; (c)
-each own cell's state plus its x and y flux differences, and the flux of
-its -z face, held in registers until the +z face of the next plane.
+The records of plane k (two slots alternate, so that the z face between
+planes k and k + 1 can read both) are staged an iteration ahead; per plane:
+  (a) a block barrier: the plane's records are there, and the fluxes of the
+      plane before were used;
+  (b) every x and y face of the plane into shared memory, then the arrival
+      at the split barrier;
+  (c) what needs no other warp: the next plane's records, and the z face
+      above each own cell, whose two sides the thread staged itself;
+  (d) the wait for the other warps' x and y fluxes, then the own cell:
+      state plus x and y flux differences plus its two z fluxes, written.
+Stage and z face between arrival and wait leave a warp that has an extra
+pass in (b) two thirds of a plane's work to catch up in: with one barrier
+before and one after (b) warps spent 18 % of their time at the two, and a
+256^3 HLLD step took 1.73 ms; split, 1.56 ms.
+A grid without z faces (ZACT false) has one plane and nothing to overlap:
+one record slot and two block barriers.
 */
-template <int SOLVER, int TY, bool CO = false>
-__device__ __forceinline__ void tile_step(const Step_Params& P, double* const smem, const double dt,
-                                          const int bx, const int by, const int bz,
+template <int SOLVER, int TY, bool ZACT, bool CO = false>
+__device__ __forceinline__ void tile_step(const Step_Params& P, double* const smem, Split_Barrier& bar,
+                                          const double dt, const int bx, const int by, const int bz,
                                           double& s0, double& s1, double& s2, bool& zero)
 {
 	constexpr int NF = Flux_Rows<SOLVER>::N;
-	using T = Tile<TY, NF>;
+	using T = Tile<TY, ZACT, NF>;
 	double* const rec_base = smem;
-	double* const fx = smem + 2 * T::REC;        // [NF][TY][TX + 1]
+	double* const fx = smem + T::SLOTS * T::REC; // [NF][TY][TX + 1]
 	double* const fy = fx + NF * T::FXN;         // [NF][TY + 1][TX]
 	uint8_t* const bad_base = reinterpret_cast<uint8_t*>(fy + NF * T::FYN);
 
 	constexpr bool YACT = TY > 1;
-	const bool zact = P.active[2] != 0;
 	const int nx = P.L.n[0], ny = P.L.n[1];
 	const int tx = threadIdx.x, ty = threadIdx.y;
 	const int warp = ty, lane = tx;  // TX = 32: one warp per tile row
@@ -532,34 +564,22 @@ __device__ __forceinline__ void tile_step(const Step_Params& P, double* const sm
 	// the planes of this block
 	int kb, ke;
 	tile_planes(P, bz, kb, ke);
-	const int kfirst = zact ? kb - 1 : kb;
-	const int klast = zact ? ke : ke - 1;
+	const int kfirst = ZACT ? kb - 1 : kb;
+	const int klast = ZACT ? ke : ke - 1;
 	const int ri = (ty + T::JO) * T::W + tx + 1;
 	// the flux terms are dt F / dx: dt / dx once per axis and cell
 	const double cx = dt * P.inv_len[0], cy = dt * P.inv_len[1], cz = dt * P.inv_len[2];
 
-	// the cell below the current plane: its state plus its x and y flux differences plus the
-	// flux of its -z face, all scaled; its +z face completes it
-	double Acc[8];
-	#pragma unroll
-	for (int v = 0; v < 8; v++) Acc[v] = 0.0;
-	// the own column's fast speed along z in the previous and the current plane
-	double cfz_prev = 0.0, cfz = 0.0;
-
-	for (int k = kfirst; k <= klast; k++) {
-		const int slot = (k - kfirst) & 1;
+	// a plane's records: own cells, and the halo for planes with x / y faces, spread over warps: the
+	// rows below / above the tile on warps 0 and 1, the columns left / right of it on warp 2 (warp 0
+	// when y is inactive).  Returns the own column's fast speed along z.
+	const auto stage_plane = [&](const int k) -> double {
+		const int slot = ZACT ? (k - kfirst) & 1 : 0;
 		double* const rec = rec_base + slot * T::REC;
 		uint8_t* const bad = bad_base + slot * T::CELLS;
-		const double* const prev = rec_base + (slot ^ 1) * T::REC;
-		const uint8_t* const prev_bad = bad_base + (slot ^ 1) * T::CELLS;
-		const bool inner = k >= kb and k < ke;
-
-		// (a) stage the plane: own cells, and the halo for planes with x / y faces
-		cfz_prev = cfz;
-		if (stage) cfz = load_record<true, YACT, true, CO>(P, rec, bad, T::CELLS, ri, gx, gy, k);
-		// halo, spread over warps: the rows below / above the tile on warps 0 and 1, the columns
-		// left / right of it on warp 2 (warp 0 when y is inactive)
-		if (inner) {
+		double cfz = 0.0;
+		if (stage) cfz = load_record<true, YACT, ZACT, CO>(P, rec, bad, T::CELLS, ri, gx, gy, k);
+		if (k >= kb and k < ke) {
 			if (YACT and warp < 2) {
 				const bool top = warp == 1;
 				const int hy = top ? gy0 + TY : gy0 - 1;
@@ -577,11 +597,29 @@ __device__ __forceinline__ void tile_step(const Step_Params& P, double* const sm
 				}
 			}
 		}
-		__syncthreads();
+		return cfz;
+	};
 
-		// (b) x and y faces: every thread its -x and -y face; the tile's last column and row also
-		// need their +x / +y faces, taken by one warp each in a further pass of the same loop
+	// the scaled flux of the -z face of the own cell of plane k
+	double low[8];
+	#pragma unroll
+	for (int v = 0; v < 8; v++) low[v] = 0.0;
+	// the own column's fast speed along z in plane k
+	double cfz = 0.0;
+
+	#pragma unroll 1
+	for (int k = kfirst - 1; k < ke; k++) {
+		const int slot = ZACT ? (k - kfirst) & 1 : 0;
+		double* const rec = rec_base + slot * T::REC;
+		uint8_t* const bad = bad_base + slot * T::CELLS;
+		double* const next = rec_base + (slot ^ 1) * T::REC;
+		uint8_t* const next_bad = bad_base + (slot ^ 1) * T::CELLS;
+		const bool inner = k >= kb;
+
 		if (inner) {
+			__syncthreads();
+			// (b) x and y faces: every thread its -x and -y face; the tile's last column and row also
+			// need their +x / +y faces, taken by one warp each in a further pass of the same loop
 			#pragma unroll 1
 			for (int task = 0; task < 4; task++) {
 				// 0: own -x face, 1: own -y face, 2: the tile's +x faces, 3: its +y faces
@@ -614,67 +652,68 @@ __device__ __forceinline__ void tile_step(const Step_Params& P, double* const sm
 					                           idx, s0, s1, zero, i, j, k);
 				}
 			}
+			if (ZACT) bar.arrive();
+			else __syncthreads();
 		}
-		// the z face between the previous plane and this one, by the column's owner; it completes
-		// the cell below (U += (F- - F+) dt/dx, then y, then z: solve.hpp:1551-1587)
-		if (zact and k > kfirst and own) {
-			double Fz[8];
-			solve_z<SOLVER, T::CELLS>(P, prev, prev_bad, rec, bad, ri, cfz_prev, cfz, Fz, s2, zero, gx, gy, k - 1);
-			if (k > kb) {
-				#pragma unroll
-				for (int v = 0; v < 8; v++) Acc[v] = Acc[v] - Fz[v] * cz;
-				write_cell(P, gx, gy, k - 1, Acc, dt);
-			}
+		// (c) the next plane's records (their slot's plane k - 1 was last read before this plane's
+		// barrier, but for own cells), and the z face between the planes
+		const double cfz_below = cfz;
+		if (k < klast) cfz = stage_plane(k + 1);
+		double high[8];
+		#pragma unroll
+		for (int v = 0; v < 8; v++) high[v] = 0.0;
+		if (ZACT and k >= kfirst and own) {
+			solve_z<SOLVER, T::CELLS>(P, rec, bad, next, next_bad, ri, cfz_below, cfz, high, s2, zero, gx, gy, k);
 			#pragma unroll
-			for (int v = 0; v < 8; v++) Acc[v] = Fz[v] * cz;
+			for (int v = 0; v < 8; v++) high[v] = __dmul_rn(high[v], cz);
 		}
-		__syncthreads();
-
-		// (c) the own cell: state plus x and y flux differences (plus its -z flux, held in Acc)
-		if (own and inner) {
-			// the flux row of each xyz variable in the x and the y face frames; -1: the normal
-			// field component, whose flux is zero unless the solver keeps an eighth row (adding
-			// 0.0 keeps the bits of adding a zero flux difference)
-			constexpr int XROW[8] = {0, 1, 2, 3, 4, NF == 8 ? 7 : -1, 5, 6};
-			constexpr int YROW[8] = {0, 3, 1, 2, 4, 6, NF == 8 ? 7 : -1, 5};
-			double Un[8];
-			#pragma unroll
-			for (int v = 0; v < 8; v++) {
-				const double u = rec[v * T::CELLS + ri];
-				if (XROW[v] >= 0) {
-					const double* f = fx + XROW[v] * T::FXN + ty * (TX + 1) + tx;
-					Un[v] = u + (f[0] - f[1]) * cx;
-				} else {
-					Un[v] = u + 0.0;
-				}
-			}
-			if (YACT) {
+		// (d) the own cell: U += (F- - F+) dt/dx, then y, then z (solve.hpp:1551-1587)
+		if (inner) {
+			if (ZACT and not bar.wait(P.status)) return;
+			if (own) {
+				// the flux row of each xyz variable in the x and the y face frames; -1: the normal
+				// field component, whose flux is zero unless the solver keeps an eighth row
+				constexpr int XROW[8] = {0, 1, 2, 3, 4, NF == 8 ? 7 : -1, 5, 6};
+				constexpr int YROW[8] = {0, 3, 1, 2, 4, 6, NF == 8 ? 7 : -1, 5};
+				double Un[8];
 				#pragma unroll
 				for (int v = 0; v < 8; v++) {
-					if (YROW[v] >= 0) {
-						const double* f = fy + YROW[v] * T::FYN + ty * TX + tx;
-						Un[v] += (f[0] - f[TX]) * cy;
-					} else {
-						Un[v] += 0.0;
+					Un[v] = rec[v * T::CELLS + ri];
+					if (XROW[v] >= 0) {
+						const double* f = fx + XROW[v] * T::FXN + ty * (TX + 1) + tx;
+						Un[v] = __fma_rn(__dsub_rn(f[0], f[1]), cx, Un[v]);
 					}
 				}
-			}
-			if (zact) {
-				#pragma unroll
-				for (int v = 0; v < 8; v++) Acc[v] = Un[v] + Acc[v];
-			} else {
+				if (YACT) {
+					#pragma unroll
+					for (int v = 0; v < 8; v++) {
+						if (YROW[v] >= 0) {
+							const double* f = fy + YROW[v] * T::FYN + ty * TX + tx;
+							Un[v] = __fma_rn(__dsub_rn(f[0], f[TX]), cy, Un[v]);
+						}
+					}
+				}
+				if (ZACT) {
+					#pragma unroll
+					for (int v = 0; v < 8; v++) Un[v] = __dadd_rn(Un[v], __dsub_rn(low[v], high[v]));
+				}
 				write_cell(P, gx, gy, k, Un, dt);
 			}
 		}
+		#pragma unroll
+		for (int v = 0; v < 8; v++) low[v] = high[v];
 	}
 }
 
-template <int SOLVER, int TY, int MINB>
-__global__ void __launch_bounds__(TX * TY, MINB) step_kernel(const Step_Params P)
+template <int SOLVER, int TY, bool ZACT>
+__global__ void __launch_bounds__(TX * TY, Resident<TY, ZACT>::blocks) step_kernel(const Step_Params P)
 {
 	extern __shared__ __align__(16) double smem[];
 	__shared__ double s_dt;
 	__shared__ int s_stop;
+	__shared__ unsigned long long s_bar;
+	Split_Barrier bar = split_barrier(&s_bar);
+	if (threadIdx.x == 0 and threadIdx.y == 0) bar.init(TY);
 	const bool first_block = blockIdx.x == 0 and blockIdx.y == 0 and blockIdx.z == 0;
 	const double dt = begin_step(P, &s_dt, first_block, &s_stop);
 	if (s_stop) {
@@ -683,7 +722,7 @@ __global__ void __launch_bounds__(TX * TY, MINB) step_kernel(const Step_Params P
 	}
 	double s0 = 0.0, s1 = 0.0, s2 = 0.0;
 	bool zero = false;
-	tile_step<SOLVER, TY>(P, smem, dt, blockIdx.x, blockIdx.y, blockIdx.z, s0, s1, s2, zero);
+	tile_step<SOLVER, TY, ZACT>(P, smem, bar, dt, blockIdx.x, blockIdx.y, blockIdx.z, s0, s1, s2, zero);
 	double smax[3] = {s0, s1, s2};
 	flush_speeds(P, smax, zero);
 }
@@ -695,8 +734,8 @@ stride; each box has its own parameters (state buffers, layout, boundary
 kinds, reduction ring, clock, status), so each advances with its own dt.
 The block holding a box's first item advances that box's clock.
 */
-template <int SOLVER, int TY, int MINB>
-__global__ void __launch_bounds__(TX * TY, MINB) batch_step_kernel(const Step_Params* __restrict__ boxes,
+template <int SOLVER, int TY, bool ZACT>
+__global__ void __launch_bounds__(TX * TY, Resident<TY, ZACT>::blocks) batch_step_kernel(const Step_Params* __restrict__ boxes,
                                                                   const int4* __restrict__ items,
                                                                   const int nitems, const int phase)
 {
@@ -704,7 +743,10 @@ __global__ void __launch_bounds__(TX * TY, MINB) batch_step_kernel(const Step_Pa
 	__shared__ Step_Params sp;
 	__shared__ double s_dt;
 	__shared__ int s_stop;
+	__shared__ unsigned long long s_bar;
 	const int tid = threadIdx.y * blockDim.x + threadIdx.x;
+	Split_Barrier bar = split_barrier(&s_bar);
+	if (tid == 0) bar.init(TY);
 	for (int item = blockIdx.x; item < nitems; item += gridDim.x) {
 		const int4 w = items[item];
 		__syncthreads();  // the previous item is done with sp
@@ -722,7 +764,7 @@ __global__ void __launch_bounds__(TX * TY, MINB) batch_step_kernel(const Step_Pa
 		}
 		double s0 = 0.0, s1 = 0.0, s2 = 0.0;
 		bool zero = false;
-		tile_step<SOLVER, TY>(sp, smem, dt, w.y % tiles_x, w.y / tiles_x, w.z, s0, s1, s2, zero);
+		tile_step<SOLVER, TY, ZACT>(sp, smem, bar, dt, w.y % tiles_x, w.y / tiles_x, w.z, s0, s1, s2, zero);
 		double smax[3] = {s0, s1, s2};
 		flush_speeds(sp, smax, zero);
 	}
@@ -948,8 +990,8 @@ box, and every block stops at its next item.  boxes_even / boxes_odd are
 the boxes' parameters of the two state parities, the first used by step
 step0.  Loads that read what another block wrote before go through L2 (CO).
 */
-template <int SOLVER, int TY, int MINB>
-__global__ void __launch_bounds__(TX * TY, MINB) batch_run_kernel(
+template <int SOLVER, int TY, bool ZACT>
+__global__ void __launch_bounds__(TX * TY, Resident<TY, ZACT>::blocks) batch_run_kernel(
 	const Step_Params* __restrict__ boxes_even, const Step_Params* __restrict__ boxes_odd,
 	const int4* __restrict__ items, const int nitems, const int* __restrict__ box_items, unsigned int* done,
 	const int nboxes, const long long step0, const int nsteps, Run_Sync* sync, const long long wait_limit)
@@ -960,7 +1002,10 @@ __global__ void __launch_bounds__(TX * TY, MINB) batch_run_kernel(
 	__shared__ unsigned int s_q;
 	__shared__ int s_go;
 	__shared__ int s_stop;
+	__shared__ unsigned long long s_bar;
 	const int tid = threadIdx.y * blockDim.x + threadIdx.x;
+	Split_Barrier bar = split_barrier(&s_bar);
+	if (tid == 0) bar.init(TY);
 	const int nthreads = blockDim.x * blockDim.y;
 	const unsigned int total = (unsigned int)nsteps * (unsigned int)nitems;
 	for (;;) {
@@ -1011,7 +1056,7 @@ __global__ void __launch_bounds__(TX * TY, MINB) batch_run_kernel(
 			if (s_stop) {
 				tile_hold<TY, true>(sp, w.y % tiles_x, w.y / tiles_x, w.z);
 			} else {
-				tile_step<SOLVER, TY, true>(sp, smem, dt, w.y % tiles_x, w.y / tiles_x, w.z, smax[0], smax[1],
+				tile_step<SOLVER, TY, ZACT, true>(sp, smem, bar, dt, w.y % tiles_x, w.y / tiles_x, w.z, smax[0], smax[1],
 				                            smax[2], zero);
 			}
 		} else if (not stopped_before(sp)) {
@@ -1137,267 +1182,146 @@ __global__ void totals_kernel(const double* __restrict__ state, const Layout L, 
 
 // ------------------------------------------------------------------ launchers
 
-template <int SOLVER, int TY>
-static int prepare_t()
+/*
+Calls body(solver, rows, zact) with the values of kind as integral
+constants: the solver, the tile rows (1 where y is inactive) and whether
+there are z faces (only with y active).
+*/
+template <int N> using Const = std::integral_constant<int, N>;
+
+template <int SOLVER, class Body> static int with_rows(const Tile_Kind& kind, const Body& body)
 {
-	const auto kernel = step_kernel<SOLVER, TY, Step_Minb<SOLVER, TY>::value>;
-	cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-	                                     int(tile_bytes<SOLVER, TY>()));
-	// all of the SM's memory as shared memory, so that the blocks the registers allow fit
-	if (e == cudaSuccess) e = cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
-	return e == cudaSuccess ? PAMHD_OK : PAMHD_ERR_CUDA;
+	if (kind.rows == 1 and not kind.zact) return body(Const<SOLVER>{}, Const<1>{}, std::false_type{});
+	if (kind.rows == TY_3D) {
+		return kind.zact ? body(Const<SOLVER>{}, Const<TY_3D>{}, std::true_type{})
+		                 : body(Const<SOLVER>{}, Const<TY_3D>{}, std::false_type{});
+	}
+	if (kind.rows == TY_WIDE) {
+		return kind.zact ? body(Const<SOLVER>{}, Const<TY_WIDE>{}, std::true_type{})
+		                 : body(Const<SOLVER>{}, Const<TY_WIDE>{}, std::false_type{});
+	}
+	return PAMHD_ERR_ARGUMENT;
 }
 
-int prepare_step_kernels(const int solver, const bool y)
+template <class Body> static int with_kind(const Tile_Kind& kind, const Body& body)
 {
-	switch (solver) {
-	case PAMHD_RUSANOV: return y ? prepare_t<PAMHD_RUSANOV, Step_Shape<PAMHD_RUSANOV>::rows>() : prepare_t<PAMHD_RUSANOV, 1>();
-	case PAMHD_HLL_ATHENA: return y ? prepare_t<PAMHD_HLL_ATHENA, Step_Shape<PAMHD_HLL_ATHENA>::rows>() : prepare_t<PAMHD_HLL_ATHENA, 1>();
-	case PAMHD_HLLD_ATHENA: return y ? prepare_t<PAMHD_HLLD_ATHENA, Step_Shape<PAMHD_HLLD_ATHENA>::rows>() : prepare_t<PAMHD_HLLD_ATHENA, 1>();
-	case PAMHD_ROE_ATHENA: return y ? prepare_t<PAMHD_ROE_ATHENA, Step_Shape<PAMHD_ROE_ATHENA>::rows>() : prepare_t<PAMHD_ROE_ATHENA, 1>();
+	switch (kind.solver) {
+	case PAMHD_RUSANOV: return with_rows<PAMHD_RUSANOV>(kind, body);
+	case PAMHD_HLL_ATHENA: return with_rows<PAMHD_HLL_ATHENA>(kind, body);
+	case PAMHD_HLLD_ATHENA: return with_rows<PAMHD_HLLD_ATHENA>(kind, body);
+	case PAMHD_ROE_ATHENA: return with_rows<PAMHD_ROE_ATHENA>(kind, body);
 	default: return PAMHD_ERR_ARGUMENT;
 	}
 }
 
-template <int SOLVER, int TY>
-static int launch_step_t(const Step_Params& P, cudaStream_t stream)
+static int status_of(const cudaError_t e)
 {
-	const size_t smem = tile_bytes<SOLVER, TY>();
-	const dim3 block(TX, TY);
+	return e == cudaSuccess ? PAMHD_OK : PAMHD_ERR_CUDA;
+}
+
+/*
+The single-grid step's tile: 32 x 8, two blocks of 256 threads per SM (a
+taller tile solves fewer halo faces and records per cell); Roe's solver
+needs more registers, so it keeps 32 x 4 tiles at three blocks per SM.
+*/
+Tile_Kind step_tile(const int solver, const bool yact, const bool zact)
+{
+	return Tile_Kind{solver, not yact ? 1 : (solver == PAMHD_ROE_ATHENA ? TY_3D : TY_WIDE), zact};
+}
+
+int prepare_step_kernels(const Tile_Kind& kind)
+{
+	return with_kind(kind, [](auto solver, auto rows, auto zact) {
+		const auto kernel = step_kernel<solver(), rows(), zact()>;
+		cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+		                                     int(tile_bytes<solver(), rows(), zact()>()));
+		// all of the SM's memory as shared memory, so that the blocks the registers allow fit
+		if (e == cudaSuccess) e = cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
+		return status_of(e);
+	});
+}
+
+int launch_step(const Step_Params& P, const int solver, cudaStream_t stream)
+{
 	const int nz = P.L.n[2];
 	const int chunks = P.kpart == 1 ? (nz > 1 ? 2 : 1)
 	                 : P.kpart == 2 ? (nz - 2 + P.kchunk - 1) / P.kchunk
 	                 : (nz + P.kchunk - 1) / P.kchunk;
 	if (chunks < 1) return PAMHD_OK;  // no planes between the first and the last
-	const dim3 grid((P.L.n[0] + TX - 1) / TX, (P.L.n[1] + TY - 1) / TY, chunks);
-	step_kernel<SOLVER, TY, Step_Minb<SOLVER, TY>::value><<<grid, block, smem, stream>>>(P);
-	return cudaGetLastError() == cudaSuccess ? PAMHD_OK : PAMHD_ERR_CUDA;
+	return with_kind(step_tile(solver, P.active[1] != 0, P.active[2] != 0), [&](auto solver_, auto rows, auto zact) {
+		const dim3 grid((P.L.n[0] + TX - 1) / TX, (P.L.n[1] + rows() - 1) / rows(), chunks);
+		step_kernel<solver_(), rows(), zact()>
+			<<<grid, dim3(TX, rows()), tile_bytes<solver_(), rows(), zact()>(), stream>>>(P);
+		return status_of(cudaGetLastError());
+	});
 }
 
-int launch_step(const Step_Params& P, const int solver, cudaStream_t stream)
+int prepare_batch_kernels(const Tile_Kind& kind)
 {
-	const bool y = P.active[1] != 0;
-	switch (solver) {
-	case PAMHD_RUSANOV: return y ? launch_step_t<PAMHD_RUSANOV, Step_Shape<PAMHD_RUSANOV>::rows>(P, stream) : launch_step_t<PAMHD_RUSANOV, 1>(P, stream);
-	case PAMHD_HLL_ATHENA: return y ? launch_step_t<PAMHD_HLL_ATHENA, Step_Shape<PAMHD_HLL_ATHENA>::rows>(P, stream) : launch_step_t<PAMHD_HLL_ATHENA, 1>(P, stream);
-	case PAMHD_HLLD_ATHENA: return y ? launch_step_t<PAMHD_HLLD_ATHENA, Step_Shape<PAMHD_HLLD_ATHENA>::rows>(P, stream) : launch_step_t<PAMHD_HLLD_ATHENA, 1>(P, stream);
-	case PAMHD_ROE_ATHENA: return y ? launch_step_t<PAMHD_ROE_ATHENA, Step_Shape<PAMHD_ROE_ATHENA>::rows>(P, stream) : launch_step_t<PAMHD_ROE_ATHENA, 1>(P, stream);
-	default: return PAMHD_ERR_ARGUMENT;
-	}
+	return with_kind(kind, [](auto solver, auto rows, auto zact) {
+		return status_of(cudaFuncSetAttribute(batch_step_kernel<solver(), rows(), zact()>,
+		                                      cudaFuncAttributeMaxDynamicSharedMemorySize,
+		                                      int(tile_bytes<solver(), rows(), zact()>())));
+	});
 }
 
-// tile rows the batched step is built for (the autotuner picks one): 1 when y is inactive
-constexpr int TY_WIDE = 8;
-constexpr int MINB_WIDE = 2;   // resident blocks per SM of the 32 x 8 tile
-
-template <int TY> struct Batch_Build { static constexpr int MINB_OF = MINB; };
-template <> struct Batch_Build<TY_WIDE> { static constexpr int MINB_OF = MINB_WIDE; };
-
-template <int SOLVER, int TY>
-static int prepare_batch_t()
+int batch_blocks_per_sm(const Tile_Kind& kind, int* blocks)
 {
-	const cudaError_t e = cudaFuncSetAttribute(batch_step_kernel<SOLVER, TY, Batch_Build<TY>::MINB_OF>,
-	                                           cudaFuncAttributeMaxDynamicSharedMemorySize, int(tile_bytes<SOLVER, TY>()));
-	return e == cudaSuccess ? PAMHD_OK : PAMHD_ERR_CUDA;
+	return with_kind(kind, [&](auto solver, auto rows, auto zact) {
+		return status_of(cudaOccupancyMaxActiveBlocksPerMultiprocessor(
+			blocks, batch_step_kernel<solver(), rows(), zact()>, TX * rows(),
+			tile_bytes<solver(), rows(), zact()>()));
+	});
 }
 
-template <int SOLVER>
-static int prepare_batch_s(const int ty)
+int prepare_batch_run_kernels(const Tile_Kind& kind)
 {
-	switch (ty) {
-	case 1: return prepare_batch_t<SOLVER, 1>();
-	case TY_3D: return prepare_batch_t<SOLVER, TY_3D>();
-	case TY_WIDE: return prepare_batch_t<SOLVER, TY_WIDE>();
-	default: return PAMHD_ERR_ARGUMENT;
-	}
+	return with_kind(kind, [](auto solver, auto rows, auto zact) {
+		return status_of(cudaFuncSetAttribute(batch_run_kernel<solver(), rows(), zact()>,
+		                                      cudaFuncAttributeMaxDynamicSharedMemorySize,
+		                                      int(tile_bytes<solver(), rows(), zact()>())));
+	});
 }
 
-int prepare_batch_kernels(const int solver, const int ty)
+int batch_run_blocks_per_sm(const Tile_Kind& kind, int* blocks)
 {
-	switch (solver) {
-	case PAMHD_RUSANOV: return prepare_batch_s<PAMHD_RUSANOV>(ty);
-	case PAMHD_HLL_ATHENA: return prepare_batch_s<PAMHD_HLL_ATHENA>(ty);
-	case PAMHD_HLLD_ATHENA: return prepare_batch_s<PAMHD_HLLD_ATHENA>(ty);
-	case PAMHD_ROE_ATHENA: return prepare_batch_s<PAMHD_ROE_ATHENA>(ty);
-	default: return PAMHD_ERR_ARGUMENT;
-	}
-}
-
-template <int SOLVER, int TY>
-static cudaError_t occupancy_t(int* blocks)
-{
-	return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks, batch_step_kernel<SOLVER, TY, Batch_Build<TY>::MINB_OF>,
-	                                                     TX * TY, tile_bytes<SOLVER, TY>());
-}
-
-template <int SOLVER>
-static cudaError_t occupancy_s(const int ty, int* blocks)
-{
-	switch (ty) {
-	case 1: return occupancy_t<SOLVER, 1>(blocks);
-	case TY_3D: return occupancy_t<SOLVER, TY_3D>(blocks);
-	case TY_WIDE: return occupancy_t<SOLVER, TY_WIDE>(blocks);
-	default: return cudaErrorInvalidValue;
-	}
-}
-
-int batch_blocks_per_sm(const int solver, const int ty, int* blocks)
-{
-	cudaError_t e = cudaErrorInvalidValue;
-	switch (solver) {
-	case PAMHD_RUSANOV: e = occupancy_s<PAMHD_RUSANOV>(ty, blocks); break;
-	case PAMHD_HLL_ATHENA: e = occupancy_s<PAMHD_HLL_ATHENA>(ty, blocks); break;
-	case PAMHD_HLLD_ATHENA: e = occupancy_s<PAMHD_HLLD_ATHENA>(ty, blocks); break;
-	case PAMHD_ROE_ATHENA: e = occupancy_s<PAMHD_ROE_ATHENA>(ty, blocks); break;
-	default: return PAMHD_ERR_ARGUMENT;
-	}
-	return e == cudaSuccess ? PAMHD_OK : PAMHD_ERR_CUDA;
-}
-
-template <int SOLVER, int TY>
-static int prepare_run_t()
-{
-	const cudaError_t e = cudaFuncSetAttribute(batch_run_kernel<SOLVER, TY, Batch_Build<TY>::MINB_OF>,
-	                                           cudaFuncAttributeMaxDynamicSharedMemorySize, int(tile_bytes<SOLVER, TY>()));
-	return e == cudaSuccess ? PAMHD_OK : PAMHD_ERR_CUDA;
-}
-
-template <int SOLVER, int TY>
-static cudaError_t run_occupancy_t(int* blocks)
-{
-	return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks, batch_run_kernel<SOLVER, TY, Batch_Build<TY>::MINB_OF>,
-	                                                     TX * TY, tile_bytes<SOLVER, TY>());
-}
-
-template <int SOLVER, int TY>
-static int launch_run_t(const Step_Params* even, const Step_Params* odd, const int4* items, const int nitems,
-                        const int* box_items, unsigned int* done, const int nboxes, const long long step0,
-                        const int nsteps, Run_Sync* sync, const long long wait_limit, const int grid,
-                        cudaStream_t stream)
-{
-	cudaLaunchConfig_t c = {};
-	c.gridDim = dim3(grid);
-	c.blockDim = dim3(TX, TY);
-	c.dynamicSmemBytes = tile_bytes<SOLVER, TY>();
-	c.stream = stream;
-	cudaLaunchAttribute a[1];
-	a[0].id = cudaLaunchAttributeCooperative;
-	a[0].val.cooperative = 1;
-	c.attrs = a;
-	c.numAttrs = 1;
-	const cudaError_t e = cudaLaunchKernelEx(&c, batch_run_kernel<SOLVER, TY, Batch_Build<TY>::MINB_OF>, even, odd,
-	                                         items, nitems, box_items, done, nboxes, step0, nsteps, sync, wait_limit);
-	return e == cudaSuccess ? PAMHD_OK : PAMHD_ERR_CUDA;
-}
-
-template <int SOLVER>
-static int prepare_run_s(const int ty)
-{
-	switch (ty) {
-	case 1: return prepare_run_t<SOLVER, 1>();
-	case TY_3D: return prepare_run_t<SOLVER, TY_3D>();
-	case TY_WIDE: return prepare_run_t<SOLVER, TY_WIDE>();
-	default: return PAMHD_ERR_ARGUMENT;
-	}
-}
-
-template <int SOLVER>
-static cudaError_t run_occupancy_s(const int ty, int* blocks)
-{
-	switch (ty) {
-	case 1: return run_occupancy_t<SOLVER, 1>(blocks);
-	case TY_3D: return run_occupancy_t<SOLVER, TY_3D>(blocks);
-	case TY_WIDE: return run_occupancy_t<SOLVER, TY_WIDE>(blocks);
-	default: return cudaErrorInvalidValue;
-	}
-}
-
-template <int SOLVER>
-static int launch_run_s(const Step_Params* even, const Step_Params* odd, const int4* items, const int nitems,
-                        const int* box_items, unsigned int* done, const int nboxes, const long long step0,
-                        const int nsteps, Run_Sync* sync, const long long wait_limit, const int grid, const int ty,
-                        cudaStream_t stream)
-{
-	switch (ty) {
-	case 1: return launch_run_t<SOLVER, 1>(even, odd, items, nitems, box_items, done, nboxes, step0, nsteps, sync, wait_limit, grid, stream);
-	case TY_3D: return launch_run_t<SOLVER, TY_3D>(even, odd, items, nitems, box_items, done, nboxes, step0, nsteps, sync, wait_limit, grid, stream);
-	case TY_WIDE: return launch_run_t<SOLVER, TY_WIDE>(even, odd, items, nitems, box_items, done, nboxes, step0, nsteps, sync, wait_limit, grid, stream);
-	default: return PAMHD_ERR_ARGUMENT;
-	}
-}
-
-int prepare_batch_run_kernels(const int solver, const int ty)
-{
-	switch (solver) {
-	case PAMHD_RUSANOV: return prepare_run_s<PAMHD_RUSANOV>(ty);
-	case PAMHD_HLL_ATHENA: return prepare_run_s<PAMHD_HLL_ATHENA>(ty);
-	case PAMHD_HLLD_ATHENA: return prepare_run_s<PAMHD_HLLD_ATHENA>(ty);
-	case PAMHD_ROE_ATHENA: return prepare_run_s<PAMHD_ROE_ATHENA>(ty);
-	default: return PAMHD_ERR_ARGUMENT;
-	}
-}
-
-int batch_run_blocks_per_sm(const int solver, const int ty, int* blocks)
-{
-	cudaError_t e = cudaErrorInvalidValue;
-	switch (solver) {
-	case PAMHD_RUSANOV: e = run_occupancy_s<PAMHD_RUSANOV>(ty, blocks); break;
-	case PAMHD_HLL_ATHENA: e = run_occupancy_s<PAMHD_HLL_ATHENA>(ty, blocks); break;
-	case PAMHD_HLLD_ATHENA: e = run_occupancy_s<PAMHD_HLLD_ATHENA>(ty, blocks); break;
-	case PAMHD_ROE_ATHENA: e = run_occupancy_s<PAMHD_ROE_ATHENA>(ty, blocks); break;
-	default: return PAMHD_ERR_ARGUMENT;
-	}
-	return e == cudaSuccess ? PAMHD_OK : PAMHD_ERR_CUDA;
+	return with_kind(kind, [&](auto solver, auto rows, auto zact) {
+		return status_of(cudaOccupancyMaxActiveBlocksPerMultiprocessor(
+			blocks, batch_run_kernel<solver(), rows(), zact()>, TX * rows(),
+			tile_bytes<solver(), rows(), zact()>()));
+	});
 }
 
 int launch_batch_run(const Step_Params* even, const Step_Params* odd, const int4* items, const int nitems,
                      const int* box_items, unsigned int* done, const int nboxes, const long long step0,
-                     const int nsteps, Run_Sync* sync, const long long wait_limit, const int grid, const int solver,
-                     const int ty, cudaStream_t stream)
+                     const int nsteps, Run_Sync* sync, const long long wait_limit, const int grid,
+                     const Tile_Kind& kind, cudaStream_t stream)
 {
-	switch (solver) {
-	case PAMHD_RUSANOV: return launch_run_s<PAMHD_RUSANOV>(even, odd, items, nitems, box_items, done, nboxes, step0, nsteps, sync, wait_limit, grid, ty, stream);
-	case PAMHD_HLL_ATHENA: return launch_run_s<PAMHD_HLL_ATHENA>(even, odd, items, nitems, box_items, done, nboxes, step0, nsteps, sync, wait_limit, grid, ty, stream);
-	case PAMHD_HLLD_ATHENA: return launch_run_s<PAMHD_HLLD_ATHENA>(even, odd, items, nitems, box_items, done, nboxes, step0, nsteps, sync, wait_limit, grid, ty, stream);
-	case PAMHD_ROE_ATHENA: return launch_run_s<PAMHD_ROE_ATHENA>(even, odd, items, nitems, box_items, done, nboxes, step0, nsteps, sync, wait_limit, grid, ty, stream);
-	default: return PAMHD_ERR_ARGUMENT;
-	}
-}
-
-template <int SOLVER, int TY>
-static void launch_batch_t(const Step_Params* boxes, const int4* items, const int nitems, const int phase,
-                           const int grid, cudaStream_t stream)
-{
-	batch_step_kernel<SOLVER, TY, Batch_Build<TY>::MINB_OF><<<grid, dim3(TX, TY), tile_bytes<SOLVER, TY>(), stream>>>(
-		boxes, items, nitems, phase);
-}
-
-template <int SOLVER>
-static int launch_batch_s(const Step_Params* boxes, const int4* items, const int nitems, const int phase,
-                          const int grid, const int ty, cudaStream_t stream)
-{
-	switch (ty) {
-	case 1: launch_batch_t<SOLVER, 1>(boxes, items, nitems, phase, grid, stream); break;
-	case TY_3D: launch_batch_t<SOLVER, TY_3D>(boxes, items, nitems, phase, grid, stream); break;
-	case TY_WIDE: launch_batch_t<SOLVER, TY_WIDE>(boxes, items, nitems, phase, grid, stream); break;
-	default: return PAMHD_ERR_ARGUMENT;
-	}
-	return PAMHD_OK;
+	return with_kind(kind, [&](auto solver, auto rows, auto zact) {
+		cudaLaunchConfig_t c = {};
+		c.gridDim = dim3(grid);
+		c.blockDim = dim3(TX, rows());
+		c.dynamicSmemBytes = tile_bytes<solver(), rows(), zact()>();
+		c.stream = stream;
+		cudaLaunchAttribute a[1];
+		a[0].id = cudaLaunchAttributeCooperative;
+		a[0].val.cooperative = 1;
+		c.attrs = a;
+		c.numAttrs = 1;
+		return status_of(cudaLaunchKernelEx(&c, batch_run_kernel<solver(), rows(), zact()>,
+		                                    even, odd, items, nitems, box_items, done, nboxes, step0, nsteps, sync,
+		                                    wait_limit));
+	});
 }
 
 int launch_batch_step(const Step_Params* boxes, const int4* items, const int nitems, const int phase,
-                      const int grid, const int solver, const int ty, cudaStream_t stream)
+                      const int grid, const Tile_Kind& kind, cudaStream_t stream)
 {
-	int rc = PAMHD_ERR_ARGUMENT;
-	switch (solver) {
-	case PAMHD_RUSANOV: rc = launch_batch_s<PAMHD_RUSANOV>(boxes, items, nitems, phase, grid, ty, stream); break;
-	case PAMHD_HLL_ATHENA: rc = launch_batch_s<PAMHD_HLL_ATHENA>(boxes, items, nitems, phase, grid, ty, stream); break;
-	case PAMHD_HLLD_ATHENA: rc = launch_batch_s<PAMHD_HLLD_ATHENA>(boxes, items, nitems, phase, grid, ty, stream); break;
-	case PAMHD_ROE_ATHENA: rc = launch_batch_s<PAMHD_ROE_ATHENA>(boxes, items, nitems, phase, grid, ty, stream); break;
-	default: return PAMHD_ERR_ARGUMENT;
-	}
-	if (rc != PAMHD_OK) return rc;
-	return cudaGetLastError() == cudaSuccess ? PAMHD_OK : PAMHD_ERR_CUDA;
+	return with_kind(kind, [&](auto solver, auto rows, auto zact) {
+		batch_step_kernel<solver(), rows(), zact()>
+			<<<grid, dim3(TX, rows()), tile_bytes<solver(), rows(), zact()>(), stream>>>(boxes, items, nitems, phase);
+		return status_of(cudaGetLastError());
+	});
 }
 
 int launch_batch_boundary_speeds(const Step_Params* boxes, const int nboxes, const int largest, const int phase,
