@@ -649,7 +649,8 @@ __device__ __forceinline__ double flux_roe(const Side& L, const Side& R, const G
 	const Rd droe = sdl * sdr, di = il * ir;
 	const Rd isqrtd = rsqrt_nr(droe), sqrtd = droe * isqrtd;
 	const Rd v1 = mad(wl, L.v0, wr * Rd(R.v0)), v2 = mad(wl, L.v1, wr * Rd(R.v1)), v3 = mad(wl, L.v2, wr * Rd(R.v2));
-	const Rd b2 = mad(wr, byl, wl * byr), b3 = mad(wr, bzl, wl * bzr);
+	// products rounded: opposite fields at equal densities average to exactly 0
+	const Rd b2 = wr * byl + wl * byr, b3 = wr * bzl + wl * bzr;
 	const Rd dby = byl - byr, dbz = bzl - bzr;
 	const Rd x = half * mad(dby, dby, dbz * dbz) * (isd * isd);
 	const Rd y = half * (Rd(L.rho) + Rd(R.rho)) * di;
