@@ -282,7 +282,7 @@ int forward_step(pamhd_ctx& x, const double dt)
 	P.out = x.state[x.cur ^ 1];
 	P.phase = int(x.steps % 3);
 	P.forced_dt = dt;
-	if (x.needs_boundary_speeds) PAMHD_TRY(launch_boundary_speeds(P, x.cfg.solver, x.stream));
+	P.boundary = x.boundary_layers;
 	PAMHD_TRY(launch_step(P, x.cfg.solver, x.stream));
 	x.cur ^= 1;
 	x.steps++;

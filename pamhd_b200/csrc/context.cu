@@ -34,7 +34,7 @@ int check(const cudaError_t e)
 
 void set_params(pamhd_ctx& x)
 {
-	x.needs_boundary_speeds = grid_params(x.cfg, x.L, x.base);
+	x.boundary_layers = grid_params(x.cfg, x.L, x.base) ? boundary_layers(x.base, x.cfg.solver) : 0;
 	Step_Params& P = x.base;
 	P.red = x.red;
 	P.clock = x.clock;
@@ -55,8 +55,8 @@ Step_Params params_for(const pamhd_ctx& x, const long long step, const int cur)
 
 int issue_step(pamhd_ctx& x)
 {
-	const Step_Params P = params_for(x, x.steps, x.cur);
-	if (x.needs_boundary_speeds) PAMHD_TRY(launch_boundary_speeds(P, x.cfg.solver, x.stream));
+	Step_Params P = params_for(x, x.steps, x.cur);
+	P.boundary = x.boundary_layers;
 	PAMHD_TRY(launch_step(P, x.cfg.solver, x.stream));
 	x.cur ^= 1;
 	x.steps++;
@@ -69,7 +69,7 @@ int issue_step_part(pamhd_ctx& x, const int part)
 {
 	Step_Params P = params_for(x, x.steps, x.cur);
 	P.kpart = part;
-	if (part == 1 and x.needs_boundary_speeds) PAMHD_TRY(launch_boundary_speeds(P, x.cfg.solver, x.stream));
+	P.boundary = part == 1 ? x.boundary_layers : 0;
 	PAMHD_TRY(launch_step(P, x.cfg.solver, x.stream));
 	if (part == 2) {
 		x.cur ^= 1;

@@ -37,7 +37,7 @@ struct pamhd_ctx {
 	double* staging = nullptr;
 	double* partial = nullptr;
 	int partial_blocks = 296;
-	bool needs_boundary_speeds = false;
+	int boundary_layers = 0;   // block layers of the step that solve ghost-ghost faces
 	cudaGraphExec_t graph = nullptr;
 	bool loaded = false;
 	Adjoint_Work* adjoint = nullptr;  // adjoint workspace, kept between pamhd_gpu_adjoint calls

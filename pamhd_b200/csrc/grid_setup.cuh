@@ -12,10 +12,6 @@ constant part of its step parameters.
 
 #include "step.cuh"
 
-#ifndef PAMHD_CHUNK_BLOCKS
-#define PAMHD_CHUNK_BLOCKS 4736   // blocks of a step the z chunking aims at: 32 per SM
-#endif
-
 namespace pamhd_b200 {
 
 inline int validate(const pamhd_cfg& c)
@@ -118,6 +114,35 @@ inline Layout make_layout(const pamhd_cfg& c)
 }
 
 /*
+z planes per block of a step: the chunk length with the shortest estimated
+step.  A block of kc planes takes about kc + 1 plane times (the planes
+before and after the chunk, and the block's start and end); 148 SMs run
+`resident` blocks each, and a wave with fewer blocks per SM is shorter,
+since the blocks of an SM share its FP64 pipe: two side by side take 1.6
+times as long as one alone.  Grids of many waves keep the 16 planes of
+before (256^3: 4096 blocks); smaller ones get shorter chunks that fill the
+SMs, e.g. 96 x 64 x 50 cells 240 blocks of 5 planes instead of 72 of 17.
+*/
+inline int planes_per_block(const long long tiles, const int nz, const int resident)
+{
+	constexpr int SMS = 148;
+	const auto wave = [&](const long long per_sm) { return (1.0 + 0.6 * (per_sm - 1)) / (1.0 + 0.6 * (resident - 1)); };
+	int best = nz;
+	double shortest = 1e300;
+	for (int c = 1; c <= std::min(nz, 4096); c++) {
+		const int kc = (nz + c - 1) / c;
+		const long long blocks = tiles * ((nz + kc - 1) / kc);
+		const long long full = blocks / (SMS * resident), rest = blocks % (SMS * resident);
+		const double time = (full + (rest > 0 ? wave((rest + SMS - 1) / SMS) : 0.0)) * (kc + 1);
+		if (time < shortest) {
+			shortest = time;
+			best = kc;
+		}
+	}
+	return best;
+}
+
+/*
 Constant step parameters of one grid; the buffers (state, reduction ring,
 clock, status, control, dt history) are filled in by the caller.  Returns
 whether the grid needs the boundary-layer speed pass (a non-periodic
@@ -150,12 +175,9 @@ inline bool grid_params(const pamhd_cfg& c, const Layout& L, Step_Params& P, con
 		const bool own_side = c.bc_lo[d] != PAMHD_BC_EXTERNAL or c.bc_hi[d] != PAMHD_BC_EXTERNAL;
 		if (P.active[d] and not P.periodic[d] and own_side and active_count > 1) needs_boundary_speeds = true;
 	}
-	// z planes per block: enough blocks for several waves on 148 SMs, few redundant z faces
-	const int ty = step_tile(c.solver, P.active[1], P.active[2]).rows;
-	const long long tiles = (long long)((c.n[0] + 31) / 32) * ((c.n[1] + ty - 1) / ty);
-	long long chunks = (PAMHD_CHUNK_BLOCKS + tiles - 1) / tiles;
-	chunks = std::max(1LL, std::min(chunks, (long long)std::max(1, c.n[2] / 16)));
-	P.kchunk = int((c.n[2] + chunks - 1) / chunks);
+	const Tile_Kind kind = step_tile(c.solver, P.active[1], P.active[2]);
+	const long long tiles = (long long)((c.n[0] + 31) / 32) * ((c.n[1] + kind.rows - 1) / kind.rows);
+	P.kchunk = planes_per_block(tiles, c.n[2], kind.resident());
 	if (kchunk_cap > 0) P.kchunk = std::min(P.kchunk, kchunk_cap);
 	return needs_boundary_speeds;
 }

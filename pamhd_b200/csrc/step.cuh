@@ -107,6 +107,7 @@ struct Step_Params {
 	int kchunk;          // z planes per block
 	double forced_dt;    // >= 0: the step's dt (a prescribed schedule); < 0: the CFL rule
 	int kpart;           // z planes a launch computes: 0 all, 1 the first and last only, 2 the others
+	int boundary;        // block layers of the step's launch that solve ghost-ghost faces (0: none)
 	const Inflow_Table* inflow;  // [3][2] by dimension and side (lo, hi) in device memory, or nullptr
 };
 
@@ -115,11 +116,16 @@ struct Tile_Kind {
 	int solver;
 	int rows;
 	bool zact;
+	// resident blocks per SM asked of the register allocator: 16 warps of at most 128 registers with
+	// 32 x 8 tiles, 12 warps of at most 168 with 32 x 4 (and one-row) tiles
+	static constexpr int resident_of(const int rows) { return rows == 8 ? 2 : 3; }
+	int resident() const { return resident_of(rows); }
 };
 
 // launchers (step_kernels.cu)
 int launch_step(const Step_Params& P, int solver, cudaStream_t stream);
-int launch_boundary_speeds(const Step_Params& P, int solver, cudaStream_t stream);
+// block layers for the ghost-ghost faces of a grid with non-periodic sides (Step_Params::boundary)
+int boundary_layers(const Step_Params& P, int solver);
 int launch_scatter(const double* packed, double* var_base, const Layout& L, cudaStream_t stream);
 int launch_gather(const double* var_base, double* packed, const Layout& L, cudaStream_t stream);
 int launch_fill_ghosts_values(const Step_Params& P, double* state, const double lo[3][8], const double hi[3][8],

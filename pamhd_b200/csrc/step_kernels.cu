@@ -36,13 +36,9 @@ constexpr int TX = 32;
 constexpr int TY_3D = 4;     // the smaller tile: 32 x 4
 constexpr int TY_WIDE = 8;   // the larger: 32 x 8
 
-// resident blocks per SM asked of the register allocator: 16 warps of at most 128 registers with
-// 32 x 8 tiles, 12 warps of at most 168 with 32 x 4 (and one-row) tiles
-template <int TY, bool ZACT> struct Resident { static constexpr int blocks = TY == TY_WIDE ? 2 : 3; };
-
 // record of a cell in shared memory: rho, mom xyz, E, B xyz, 1/rho, thermal plus magnetic
-// pressure, cf x, cf y (the fast
-// speed along z is needed by the column's owner only, which keeps it in a register)
+// pressure, cf x, cf y (the fast speed along z is needed by the column's owner only, which keeps
+// it in a register)
 constexpr int NV = 12;
 enum { R_RINV = 8, R_PT = 9, R_CF = 10 };
 
@@ -705,28 +701,6 @@ __device__ __forceinline__ void tile_step(const Step_Params& P, double* const sm
 	}
 }
 
-template <int SOLVER, int TY, bool ZACT>
-__global__ void __launch_bounds__(TX * TY, Resident<TY, ZACT>::blocks) step_kernel(const Step_Params P)
-{
-	extern __shared__ __align__(16) double smem[];
-	__shared__ double s_dt;
-	__shared__ int s_stop;
-	__shared__ unsigned long long s_bar;
-	Split_Barrier bar = split_barrier(&s_bar);
-	if (threadIdx.x == 0 and threadIdx.y == 0) bar.init(TY);
-	const bool first_block = blockIdx.x == 0 and blockIdx.y == 0 and blockIdx.z == 0;
-	const double dt = begin_step(P, &s_dt, first_block, &s_stop);
-	if (s_stop) {
-		tile_hold<TY, false>(P, blockIdx.x, blockIdx.y, blockIdx.z);
-		return;
-	}
-	double s0 = 0.0, s1 = 0.0, s2 = 0.0;
-	bool zero = false;
-	tile_step<SOLVER, TY, ZACT>(P, smem, bar, dt, blockIdx.x, blockIdx.y, blockIdx.z, s0, s1, s2, zero);
-	double smax[3] = {s0, s1, s2};
-	flush_speeds(P, smax, zero);
-}
-
 /*
 The batched step: every box of an ensemble advances one step in one launch.
 Blocks walk the work-item table (box, tile x, tile y, z chunk) with a grid
@@ -735,7 +709,7 @@ kinds, reduction ring, clock, status), so each advances with its own dt.
 The block holding a box's first item advances that box's clock.
 */
 template <int SOLVER, int TY, bool ZACT>
-__global__ void __launch_bounds__(TX * TY, Resident<TY, ZACT>::blocks) batch_step_kernel(const Step_Params* __restrict__ boxes,
+__global__ void __launch_bounds__(TX * TY, Tile_Kind::resident_of(TY)) batch_step_kernel(const Step_Params* __restrict__ boxes,
                                                                   const int4* __restrict__ items,
                                                                   const int nitems, const int phase)
 {
@@ -846,48 +820,81 @@ __device__ __forceinline__ void boundary_face(const Step_Params& P, const int d,
 
 /*
 Speeds of the faces between two boundary ghosts of a non-periodic side
-(cells of class 0 on both sides).  The reference solves those faces too
-(mhd/solve.hpp:254-311 visits every cell of class >= 0) and their speeds
-enter the timestep (:1965-2005); their fluxes change nothing.
-blockIdx.y enumerates (ghost dimension d, side, tangential axis e).
+(cells of class 0 on both sides), by threads first, first + stride, ...
+The reference solves those faces too (mhd/solve.hpp:254-311 visits every
+cell of class >= 0) and their speeds enter the timestep (:1965-2005); their
+fluxes change nothing.
 */
-template <int SOLVER>
-__device__ __forceinline__ void boundary_speeds(const Step_Params& P)
+template <int SOLVER, bool CO>
+__device__ __forceinline__ void boundary_faces(const Step_Params& P, const long long first, const long long stride,
+                                               double smax[3], bool& zero)
 {
-	// a grid that stopped solves no face (the value is the same for every thread)
-	if (stopped_before(P)) return;
 	int combos[12][3];
 	const int nc = boundary_combos(P, combos);
-	double smax[3] = {0.0, 0.0, 0.0};
-	bool zero = false;
-	if ((int)blockIdx.y < nc) {
-		const int d = combos[blockIdx.y][0], side = combos[blockIdx.y][1], e = combos[blockIdx.y][2];
-		const long long count = boundary_count(P, d, e);
-		for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < count;
-		     t += (long long)gridDim.x * blockDim.x) {
-			boundary_face<SOLVER, false>(P, d, side, e, t, smax, zero);
+	#pragma unroll 1
+	for (int c = 0; c < nc; c++) {
+		const long long count = boundary_count(P, combos[c][0], combos[c][2]);
+		#pragma unroll 1
+		for (long long t = first; t < count; t += stride) {
+			boundary_face<SOLVER, CO>(P, combos[c][0], combos[c][1], combos[c][2], t, smax, zero);
 		}
 	}
+}
+
+/*
+One step of a grid.  The last P.boundary layers of blocks solve the
+ghost-ghost faces of non-periodic sides: they read and reduce what the
+tiles do, and fill the SMs as the tiles' last wave drains (as a launch of
+its own before the step they took 12 of 110 us on a 96 x 64 x 50 grid).
+*/
+template <int SOLVER, int TY, bool ZACT>
+__global__ void __launch_bounds__(TX * TY, Tile_Kind::resident_of(TY)) step_kernel(const Step_Params P)
+{
+	extern __shared__ __align__(16) double smem[];
+	__shared__ double s_dt;
+	__shared__ int s_stop;
+	__shared__ unsigned long long s_bar;
+	Split_Barrier bar = split_barrier(&s_bar);
+	if (threadIdx.x == 0 and threadIdx.y == 0) bar.init(TY);
+	const bool first_block = blockIdx.x == 0 and blockIdx.y == 0 and blockIdx.z == 0;
+	const double dt = begin_step(P, &s_dt, first_block, &s_stop);
+	if (s_stop) {
+		if (blockIdx.z < gridDim.z - P.boundary) tile_hold<TY, false>(P, blockIdx.x, blockIdx.y, blockIdx.z);
+		return;
+	}
+	double s0 = 0.0, s1 = 0.0, s2 = 0.0;
+	bool zero = false;
+	const int chunks = gridDim.z - P.boundary;
+	if ((int)blockIdx.z >= chunks) {
+		double smax[3] = {0.0, 0.0, 0.0};
+		const long long block = (blockIdx.z - chunks) * (long long)gridDim.x * gridDim.y + blockIdx.y * gridDim.x + blockIdx.x;
+		boundary_faces<SOLVER, false>(P, block * (TX * TY) + threadIdx.y * TX + threadIdx.x,
+		                              P.boundary * (long long)gridDim.x * gridDim.y * (TX * TY), smax, zero);
+		flush_speeds(P, smax, zero);
+		return;
+	}
+	tile_step<SOLVER, TY, ZACT>(P, smem, bar, dt, blockIdx.x, blockIdx.y, blockIdx.z, s0, s1, s2, zero);
+	double smax[3] = {s0, s1, s2};
 	flush_speeds(P, smax, zero);
 }
 
-template <int SOLVER>
-__global__ void boundary_speed_kernel(const Step_Params P)
-{
-	boundary_speeds<SOLVER>(P);
-}
-
-// the same for every box of a batch: blockIdx.z is the box
+// the ghost-ghost faces of every box of a batch, blockIdx.y the box
 template <int SOLVER>
 __global__ void batch_boundary_speed_kernel(const Step_Params* __restrict__ boxes, const int phase)
 {
 	__shared__ Step_Params sp;
 	if (threadIdx.x == 0) {
-		sp = boxes[blockIdx.z];
+		sp = boxes[blockIdx.y];
 		sp.phase = phase;
 	}
 	__syncthreads();
-	boundary_speeds<SOLVER>(sp);
+	// a box that stopped solves no face (the value is the same for every thread)
+	if (stopped_before(sp)) return;
+	double smax[3] = {0.0, 0.0, 0.0};
+	bool zero = false;
+	boundary_faces<SOLVER, false>(sp, blockIdx.x * (long long)blockDim.x + threadIdx.x,
+	                              (long long)gridDim.x * blockDim.x, smax, zero);
+	flush_speeds(sp, smax, zero);
 }
 
 // ------------------------------------------------------------------ layout and ghosts
@@ -991,7 +998,7 @@ the boxes' parameters of the two state parities, the first used by step
 step0.  Loads that read what another block wrote before go through L2 (CO).
 */
 template <int SOLVER, int TY, bool ZACT>
-__global__ void __launch_bounds__(TX * TY, Resident<TY, ZACT>::blocks) batch_run_kernel(
+__global__ void __launch_bounds__(TX * TY, Tile_Kind::resident_of(TY)) batch_run_kernel(
 	const Step_Params* __restrict__ boxes_even, const Step_Params* __restrict__ boxes_odd,
 	const int4* __restrict__ items, const int nitems, const int* __restrict__ box_items, unsigned int* done,
 	const int nboxes, const long long step0, const int nsteps, Run_Sync* sync, const long long wait_limit)
@@ -1249,7 +1256,7 @@ int launch_step(const Step_Params& P, const int solver, cudaStream_t stream)
 	                 : (nz + P.kchunk - 1) / P.kchunk;
 	if (chunks < 1) return PAMHD_OK;  // no planes between the first and the last
 	return with_kind(step_tile(solver, P.active[1] != 0, P.active[2] != 0), [&](auto solver_, auto rows, auto zact) {
-		const dim3 grid((P.L.n[0] + TX - 1) / TX, (P.L.n[1] + rows() - 1) / rows(), chunks);
+		const dim3 grid((P.L.n[0] + TX - 1) / TX, (P.L.n[1] + rows() - 1) / rows(), chunks + P.boundary);
 		step_kernel<solver_(), rows(), zact()>
 			<<<grid, dim3(TX, rows()), tile_bytes<solver_(), rows(), zact()>(), stream>>>(P);
 		return status_of(cudaGetLastError());
@@ -1327,7 +1334,7 @@ int launch_batch_step(const Step_Params* boxes, const int4* items, const int nit
 int launch_batch_boundary_speeds(const Step_Params* boxes, const int nboxes, const int largest, const int phase,
                                  const int solver, cudaStream_t stream)
 {
-	const dim3 grid(min(1024, (largest + 255) / 256), 12, nboxes);
+	const dim3 grid(min(1024, (largest + 255) / 256), nboxes);
 	switch (solver) {
 	case PAMHD_RUSANOV: batch_boundary_speed_kernel<PAMHD_RUSANOV><<<grid, 256, 0, stream>>>(boxes, phase); break;
 	case PAMHD_HLL_ATHENA: batch_boundary_speed_kernel<PAMHD_HLL_ATHENA><<<grid, 256, 0, stream>>>(boxes, phase); break;
@@ -1338,28 +1345,19 @@ int launch_batch_boundary_speeds(const Step_Params* boxes, const int nboxes, con
 	return cudaGetLastError() == cudaSuccess ? PAMHD_OK : PAMHD_ERR_CUDA;
 }
 
-int launch_boundary_speeds(const Step_Params& P, const int solver, cudaStream_t stream)
+int boundary_layers(const Step_Params& P, const int solver)
 {
-	int combos = 0, largest = 0;
+	long long faces = 0;
 	for (int d = 0; d < 3; d++) {
 		if (not P.active[d] or P.periodic[d]) continue;
 		for (int e = 0; e < 3; e++) {
-			if (e == d or not P.active[e]) continue;
-			combos += 2;
-			const int f = 3 - d - e;
-			largest = max(largest, P.L.n[e] * P.L.n[f]);
+			if (e != d and P.active[e]) faces += 2LL * P.L.n[e] * P.L.n[3 - d - e];
 		}
 	}
-	if (combos == 0) return PAMHD_OK;
-	const dim3 grid(min(1024, (largest + 255) / 256), combos);
-	switch (solver) {
-	case PAMHD_RUSANOV: boundary_speed_kernel<PAMHD_RUSANOV><<<grid, 256, 0, stream>>>(P); break;
-	case PAMHD_HLL_ATHENA: boundary_speed_kernel<PAMHD_HLL_ATHENA><<<grid, 256, 0, stream>>>(P); break;
-	case PAMHD_HLLD_ATHENA: boundary_speed_kernel<PAMHD_HLLD_ATHENA><<<grid, 256, 0, stream>>>(P); break;
-	case PAMHD_ROE_ATHENA: boundary_speed_kernel<PAMHD_ROE_ATHENA><<<grid, 256, 0, stream>>>(P); break;
-	default: return PAMHD_ERR_ARGUMENT;
-	}
-	return cudaGetLastError() == cudaSuccess ? PAMHD_OK : PAMHD_ERR_CUDA;
+	// about a face per thread
+	const int rows = step_tile(solver, P.active[1] != 0, P.active[2] != 0).rows;
+	const long long layer = (long long)((P.L.n[0] + TX - 1) / TX) * ((P.L.n[1] + rows - 1) / rows) * TX * rows;
+	return int(min(1024LL, (faces + layer - 1) / layer));
 }
 
 int launch_scatter(const double* packed, double* var_base, const Layout& L, cudaStream_t stream)

@@ -41,6 +41,28 @@ def pair(port, n, solver, lengths, gamma, mu0, cfl, bc_lo=(0, 0, 0), bc_hi=(0, 0
 
 # ---------------------------------------------------------------- solver level
 
+@pytest.mark.parametrize("bc", ["periodic", "copy"])
+@pytest.mark.parametrize("n", [(33, 9, 2), (70, 17, 37), (31, 40, 3), (64, 8, 19)])
+def test_short_z_chunks_match_oracle(port, n, bc):
+    """Small 3-D grids, whose blocks take a few planes each (the last chunk of 37 planes a single
+    one) and whose tiles end one cell short of, at and one cell past 32 columns and 8 rows; on open
+    sides the step's own blocks solve the ghost-ghost faces.  Per step, the bar of this file."""
+    kinds = ((pg.BC_COPY,) * 3 if bc == "copy" else (pg.BC_PERIODIC,) * 3,) * 2
+    L = (0.1, 0.12, 0.09)
+    U = states.smooth_3d((n[2], n[1], n[0]), np.random.default_rng(3))
+    gpu = pg.Context(pg.Config(n=n, solver=pg.HLLD, cell_length=L, time_step_factor=0.4, bc_lo=kinds[0],
+                               bc_hi=kinds[1]))
+    ora = port.grid(po.make_cfg(n, pg.HLLD, L, states.GAMMA_53, 1.0, 0.4, *kinds), threads=4)
+    gpu.set_state(U)
+    ora.set_state(U)
+    for s in range(4):
+        dg = gpu.step(0.0 if s == 0 else 1.0)
+        do, flag, _, _ = ora.step(0.0 if s == 0 else 1.0)
+        assert flag == 0
+        assert abs(dg - do) <= 1e-13 * max(do, 1e-300), s
+        assert field_err(gpu.get_state(), ora.get_state()) <= STEP_TOL, s
+
+
 @pytest.mark.parametrize("normal", ["field", "none"])
 def test_roe_aligned_faces_match_oracle(port, normal):
     """Faces without a transverse field in the Roe average (no transverse field at all, or opposite
