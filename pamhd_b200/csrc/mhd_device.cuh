@@ -55,6 +55,24 @@ __device__ __forceinline__ bool is_finite(const double x)
 	return ((unsigned int)__double2hiint(x) & 0x7fffffffu) < 0x7ff00000u;
 }
 
+// the sign bit: x < 0 for any number but -0
+__device__ __forceinline__ bool is_negative(const double x)
+{
+	return __double2hiint(x) < 0;
+}
+
+// zero, negative or not a number (an infinite x counts too: its timestep is 0 as well)
+__device__ __forceinline__ bool no_speed(const double x)
+{
+	return (unsigned int)__double2hiint(x) - 1u >= 0x7ff00000u - 1u;
+}
+
+// the larger of two numbers (fmax() also sorts out NaN, which takes twice the instructions)
+__device__ __forceinline__ double larger(const double a, const double b)
+{
+	return a > b ? a : b;
+}
+
 // physical constants of one run
 struct Gas {
 	double gamma;     // adiabatic index
@@ -314,8 +332,8 @@ __device__ __forceinline__ double flux_rusanov(const Side& L, const Side& R, con
                                                uint32_t& flag, const double* bg = nullptr)
 {
 	using A = Ar;
-	const double fast = fmax(L.cf, R.cf);
-	const double s = A::add(fmax(fabs(L.v0), fabs(R.v0)), fast);
+	const double fast = larger(L.cf, R.cf);
+	const double s = A::add(larger(fabs(L.v0), fabs(R.v0)), fast);
 	double FL[8], FR[8];
 	if (BG) {
 		physical_flux_bg(L, bg[0], bg[1], bg[2], g, FL);
@@ -347,11 +365,11 @@ __device__ __forceinline__ double flux_hll(const Side& L, const Side& R, const G
                                            uint32_t& /*flag*/, const double* bg = nullptr)
 {
 	using A = Ar;
-	const double fast = fmax(L.cf, R.cf);
+	const double fast = larger(L.cf, R.cf);
 	const bool order = L.v0 <= R.v0;
 	const double s_neg = A::sub(order ? L.v0 : R.v0, fast);
 	const double s_pos = A::add(order ? R.v0 : L.v0, fast);
-	const double bm = fmin(s_neg, 0.0), bp = fmax(s_pos, 0.0);
+	const double bm = is_negative(s_neg) ? s_neg : 0.0, bp = is_negative(s_pos) ? 0.0 : s_pos;
 	const double width = A::sub(bp, bm);
 	if (not is_positive_normal(width)) {
 		#pragma unroll
@@ -374,7 +392,7 @@ __device__ __forceinline__ double flux_hll(const Side& L, const Side& R, const G
 	for (int v = 0; v < 8; v++) {
 		F[v] = v == 5 ? 0.0 : A::fma(wl, A::fma(-bm, UL[v], FL[v]), A::mul(wr, A::fma(-bp, UR[v], FR[v])));
 	}
-	return fmax(bp, -bm);
+	return larger(bp, -bm);
 }
 
 // transverse velocity and field of one side's star state (Miyoshi & Kusano eqns 44-47): v - b t1
@@ -450,17 +468,16 @@ __device__ __forceinline__ double flux_hlld(const Side& L, const Side& R, const 
                                             const PICK& pick)
 {
 	using A = Ar;
-	const double fast = fmax(L.cf, R.cf);
+	const double fast = larger(L.cf, R.cf);
 	const bool order = L.v0 <= R.v0;
 	const double s_neg = A::sub(order ? L.v0 : R.v0, fast);  // eqn 67
 	const double s_pos = A::add(order ? R.v0 : L.v0, fast);
+	const double speed = larger(fabs(s_neg), fabs(s_pos));
 
-	if (s_neg >= 0.0 or s_pos <= 0.0) {
-		const bool from_left = s_neg >= 0.0;
-		physical_flux(pick(from_left), g, F);
-		return from_left ? fabs(s_pos) : fabs(s_neg);
+	if (not is_negative(s_neg) or is_negative(s_pos)) {
+		physical_flux(pick(not is_negative(s_neg)), g, F);
+		return speed;
 	}
-	const double speed = fmax(-s_neg, s_pos);
 
 	const double bx = A::mul(0.5, A::add(L.b0, R.b0));
 	const double bxm = A::mul(bx, g.inv_mu0), bx2_mu = A::mul(bx, bxm);
@@ -485,9 +502,9 @@ __device__ __forceinline__ double flux_hlld(const Side& L, const Side& R, const 
 	const Star_T tr = star_transverse(R, rsdR, sdR, smR, s_mid, bxm, bx2_mu, thr);
 
 	// region order of hlld_athena.hpp:475-552: S*_L >= 0, S_M >= 0, S*_R > 0, else
-	const bool left = s_mid >= 0.0;
-	const bool star_l = ssL >= 0.0;
-	const bool star_r = not star_l and not left and not (ssR > 0.0);
+	const bool left = not is_negative(s_mid);
+	const bool star_l = not is_negative(ssL);
+	const bool star_r = not star_l and not left and is_negative(ssR);
 	const bool useL = star_l or (not star_r and left);   // the side the flux is taken from
 	// the double-star region (the star state itself when Bx ~ 0)
 	const bool two = not star_l and not star_r and not (A::mul(A::mul(0.5, bx), bx) < thr);
@@ -526,13 +543,9 @@ __device__ __forceinline__ double flux_hlld(const Side& L, const Side& R, const 
 	F[3] = A::fma(F[0], w2, A::fma(-bxm, b2, -A::mul(overm, S.b2)));
 	F[4] = A::fma(A::add(e, ptst), s_mid, A::fma(-bxm, vb2, -A::mul(overm, vb)));
 	F[5] = 0.0;
-	F[6] = A::fma(s_mid, b1, A::fma(-bx, w1, -A::mul(over, S.v1)));
-	F[7] = A::fma(s_mid, b2, A::fma(-bx, w2, -A::mul(over, S.v2)));
-	if (ts.keep) {
-		const double kv = A::sub(S.v0, s_mid);
-		F[6] = A::fma(kv, S.b1, F[6]);
-		F[7] = A::fma(kv, S.b2, F[7]);
-	}
+	const double kv = ts.keep ? A::sub(S.v0, s_mid) : 0.0;
+	F[6] = A::fma(kv, S.b1, A::fma(s_mid, b1, A::fma(-bx, w1, -A::mul(over, S.v1))));
+	F[7] = A::fma(kv, S.b2, A::fma(s_mid, b2, A::fma(-bx, w2, -A::mul(over, S.v2))));
 	return speed;
 }
 

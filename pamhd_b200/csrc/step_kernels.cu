@@ -56,11 +56,11 @@ template <int TY, bool ZACT, int NF = 8> struct Tile {
 	static constexpr int H = TY + 2 * JO;                  // record rows
 	static constexpr int CELLS = W * H;
 	static constexpr int REC = NV * CELLS;                 // doubles per plane slot
-	static constexpr int FXN = TY * (TX + 1);              // x faces of a plane
-	static constexpr int FYN = (TY > 1) ? (TY + 1) * TX : 0;
 	static constexpr int SLOTS = ZACT ? 2 : 1;             // planes whose records are held
-	// the record slots, the x and y face fluxes, one validity byte per cell and slot
-	static constexpr size_t BYTES = size_t(SLOTS * REC + NF * FXN + NF * FYN) * 8 + size_t(SLOTS * CELLS);
+	// the record slots; the x and the y face fluxes of a plane, indexed as the record of the cell on
+	// the face's positive side, so that one index per thread serves records and fluxes; one
+	// validity byte per cell and slot
+	static constexpr size_t BYTES = size_t(SLOTS * REC + NF * CELLS * (1 + JO)) * 8 + size_t(SLOTS * CELLS);
 };
 
 template <int SOLVER, int TY, bool ZACT> constexpr size_t tile_bytes()
@@ -350,9 +350,8 @@ non-coherent L1 could hold a line of the same buffer from two steps before).
 */
 template <bool CX, bool CY, bool CZ, bool CO>
 __device__ __forceinline__ double load_record(const Step_Params& P, double* rec, uint8_t* bad, const int cells,
-                                              const int ri, const int i, const int j, const int k)
+                                              const int ri, const long long off)
 {
-	const long long off = P.L.offset(i, j, k);
 	double U[8];
 	#pragma unroll
 	for (int v = 0; v < 8; v++) U[v] = CO ? __ldcg(P.in + v * P.L.var + off) : __ldg(P.in + v * P.L.var + off);
@@ -412,8 +411,8 @@ __device__ __forceinline__ void solve_z(const Step_Params& P, const double* rec_
 	};
 	const double s = solve_face<SOLVER>(L, R, P.gas, F, flag, pick);
 	if (flag != 0) record_failure(P, flag, i, j, k, 3);
-	smax = fmax(smax, s);
-	zero = zero or not (s > 0.0);
+	smax = larger(s, smax);
+	zero = zero or no_speed(s);
 	d[0] = F[0];
 	unrotate<2>(F[1], F[2], F[3], d[1], d[2], d[3]);
 	d[4] = F[4];
@@ -421,34 +420,40 @@ __device__ __forceinline__ void solve_z(const Step_Params& P, const double* rec_
 }
 
 /*
-One x or y face (axis a, 0 or 1, known only at run time) between record
-positions rl and rr of one slot.  The x and y faces of a plane share this
-one inlined solver instance (half the code of one instance per axis, which
-the instruction cache rewards); the rotation into the face frame is a
-choice of record rows to read.  The unscaled flux goes to out[r][idx] in
-the face frame, Flux_Rows<SOLVER>::N rows (the caller rotates it back).
+One x or y face (axis a, 0 or 1, known only at run time) on the negative
+side of record position rr of a slot.  The x and y faces of a plane share
+this one inlined solver instance (half the code of one instance per axis,
+which the instruction cache rewards).  The rotation into the face frame is
+a choice of record rows to read, two offsets per side: x reads rows m_x,
+m_y, m_z; y reads m_y, m_z (one row on) and m_x.  The unscaled flux goes to
+out[r][rr] in the face frame, Flux_Rows<SOLVER>::N rows (the caller rotates
+it back).  Returns the face's signal speed.
 */
-template <int SOLVER, int CELLS>
-__device__ __forceinline__ void solve_xy(const Step_Params& P, const double* rec, const uint8_t* bad,
-                                         const int rl, const int rr, const int a, double* out, const int nout,
-                                         const int idx, double& s0, double& s1, bool& zero,
-                                         const int i, const int j, const int k)
+template <int SOLVER, int TY, class T>
+__device__ __forceinline__ double solve_xy(const Step_Params& P, const double* rec, const uint8_t* bad,
+                                           const int rr, const int a, double* const out, const int gx0,
+                                           const int gy0, const int k)
 {
-	const int a1 = a + 1, a2 = a == 0 ? 2 : 0;  // the face frame's tangential axes
+	constexpr int C = T::CELLS;
+	const int rl = rr - (a == 0 ? 1 : T::W);
+	const int near = a * C, far = a == 0 ? 2 * C : 0;
 	auto side = [&](const int r) {
+		const double* const c = rec + r;
+		const double* const n = c + near;
+		const double* const f = c + far;
 		Side s;
-		s.rho = rec[r];
-		s.m0 = rec[(1 + a) * CELLS + r];
-		s.m1 = rec[(1 + a1) * CELLS + r];
-		s.m2 = rec[(1 + a2) * CELLS + r];
-		s.E = rec[4 * CELLS + r];
-		s.b0 = rec[(5 + a) * CELLS + r];
-		s.b1 = rec[(5 + a1) * CELLS + r];
-		s.b2 = rec[(5 + a2) * CELLS + r];
-		s.rinv = rec[R_RINV * CELLS + r];
-		s.pt = rec[R_PT * CELLS + r];
+		s.rho = c[0];
+		s.m0 = n[C];
+		s.m1 = n[2 * C];
+		s.m2 = f[C];
+		s.E = c[4 * C];
+		s.b0 = n[5 * C];
+		s.b1 = n[6 * C];
+		s.b2 = f[5 * C];
+		s.rinv = c[R_RINV * C];
+		s.pt = c[R_PT * C];
 		s.p = 0.0;  // not read without a background field
-		s.cf = rec[(R_CF + a) * CELLS + r];
+		s.cf = n[R_CF * C];
 		s.v0 = s.m0 * s.rinv;
 		s.v1 = s.m1 * s.rinv;
 		s.v2 = s.m2 * s.rinv;
@@ -461,17 +466,16 @@ __device__ __forceinline__ void solve_xy(const Step_Params& P, const double* rec
 	uint32_t flag = 0;
 	const auto pick = [&](const bool left) { return side(left ? rl : rr); };
 	const double sp = solve_face<SOLVER>(L, R, P.gas, F, flag, pick);
-	if (flag != 0) record_failure(P, flag, i, j, k, a + 1);
-	if (a == 0) s0 = fmax(s0, sp); else s1 = fmax(s1, sp);
-	zero = zero or not (sp > 0.0);
-	out[idx] = F[0];
-	out[1 * nout + idx] = F[1];
-	out[2 * nout + idx] = F[2];
-	out[3 * nout + idx] = F[3];
-	out[4 * nout + idx] = F[4];
-	out[5 * nout + idx] = F[6];
-	out[6 * nout + idx] = F[7];
-	if (Flux_Rows<SOLVER>::N == 8) out[7 * nout + idx] = F[5];
+	if (flag != 0) record_failure(P, flag, gx0 + rl % T::W - 1, gy0 + rl / T::W - T::JO, k, a + 1);
+	out[rr] = F[0];
+	out[C + rr] = F[1];
+	out[2 * C + rr] = F[2];
+	out[3 * C + rr] = F[3];
+	out[4 * C + rr] = F[4];
+	out[5 * C + rr] = F[6];
+	out[6 * C + rr] = F[7];
+	if (Flux_Rows<SOLVER>::N == 8) out[7 * C + rr] = F[5];
+	return sp;
 }
 
 // ------------------------------------------------------------------ the step
@@ -538,9 +542,9 @@ __device__ __forceinline__ void tile_step(const Step_Params& P, double* const sm
 	constexpr int NF = Flux_Rows<SOLVER>::N;
 	using T = Tile<TY, ZACT, NF>;
 	double* const rec_base = smem;
-	double* const fx = smem + T::SLOTS * T::REC; // [NF][TY][TX + 1]
-	double* const fy = fx + NF * T::FXN;         // [NF][TY + 1][TX]
-	uint8_t* const bad_base = reinterpret_cast<uint8_t*>(fy + NF * T::FYN);
+	double* const fx = smem + T::SLOTS * T::REC;   // [NF][CELLS]
+	double* const fy = fx + NF * T::CELLS;         // [NF][CELLS] (y active)
+	uint8_t* const bad_base = reinterpret_cast<uint8_t*>(fx + NF * T::CELLS * (1 + T::JO));
 
 	constexpr bool YACT = TY > 1;
 	const int nx = P.L.n[0], ny = P.L.n[1];
@@ -566,35 +570,50 @@ __device__ __forceinline__ void tile_step(const Step_Params& P, double* const sm
 	// the flux terms are dt F / dx: dt / dx once per axis and cell
 	const double cx = dt * P.inv_len[0], cy = dt * P.inv_len[1], cz = dt * P.inv_len[2];
 
-	// a plane's records: own cells, and the halo for planes with x / y faces, spread over warps: the
-	// rows below / above the tile on warps 0 and 1, the columns left / right of it on warp 2 (warp 0
-	// when y is inactive).  Returns the own column's fast speed along z.
+	// this thread's halo cell of planes with x / y faces, if any: the rows below / above the tile on
+	// warps 0 and 1, the columns left / right of it on warp 2 (warp 0 when y is inactive)
+	int hri = -1;
+	long long hoff = 0;
+	if (YACT and warp < 2) {
+		const int hy = warp == 1 ? gy0 + TY : gy0 - 1;
+		if (gx < nx and hy <= ny) {
+			hri = (warp == 1 ? TY + 1 : 0) * T::W + lane + 1;
+			hoff = P.L.offset(gx, hy, 0);
+		}
+	} else if (warp == XHALO_WARP and lane < 2 * TY) {
+		const int row = lane % TY;
+		const bool right = lane >= TY;
+		const int hx = right ? gx0 + TX : gx0 - 1;
+		if (gy0 + row < ny and hx <= nx) {
+			hri = (row + T::JO) * T::W + (right ? TX + 1 : 0);
+			hoff = P.L.offset(hx, gy0 + row, 0);
+		}
+	}
+	const long long col = P.L.offset(gx, gy, 0);
+	// a plane's records: own cells, and the halo.  Returns the own column's fast speed along z.
 	const auto stage_plane = [&](const int k) -> double {
 		const int slot = ZACT ? (k - kfirst) & 1 : 0;
 		double* const rec = rec_base + slot * T::REC;
 		uint8_t* const bad = bad_base + slot * T::CELLS;
 		double cfz = 0.0;
-		if (stage) cfz = load_record<true, YACT, ZACT, CO>(P, rec, bad, T::CELLS, ri, gx, gy, k);
-		if (k >= kb and k < ke) {
-			if (YACT and warp < 2) {
-				const bool top = warp == 1;
-				const int hy = top ? gy0 + TY : gy0 - 1;
-				if (gx0 + lane < nx and hy <= ny) {
-					const int hri = (top ? TY + 1 : 0) * T::W + lane + 1;
-					load_record<false, true, false, CO>(P, rec, bad, T::CELLS, hri, gx0 + lane, hy, k);
-				}
-			} else if (warp == XHALO_WARP and lane < 2 * TY) {
-				const int row = lane % TY;
-				const bool right = lane >= TY;
-				const int hx = right ? gx0 + TX : gx0 - 1;
-				if (gy0 + row < ny and hx <= nx) {
-					const int hri = (row + T::JO) * T::W + (right ? TX + 1 : 0);
-					load_record<true, false, false, CO>(P, rec, bad, T::CELLS, hri, hx, gy0 + row, k);
-				}
-			}
+		if (stage) cfz = load_record<true, YACT, ZACT, CO>(P, rec, bad, T::CELLS, ri, col + k * P.L.plane);
+		if (k >= kb and k < ke and hri >= 0) {
+			load_record<true, YACT, false, CO>(P, rec, bad, T::CELLS, hri, hoff + k * P.L.plane);
 		}
 		return cfz;
 	};
+
+	// the x and y faces this thread solves, one bit each: 0 its -x face, 1 one of the tile's +x faces,
+	// 2 its -y face, 3 one of the tile's +y faces; the +x and +y faces are a further pass of one warp
+	// each, at record position extra
+	uint32_t tasks = 0;
+	if (gx <= nx and gy < ny) tasks |= 1u;
+	if (warp == XFACE_WARP and lane < TY and gx0 + TX <= nx and gy0 + lane < ny) tasks |= 2u;
+	if (YACT and gy <= ny and gx < nx) tasks |= 4u;
+	if (YACT and warp == YFACE_WARP and gy0 + TY <= ny and gx < nx) tasks |= 8u;
+	const int extra_x = (lane + T::JO) * T::W + TX + 1, extra_y = (TY + T::JO) * T::W + lane + 1;
+	// a cell on the grid's x or y edge also writes a ghost
+	const bool edge = gx == 0 or gx == nx - 1 or gy == 0 or gy == ny - 1;
 
 	// the scaled flux of the -z face of the own cell of plane k
 	double low[8];
@@ -614,38 +633,20 @@ __device__ __forceinline__ void tile_step(const Step_Params& P, double* const sm
 
 		if (inner) {
 			__syncthreads();
-			// (b) x and y faces: every thread its -x and -y face; the tile's last column and row also
-			// need their +x / +y faces, taken by one warp each in a further pass of the same loop
+			// (b) x and y faces, all through one call site; s0 and s1 swap places from axis to axis
 			#pragma unroll 1
-			for (int task = 0; task < 4; task++) {
-				// 0: own -x face, 1: own -y face, 2: the tile's +x faces, 3: its +y faces
-				if (task == 1 and not YACT) continue;
-				if (task == 2 and warp != XFACE_WARP) continue;
-				if (task == 3 and (not YACT or warp != YFACE_WARP)) continue;
-				const int a = (task == 0 or task == 2) ? 0 : 1;
-				const int row = task == 2 ? lane : (task == 3 ? TY : ty);
-				const int col = task == 2 ? TX : tx;
-				// one call site: the x and y faces share one inlined solver instance
-				bool ok;
-				int rl, rr, idx, i, j;
-				if (a == 0) {
-					ok = (task == 2 ? lane < TY : true) and gx0 + col <= nx and gy0 + row < ny;
-					rl = (row + T::JO) * T::W + col;
-					rr = rl + 1;
-					idx = row * (TX + 1) + col;
-					i = gx0 + col - 1;
-					j = gy0 + row;
-				} else {
-					ok = gy0 + row <= ny and gx0 + col < nx;
-					rl = row * T::W + col + 1;
-					rr = rl + T::W;
-					idx = row * TX + col;
-					i = gx0 + col;
-					j = gy0 + row - 1;
+			for (int task = 0; task < (YACT ? 4 : 2); task++) {
+				const int a = task >> 1;
+				if ((tasks >> task) & 1u) {
+					const int rr = (task & 1) == 0 ? ri : (a == 0 ? extra_x : extra_y);
+					const double sp = solve_xy<SOLVER, TY, T>(P, rec, bad, rr, a, fx + a * NF * T::CELLS, gx0, gy0, k);
+					s0 = larger(sp, s0);
+					zero = zero or no_speed(sp);
 				}
-				if (ok) {
-					solve_xy<SOLVER, T::CELLS>(P, rec, bad, rl, rr, a, a == 0 ? fx : fy, a == 0 ? T::FXN : T::FYN,
-					                           idx, s0, s1, zero, i, j, k);
+				if (YACT and (task & 1)) {
+					const double t = s0;
+					s0 = s1;
+					s1 = t;
 				}
 			}
 			if (ZACT) bar.arrive();
@@ -676,7 +677,7 @@ __device__ __forceinline__ void tile_step(const Step_Params& P, double* const sm
 				for (int v = 0; v < 8; v++) {
 					Un[v] = rec[v * T::CELLS + ri];
 					if (XROW[v] >= 0) {
-						const double* f = fx + XROW[v] * T::FXN + ty * (TX + 1) + tx;
+						const double* f = fx + XROW[v] * T::CELLS + ri;
 						Un[v] = __fma_rn(__dsub_rn(f[0], f[1]), cx, Un[v]);
 					}
 				}
@@ -684,8 +685,8 @@ __device__ __forceinline__ void tile_step(const Step_Params& P, double* const sm
 					#pragma unroll
 					for (int v = 0; v < 8; v++) {
 						if (YROW[v] >= 0) {
-							const double* f = fy + YROW[v] * T::FYN + ty * TX + tx;
-							Un[v] = __fma_rn(__dsub_rn(f[0], f[TX]), cy, Un[v]);
+							const double* f = fy + YROW[v] * T::CELLS + ri;
+							Un[v] = __fma_rn(__dsub_rn(f[0], f[T::W]), cy, Un[v]);
 						}
 					}
 				}
@@ -693,7 +694,13 @@ __device__ __forceinline__ void tile_step(const Step_Params& P, double* const sm
 					#pragma unroll
 					for (int v = 0; v < 8; v++) Un[v] = __dadd_rn(Un[v], __dsub_rn(low[v], high[v]));
 				}
-				write_cell(P, gx, gy, k, Un, dt);
+				if (edge or (ZACT and (k == 0 or k == P.L.n[2] - 1))) {
+					write_cell(P, gx, gy, k, Un, dt);
+				} else {
+					double* const to = P.out + col + k * P.L.plane;
+					#pragma unroll
+					for (int v = 0; v < 8; v++) to[v * P.L.var] = Un[v];
+				}
 			}
 		}
 		#pragma unroll
