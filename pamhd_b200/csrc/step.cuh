@@ -117,9 +117,13 @@ struct Tile_Kind {
 	int rows;
 	bool zact;
 	// resident blocks per SM asked of the register allocator: 16 warps of at most 128 registers with
-	// 32 x 8 tiles, 12 warps of at most 168 with 32 x 4 (and one-row) tiles
-	static constexpr int resident_of(const int rows) { return rows == 8 ? 2 : 3; }
-	int resident() const { return resident_of(rows); }
+	// 32 x 8 tiles and with 32 x 4 tiles of one plane, 12 warps of at most 168 with 32 x 4 tiles that
+	// march in z, with Roe's solver and with one-row tiles
+	static constexpr int resident_of(const int solver, const int rows, const bool zact)
+	{
+		return rows == 8 ? 2 : (rows == 4 and not zact and solver != PAMHD_ROE_ATHENA ? 4 : 3);
+	}
+	int resident() const { return resident_of(solver, rows, zact); }
 };
 
 // launchers (step_kernels.cu)

@@ -716,7 +716,7 @@ kinds, reduction ring, clock, status), so each advances with its own dt.
 The block holding a box's first item advances that box's clock.
 */
 template <int SOLVER, int TY, bool ZACT>
-__global__ void __launch_bounds__(TX * TY, Tile_Kind::resident_of(TY)) batch_step_kernel(const Step_Params* __restrict__ boxes,
+__global__ void __launch_bounds__(TX * TY, Tile_Kind::resident_of(SOLVER, TY, ZACT)) batch_step_kernel(const Step_Params* __restrict__ boxes,
                                                                   const int4* __restrict__ items,
                                                                   const int nitems, const int phase)
 {
@@ -855,7 +855,7 @@ tiles do, and fill the SMs as the tiles' last wave drains (as a launch of
 its own before the step they took 12 of 110 us on a 96 x 64 x 50 grid).
 */
 template <int SOLVER, int TY, bool ZACT>
-__global__ void __launch_bounds__(TX * TY, Tile_Kind::resident_of(TY)) step_kernel(const Step_Params P)
+__global__ void __launch_bounds__(TX * TY, Tile_Kind::resident_of(SOLVER, TY, ZACT)) step_kernel(const Step_Params P)
 {
 	extern __shared__ __align__(16) double smem[];
 	__shared__ double s_dt;
@@ -1005,7 +1005,7 @@ the boxes' parameters of the two state parities, the first used by step
 step0.  Loads that read what another block wrote before go through L2 (CO).
 */
 template <int SOLVER, int TY, bool ZACT>
-__global__ void __launch_bounds__(TX * TY, Tile_Kind::resident_of(TY)) batch_run_kernel(
+__global__ void __launch_bounds__(TX * TY, Tile_Kind::resident_of(SOLVER, TY, ZACT)) batch_run_kernel(
 	const Step_Params* __restrict__ boxes_even, const Step_Params* __restrict__ boxes_odd,
 	const int4* __restrict__ items, const int nitems, const int* __restrict__ box_items, unsigned int* done,
 	const int nboxes, const long long step0, const int nsteps, Run_Sync* sync, const long long wait_limit)
@@ -1234,13 +1234,18 @@ static int status_of(const cudaError_t e)
 }
 
 /*
-The single-grid step's tile: 32 x 8, two blocks of 256 threads per SM (a
-taller tile solves fewer halo faces and records per cell); Roe's solver
-needs more registers, so it keeps 32 x 4 tiles at three blocks per SM.
+The single-grid step's tile.  3-D grids: 32 x 8, two blocks of 256 threads
+per SM (a taller tile solves fewer halo faces and records per cell).  2-D
+grids: 32 x 4, four blocks of 128 threads per SM: the same 16 warps in
+blocks that wait for fewer others, and twice the blocks on small grids
+(HLLD against 32 x 8 tiles: 257 x 180 cells 10.1 us per step, was 11.2;
+512^2 33.8, was 34.4; 1024^2 118, was 128).  Roe's solver needs more
+registers than either leaves, so it keeps 32 x 4 tiles at three blocks per
+SM (at four, 512^2 took 72 us instead of 66).
 */
 Tile_Kind step_tile(const int solver, const bool yact, const bool zact)
 {
-	return Tile_Kind{solver, not yact ? 1 : (solver == PAMHD_ROE_ATHENA ? TY_3D : TY_WIDE), zact};
+	return Tile_Kind{solver, not yact ? 1 : (solver == PAMHD_ROE_ATHENA or not zact ? TY_3D : TY_WIDE), zact};
 }
 
 int prepare_step_kernels(const Tile_Kind& kind)
