@@ -145,6 +145,7 @@ int build_work(pamhd_batch& b, const int planes)
 	for (int i = 0; i < b.nboxes; i++) {
 		Step_Params P;
 		const bool nb = grid_params(b.cfg[i], b.L[i], P, planes);
+		tile_shape(b.kind(ty), b.cfg[i].n[0], b.cfg[i].n[1], P.tw, P.th);
 		P.kchunk = std::max(1, std::min(planes, b.cfg[i].n[2]));
 		b.needs_boundary = b.needs_boundary or nb;
 		for (int d = 0; d < 3; d++) {
@@ -172,8 +173,9 @@ int build_work(pamhd_batch& b, const int planes)
 	}
 	for (const int i: order) {
 		const pamhd_cfg& c = b.cfg[i];
-		const int tiles = ((c.n[0] + 31) / 32) * ((c.n[1] + ty - 1) / ty);
-		const int kc = b.params[0][i].kchunk;
+		const Step_Params& P = b.params[0][i];
+		const int tiles = ((c.n[0] + P.tw - 1) / P.tw) * ((c.n[1] + P.th - 1) / P.th);
+		const int kc = P.kchunk;
 		const int chunks = (c.n[2] + kc - 1) / kc;
 		for (int z = 0; z < chunks; z++) {
 			for (int t = 0; t < tiles; t++) items.push_back(make_int4(i, t, z, 0));
@@ -221,6 +223,27 @@ int build_work(pamhd_batch& b, const int planes)
 		cudaGraphExecDestroy(b.run_graph);
 		b.run_graph = nullptr;
 		b.run_key = -1;
+	}
+	return PAMHD_OK;
+}
+
+/*
+The work split a batch starts with (the autotuners measure others): 32 x 8
+tiles (32 x 4 for Roe, as the single-grid step) and the most z planes per
+item, up to 64, that still give 1.5 items per resident block: long items
+repeat fewer planes and start-ups (64 boxes of 32^3 to 128^3, HLL: 9.27 G
+cell-updates/s with 64 planes, 8.68 with 12), short ones keep a small
+ensemble's SMs busy (8 boxes of 24^3 to 48^3: 238 us per step with 64
+planes, 128 with 12, 129 with 8).
+*/
+int default_work(pamhd_batch& b, const int sms)
+{
+	b.ty = step_tile(b.solver, b.yact, b.zact).rows;
+	if (not b.zact) return build_work(b, 1);
+	const long long enough = 3LL * sms * b.kind(b.ty).resident() / 2;
+	for (const int planes: {64, 48, 32, 24, 16, 12}) {
+		PAMHD_TRY(build_work(b, planes));
+		if (b.nitems >= enough) break;
 	}
 	return PAMHD_OK;
 }
@@ -439,16 +462,14 @@ int pamhd_gpu_batch_create(const int32_t device, const int32_t nboxes, const pam
 		or cudaMemset(b->dt_hist, 0, size_t(b->hist_len) * nboxes * sizeof(double)) != cudaSuccess) {
 		return fail(PAMHD_ERR_CUDA);
 	}
-	b->ty = b->yact ? batch_tile_rows() : 1;
 	for (const int ty: tile_choices(*b)) {
 		if (prepare_batch_kernels(b->kind(ty)) != PAMHD_OK) return fail(PAMHD_ERR_CUDA);
 		if (prepare_batch_run_kernels(b->kind(ty)) != PAMHD_OK) return fail(PAMHD_ERR_CUDA);
 	}
-	int per_sm = 0;
-	if (batch_blocks_per_sm(b->kind(b->ty), &per_sm) != PAMHD_OK or per_sm < 1) return fail(PAMHD_ERR_CUDA);
-	int sms = 0;
+	int per_sm = 0, sms = 0;
 	cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
-	if (build_work(*b, 32) != PAMHD_OK) return fail(PAMHD_ERR_CUDA);
+	if (default_work(*b, sms) != PAMHD_OK) return fail(PAMHD_ERR_CUDA);
+	if (batch_blocks_per_sm(b->kind(b->ty), &per_sm) != PAMHD_OK or per_sm < 1) return fail(PAMHD_ERR_CUDA);
 	b->grid = std::min(b->nitems, std::max(1, sms * per_sm));
 	if (reset_run_state(*b) != PAMHD_OK) return fail(PAMHD_ERR_CUDA);
 	*out = b;

@@ -114,6 +114,45 @@ inline Layout make_layout(const pamhd_cfg& c)
 }
 
 /*
+The columns tw x th of a tile of 32 rows threads on nx x ny columns: the
+shape with the least estimated work on the grid.  With 32 x 8 tiles alone
+a grid of 100 x 100 columns has 4 x 13 tiles, a quarter of whose threads
+own no cell; 25 x 10 columns per tile leave 2 % (100^3 HLLD: 134.7 us per
+step with 32 x 8, 107.9 with 25 x 10).  A tile costs its passes: a warp's
+three face solves (x, y, z) and its records per plane count 4, the +x and
++y faces a face solve per warp of them that the threads without a cell do
+not take, the halo records a third of one per warp; half of the cost is
+latency, which a warp less does not shorten.  Rows of 32 columns, which
+are warps, run 10 % faster than others (88 x 205 x 72 HLLD: 148 us, 162
+with 18 x 14, though 4 % fewer threads idle), so a shape has to save more.
+Grids without z faces keep 32 columns: their one plane is too short for
+the run-time shape's index arithmetic (512^2: +4 %).
+*/
+inline void tile_shape(const Tile_Kind& kind, const int nx, const int ny, int& tw, int& th)
+{
+	tw = kind.zact ? 32 : Tile_Kind::flat_width_of(kind.rows);
+	th = kind.rows;
+	if (not kind.zact) return;
+	const int threads = 32 * kind.rows;
+	double least = 1e300;
+	for (int w = 16; w <= 64; w++) {
+		for (int h = 2; h * w <= threads and w + h <= threads / 2; h++) {
+			if (w * (h + 2) + 2 * h > Tile_Kind::records_of(kind.rows) or (ny + h - 1) / h > 65535) continue;
+			const double tiles = double((nx + w - 1) / w) * ((ny + h - 1) / h);
+			const int warps = (w * h + 31) / 32, spare = threads - w * h;
+			const int extra = std::max(0, w + h - 2 * spare);
+			const double passes = 4.0 * warps + (extra + 31) / 32 + (2 * (w + h) + 31) / 32 / 3.0;
+			const double time = tiles * (passes + 4.0 * kind.rows + 3.0) * (w == 32 ? 1.0 : 1.1);
+			if (time < least) {
+				least = time;
+				tw = w;
+				th = h;
+			}
+		}
+	}
+}
+
+/*
 z planes per block of a step: the chunk length with the shortest estimated
 step.  A block of kc planes takes about kc + 1 plane times (the planes
 before and after the chunk, and the block's start and end); 148 SMs run
@@ -176,7 +215,8 @@ inline bool grid_params(const pamhd_cfg& c, const Layout& L, Step_Params& P, con
 		if (P.active[d] and not P.periodic[d] and own_side and active_count > 1) needs_boundary_speeds = true;
 	}
 	const Tile_Kind kind = step_tile(c.solver, P.active[1], P.active[2]);
-	const long long tiles = (long long)((c.n[0] + 31) / 32) * ((c.n[1] + kind.rows - 1) / kind.rows);
+	tile_shape(kind, c.n[0], c.n[1], P.tw, P.th);
+	const long long tiles = (long long)((c.n[0] + P.tw - 1) / P.tw) * ((c.n[1] + P.th - 1) / P.th);
 	P.kchunk = planes_per_block(tiles, c.n[2], kind.resident());
 	if (kchunk_cap > 0) P.kchunk = std::min(P.kchunk, kchunk_cap);
 	return needs_boundary_speeds;

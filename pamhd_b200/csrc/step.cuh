@@ -104,6 +104,7 @@ struct Step_Params {
 	double* dt_hist;
 	int hist_len;
 	int phase;           // step index mod 3
+	int tw, th;          // columns of a tile along x and y
 	int kchunk;          // z planes per block
 	double forced_dt;    // >= 0: the step's dt (a prescribed schedule); < 0: the CFL rule
 	int kpart;           // z planes a launch computes: 0 all, 1 the first and last only, 2 the others
@@ -111,7 +112,8 @@ struct Step_Params {
 	const Inflow_Table* inflow;  // [3][2] by dimension and side (lo, hi) in device memory, or nullptr
 };
 
-// the kernel instance a grid or batch runs: solver, tile rows (1: y inactive), whether there are z faces
+// the kernel instance a grid or batch runs: solver, tile size (32 x rows threads; rows 1: y
+// inactive), whether there are z faces
 struct Tile_Kind {
 	int solver;
 	int rows;
@@ -124,6 +126,12 @@ struct Tile_Kind {
 		return rows == 8 ? 2 : (rows == 4 and not zact and solver != PAMHD_ROE_ATHENA ? 4 : 3);
 	}
 	int resident() const { return resident_of(solver, rows, zact); }
+	// columns along x of a tile without z faces: 32, or 31 with one row, whose last thread then takes
+	// the tile's +x face in the same pass
+	static constexpr int flat_width_of(const int rows) { return rows == 1 ? 31 : 32; }
+	// records of a plane of a tile and its halo, the most its shared memory holds: 32 x 8 columns need
+	// 336, 22 x 11 308; 32 x 4 need 200, 42 x 3 216; 31 x 1 33
+	static constexpr int records_of(const int rows) { return rows == 8 ? 352 : (rows == 4 ? 216 : 33); }
 };
 
 // launchers (step_kernels.cu)

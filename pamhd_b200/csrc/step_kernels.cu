@@ -4,8 +4,8 @@ Kernels of the fused finite-volume MHD step (sm_100a, FP64 CUDA cores).
 step_kernel<SOLVER, TY, ZACT> - one launch = one whole step (the reference's
   get_all_fluxes + update_mhd_state + minimize_timestep, mhd/solve.hpp:
   1702-1811, :1518-1614, :1933-2014, in their cell-centred form):
-  * a block owns a 32 x TY column tile and marches along z through a chunk
-    of planes ("2.5-D blocking");
+  * a block of 32 TY threads owns a tile of about as many columns and
+    marches along z through a chunk of planes ("2.5-D blocking");
   * each plane of the tile plus a one-cell halo in x and y is read once
     from HBM (coalesced along x), its derived quantities (1/rho, pressure,
     fast speeds along x, y, z) computed once per cell into shared memory;
@@ -21,8 +21,8 @@ step_kernel<SOLVER, TY, ZACT> - one launch = one whole step (the reference's
     three-slot ring; the next step's dt is computed from that ring by
     every block at kernel start, so consecutive steps never wait on the
     host and can be replayed from a CUDA graph.
-Only the redundant halo faces of each tile (1/32 + 1/TY of the x/y faces)
-and one z plane per chunk are solved twice.
+Only the redundant halo faces of each tile (with 32 x 8 columns, 1/32 + 1/8
+of the x/y faces) and one z plane per chunk are solved twice.
 */
 #include <cuda_runtime.h>
 
@@ -52,9 +52,8 @@ template <int SOLVER> struct Flux_Rows { static constexpr int N = SOLVER == PAMH
 
 template <int TY, bool ZACT, int NF = 8> struct Tile {
 	static constexpr int JO = (TY > 1) ? 1 : 0;            // halo rows exist when y is active
-	static constexpr int W = TX + 2;                       // record row width (halo columns)
-	static constexpr int H = TY + 2 * JO;                  // record rows
-	static constexpr int CELLS = W * H;
+	static constexpr int CELLS = Tile_Kind::records_of(TY);  // records of a plane, halo included
+	static constexpr int FLAT = Tile_Kind::flat_width_of(TY);
 	static constexpr int REC = NV * CELLS;                 // doubles per plane slot
 	static constexpr int SLOTS = ZACT ? 2 : 1;             // planes whose records are held
 	// the record slots; the x and the y face fluxes of a plane, indexed as the record of the cell on
@@ -258,27 +257,6 @@ __device__ __forceinline__ void flush_speeds(const Step_Params& P, double smax[3
 	}
 }
 
-// ghost copy of COPY sides: density, velocity, pressure and field of the neighbour
-// (mhd/boundaries.hpp:818-1030 with the constant-pressure field copy)
-__device__ __forceinline__ void copy_state(const double U[8], const Gas& g, double C[8])
-{
-	const double ir = 1.0 / U[0];
-	const double vx = U[1] * ir, vy = U[2] * ir, vz = U[3] * ir;
-	const double b2 = U[5] * U[5] + U[6] * U[6] + U[7] * U[7];
-	const double p = (U[4] - 0.5 * ir * (U[1] * U[1] + U[2] * U[2] + U[3] * U[3]) - 0.5 * g.inv_mu0 * b2)
-		* (g.gamma - 1.0);
-	C[0] = U[0];
-	C[1] = U[0] * vx;
-	C[2] = U[0] * vy;
-	C[3] = U[0] * vz;
-	const double ic = 1.0 / C[0];
-	const double wx = C[1] * ic, wy = C[2] * ic, wz = C[3] * ic;
-	C[4] = p / (g.gamma - 1.0) + 0.5 * C[0] * (wx * wx + wy * wy + wz * wz) + 0.5 * g.inv_mu0 * b2;
-	C[5] = U[5];
-	C[6] = U[6];
-	C[7] = U[7];
-}
-
 __device__ __forceinline__ void store_cell(double* out, const Layout& L, const int i, const int j,
                                            const int k, const double U[8])
 {
@@ -296,7 +274,10 @@ __device__ __forceinline__ const double* inflow_at(const Inflow_Table& T, const 
 }
 
 /*
-New state of an interior cell plus its periodic image / COPY ghost, and the
+New state of an interior cell plus its periodic image / COPY ghost (the
+neighbour's density, velocity, pressure and field, mhd/boundaries.hpp:
+818-1030, which is its state: taking the energy apart and together again
+cost every warp at an open side two IEEE divisions per cell), and the
 ghost of a time-stamped VALUE side at the time the new state holds: the
 step's start time plus dt, as begin_step advances the clock.
 */
@@ -315,10 +296,8 @@ __device__ void write_cell(const Step_Params& P, const int i, const int j, const
 				t[d] = n;
 				store_cell(P.out, P.L, t[0], t[1], t[2], U);
 			} else if (P.bc_lo[d] == PAMHD_BC_COPY) {
-				double C[8];
-				copy_state(U, P.gas, C);
 				t[d] = -1;
-				store_cell(P.out, P.L, t[0], t[1], t[2], C);
+				store_cell(P.out, P.L, t[0], t[1], t[2], U);
 			} else if (P.bc_lo[d] == PAMHD_BC_VALUE and P.inflow != nullptr and P.inflow[2 * d].states != nullptr) {
 				t[d] = -1;
 				store_cell(P.out, P.L, t[0], t[1], t[2], inflow_at(P.inflow[2 * d], __ldcg(&P.clock[P.phase].t) + dt));
@@ -330,10 +309,8 @@ __device__ void write_cell(const Step_Params& P, const int i, const int j, const
 				t[d] = -1;
 				store_cell(P.out, P.L, t[0], t[1], t[2], U);
 			} else if (P.bc_hi[d] == PAMHD_BC_COPY) {
-				double C[8];
-				copy_state(U, P.gas, C);
 				t[d] = n;
-				store_cell(P.out, P.L, t[0], t[1], t[2], C);
+				store_cell(P.out, P.L, t[0], t[1], t[2], U);
 			} else if (P.bc_hi[d] == PAMHD_BC_VALUE and P.inflow != nullptr and P.inflow[2 * d + 1].states != nullptr) {
 				t[d] = n;
 				store_cell(P.out, P.L, t[0], t[1], t[2], inflow_at(P.inflow[2 * d + 1], __ldcg(&P.clock[P.phase].t) + dt));
@@ -420,8 +397,8 @@ __device__ __forceinline__ void solve_z(const Step_Params& P, const double* rec_
 }
 
 /*
-One x or y face (axis a, 0 or 1, known only at run time) on the negative
-side of record position rr of a slot.  The x and y faces of a plane share
+One x or y face (axis a, 0 or 1, known only at run time) between record
+positions rl and rr of a slot.  The x and y faces of a plane share
 this one inlined solver instance (half the code of one instance per axis,
 which the instruction cache rewards).  The rotation into the face frame is
 a choice of record rows to read, two offsets per side: x reads rows m_x,
@@ -429,13 +406,12 @@ m_y, m_z; y reads m_y, m_z (one row on) and m_x.  The unscaled flux goes to
 out[r][rr] in the face frame, Flux_Rows<SOLVER>::N rows (the caller rotates
 it back).  Returns the face's signal speed.
 */
-template <int SOLVER, int TY, class T>
+template <int SOLVER, bool ZACT, class T>
 __device__ __forceinline__ double solve_xy(const Step_Params& P, const double* rec, const uint8_t* bad,
-                                           const int rr, const int a, double* const out, const int gx0,
-                                           const int gy0, const int k)
+                                           const int rl, const int rr, const int a, double* const out,
+                                           const int gx0, const int gy0, const int k)
 {
 	constexpr int C = T::CELLS;
-	const int rl = rr - (a == 0 ? 1 : T::W);
 	const int near = a * C, far = a == 0 ? 2 * C : 0;
 	auto side = [&](const int r) {
 		const double* const c = rec + r;
@@ -466,7 +442,13 @@ __device__ __forceinline__ double solve_xy(const Step_Params& P, const double* r
 	uint32_t flag = 0;
 	const auto pick = [&](const bool left) { return side(left ? rl : rr); };
 	const double sp = solve_face<SOLVER>(L, R, P.gas, F, flag, pick);
-	if (flag != 0) record_failure(P, flag, gx0 + rl % T::W - 1, gy0 + rl / T::W - T::JO, k, a + 1);
+	if (flag != 0) {
+		// the face's negative cell: one of the tile's rows (the first the halo row below), or the column
+		// left of it
+		const int tw = ZACT ? P.tw : T::FLAT + 2, columns = ZACT ? (P.th + 2 * T::JO) * tw : 1 << 30;
+		const int i = rl < columns ? rl % tw - (ZACT ? 0 : 1) : -1, j = rl < columns ? rl / tw - T::JO : rl - columns;
+		record_failure(P, flag, gx0 + i, gy0 + j, k, a + 1);
+	}
 	out[rr] = F[0];
 	out[C + rr] = F[1];
 	out[2 * C + rr] = F[2];
@@ -495,13 +477,14 @@ A step of a grid that stopped: the tile's cells are copied into the new
 state unchanged, with the ghosts a step writes, so that both states hold
 the failing step's result.  CO: loads at L2 (see load_record).
 */
-template <int TY, bool CO>
+template <bool CO>
 __device__ void tile_hold(const Step_Params& P, const int bx, const int by, const int bz)
 {
 	int kb, ke;
 	tile_planes(P, bz, kb, ke);
-	const int gx = bx * TX + threadIdx.x, gy = by * TY + threadIdx.y;
-	if (gx >= P.L.n[0] or gy >= P.L.n[1]) return;
+	const int ty = threadIdx.x / P.tw, tx = threadIdx.x - ty * P.tw;
+	const int gx = bx * P.tw + tx, gy = by * P.th + ty;
+	if (ty >= P.th or gx >= P.L.n[0] or gy >= P.L.n[1]) return;
 	for (int k = kb; k < ke; k++) {
 		const long long off = P.L.offset(gx, gy, k);
 		double U[8];
@@ -512,7 +495,7 @@ __device__ void tile_hold(const Step_Params& P, const int bx, const int by, cons
 }
 
 /*
-One work item of a step: the tile (bx, by) of 32 x TY columns over the z
+One work item of a step: the tile (bx, by) of tw x th columns over the z
 chunk bz, marched plane by plane; the face speeds are folded into
 s0, s1, s2 and zero (flushed by the caller).  Shared by the single-grid
 and the batched kernels, so that both compute the same bits.
@@ -548,45 +531,55 @@ __device__ __forceinline__ void tile_step(const Step_Params& P, double* const sm
 
 	constexpr bool YACT = TY > 1;
 	const int nx = P.L.n[0], ny = P.L.n[1];
-	const int tx = threadIdx.x, ty = threadIdx.y;
-	const int warp = ty, lane = tx;  // TX = 32: one warp per tile row
-	// warps given the halo columns and the tile's extra +x / +y faces (kept apart from the
-	// warps loading the halo rows, so that no warp does more than one extra pass per phase)
-	static_assert(TY == 1 or TY >= 4, "tile rows: 1 or at least 4");
-	constexpr int XHALO_WARP = TY >= 4 ? 2 : 0;
-	constexpr int XFACE_WARP = TY >= 4 ? TY - 2 : 0;
-	constexpr int YFACE_WARP = TY >= 4 ? TY - 1 : 0;
-	const int gx0 = bx * TX, gy0 = by * TY;
+	constexpr int THREADS = TX * TY;
+	// the tile's columns one per thread, x fastest; the threads past them (tw th <= THREADS) own none
+	// (grids without z faces keep 32 x TY, or 31 x 1 columns, known at compile time)
+	const int tw = ZACT ? P.tw : T::FLAT, th = ZACT ? P.th : TY, t = threadIdx.x;
+	const int ty = t / tw, tx = t - ty * tw;
+	const int gx0 = bx * tw, gy0 = by * th;
 	const int gx = gx0 + tx, gy = gy0 + ty;
-	const bool own = gx < nx and gy < ny;
+	const bool own = ty < th and gx < nx and gy < ny;
 	// the +x / +y ghost of a partial tile lies inside the tile's own columns / rows
-	const bool stage = gx <= nx and (TY == 1 ? gy == 0 : gy <= ny);
+	const bool stage = ty < th and gx <= nx and (TY == 1 ? gy == 0 : gy <= ny);
 	// the planes of this block
 	int kb, ke;
 	tile_planes(P, bz, kb, ke);
 	const int kfirst = ZACT ? kb - 1 : kb;
 	const int klast = ZACT ? ke : ke - 1;
-	const int ri = (ty + T::JO) * T::W + tx + 1;
+	// record positions.  Tiles that march in z: the rows of columns, the halo rows first and last, tw
+	// apart, so that a warp's own cells are 32 consecutive doubles whatever tw is (a row pitch of
+	// tw + 2 makes two-way bank conflicts wherever a warp crosses a row's end); then the halo columns
+	// left and right.  Others, whose rows are warps: the halo columns at their rows' ends.
+	const int pitch = ZACT ? tw : T::FLAT + 2;
+	const int left_column = (th + 2 * T::JO) * tw, right_column = left_column + th;
+	const auto at = [&](const int row, const int x) { return (row + T::JO) * pitch + x + (ZACT ? 0 : 1); };
+	const auto left_of_row = [&](const int row) { return ZACT ? left_column + row : at(row, -1); };
+	const auto right_of_row = [&](const int row) { return ZACT ? right_column + row : at(row, tw); };
+	const int ri = at(ty, tx);
+	const int r_east = ZACT and tx == tw - 1 ? right_of_row(ty) : ri + 1;
 	// the flux terms are dt F / dx: dt / dx once per axis and cell
 	const double cx = dt * P.inv_len[0], cy = dt * P.inv_len[1], cz = dt * P.inv_len[2];
 
-	// this thread's halo cell of planes with x / y faces, if any: the rows below / above the tile on
-	// warps 0 and 1, the columns left / right of it on warp 2 (warp 0 when y is inactive)
+	// this thread's halo cell of planes with x / y faces, if any: first the rows below and above the
+	// tile, then the columns left and right of it
 	int hri = -1;
 	long long hoff = 0;
-	if (YACT and warp < 2) {
-		const int hy = warp == 1 ? gy0 + TY : gy0 - 1;
-		if (gx < nx and hy <= ny) {
-			hri = (warp == 1 ? TY + 1 : 0) * T::W + lane + 1;
-			hoff = P.L.offset(gx, hy, 0);
-		}
-	} else if (warp == XHALO_WARP and lane < 2 * TY) {
-		const int row = lane % TY;
-		const bool right = lane >= TY;
-		const int hx = right ? gx0 + TX : gx0 - 1;
-		if (gy0 + row < ny and hx <= nx) {
-			hri = (row + T::JO) * T::W + (right ? TX + 1 : 0);
-			hoff = P.L.offset(hx, gy0 + row, 0);
+	{
+		const int rows = YACT ? 2 * tw : 0;
+		if (t < rows) {
+			const bool top = t >= tw;
+			const int x = top ? t - tw : t, hy = top ? gy0 + th : gy0 - 1;
+			if (gx0 + x < nx and hy <= ny) {
+				hri = at(top ? th : -1, x);
+				hoff = P.L.offset(gx0 + x, hy, 0);
+			}
+		} else if (t < rows + 2 * th) {
+			const bool right = t >= rows + th;
+			const int y = t - rows - (right ? th : 0), hx = right ? gx0 + tw : gx0 - 1;
+			if (gy0 + y < ny and hx <= nx) {
+				hri = right ? right_of_row(y) : left_of_row(y);
+				hoff = P.L.offset(hx, gy0 + y, 0);
+			}
 		}
 	}
 	const long long col = P.L.offset(gx, gy, 0);
@@ -603,15 +596,32 @@ __device__ __forceinline__ void tile_step(const Step_Params& P, double* const sm
 		return cfz;
 	};
 
-	// the x and y faces this thread solves, one bit each: 0 its -x face, 1 one of the tile's +x faces,
-	// 2 its -y face, 3 one of the tile's +y faces; the +x and +y faces are a further pass of one warp
-	// each, at record position extra
-	uint32_t tasks = 0;
-	if (gx <= nx and gy < ny) tasks |= 1u;
-	if (warp == XFACE_WARP and lane < TY and gx0 + TX <= nx and gy0 + lane < ny) tasks |= 2u;
-	if (YACT and gy <= ny and gx < nx) tasks |= 4u;
-	if (YACT and warp == YFACE_WARP and gy0 + TY <= ny and gx < nx) tasks |= 8u;
-	const int extra_x = (lane + T::JO) * T::W + TX + 1, extra_y = (TY + T::JO) * T::W + lane + 1;
+	// the x and y faces this thread solves, at most one per pass, as positive record position |
+	// (ZACT) negative one << 10 | axis << 20, or -1: an owner its -x and its -y face; the tile's +x and
+	// +y faces (numbered in this order) go to the threads without a cell, two each, and what they
+	// leave to a further pass of the last warps.  32 x TY tiles of one plane (every thread owns a
+	// column) give the last two warps a pass each for the +x and the +y faces, so that a pass has one
+	// axis, known to the whole warp (512^2 Roe: 66 us per step, 70 with mixed axes)
+	constexpr int NONE = -1;
+	const auto face_of = [](const int rr, const int rl, const int a) { return rr | (ZACT ? rl << 10 : 0) | (a << 20); };
+	const auto extra = [&](const int e) -> int {
+		if (e < th) return (gx0 + tw <= nx and gy0 + e < ny) ? face_of(right_of_row(e), at(e, tw - 1), 0) : NONE;
+		const int x = e - th;
+		return (YACT and x < tw and gy0 + th <= ny and gx0 + x < nx) ? face_of(at(th, x), at(th - 1, x), 1) : NONE;
+	};
+	const int spare = THREADS - tw * th;
+	int face0 = NONE, face1 = NONE;
+	if (ty < th) {
+		if (gx <= nx and gy < ny) face0 = face_of(ri, tx == 0 ? left_of_row(ty) : ri - 1, 0);
+		if (YACT and gy <= ny and gx < nx) face1 = face_of(ri, ri - pitch, 1);
+	} else {
+		face0 = extra(t - tw * th);
+		if (YACT) face1 = extra(t - tw * th + spare);
+	}
+	const int last = THREADS - 1 - t;
+	const int face2 = ZACT ? extra(2 * spare + last)
+	                : (YACT and last >= 32 and last - 32 < th ? extra(last - 32) : NONE);
+	const int face3 = not ZACT and YACT and last < tw ? extra(th + last) : NONE;
 	// a cell on the grid's x or y edge also writes a ghost
 	const bool edge = gx == 0 or gx == nx - 1 or gy == 0 or gy == ny - 1;
 
@@ -633,20 +643,18 @@ __device__ __forceinline__ void tile_step(const Step_Params& P, double* const sm
 
 		if (inner) {
 			__syncthreads();
-			// (b) x and y faces, all through one call site; s0 and s1 swap places from axis to axis
+			// (b) x and y faces, all through one call site
 			#pragma unroll 1
-			for (int task = 0; task < (YACT ? 4 : 2); task++) {
-				const int a = task >> 1;
-				if ((tasks >> task) & 1u) {
-					const int rr = (task & 1) == 0 ? ri : (a == 0 ? extra_x : extra_y);
-					const double sp = solve_xy<SOLVER, TY, T>(P, rec, bad, rr, a, fx + a * NF * T::CELLS, gx0, gy0, k);
-					s0 = larger(sp, s0);
+			for (int pass = 0; pass < (ZACT ? 3 : (YACT ? 4 : 1)); pass++) {
+				// own x, own y, further ones; or (one plane) own x, further x, own y, further y
+				const int face = pass == 0 ? face0 : (pass == (ZACT ? 1 : 2) ? face1 : (pass == 3 ? face3 : face2));
+				if (face >= 0) {
+					const int a = ZACT ? face >> 20 : pass >> 1;
+					const int rr = face & 1023, rl = ZACT ? (face >> 10) & 1023 : rr - (a == 0 ? 1 : pitch);
+					const double sp = solve_xy<SOLVER, ZACT, T>(P, rec, bad, rl, rr, a, fx + a * NF * T::CELLS, gx0, gy0, k);
+					const double m = larger(sp, a == 0 ? s0 : s1);
+					if (a == 0) s0 = m; else s1 = m;
 					zero = zero or no_speed(sp);
-				}
-				if (YACT and (task & 1)) {
-					const double t = s0;
-					s0 = s1;
-					s1 = t;
 				}
 			}
 			if (ZACT) bar.arrive();
@@ -677,8 +685,8 @@ __device__ __forceinline__ void tile_step(const Step_Params& P, double* const sm
 				for (int v = 0; v < 8; v++) {
 					Un[v] = rec[v * T::CELLS + ri];
 					if (XROW[v] >= 0) {
-						const double* f = fx + XROW[v] * T::CELLS + ri;
-						Un[v] = __fma_rn(__dsub_rn(f[0], f[1]), cx, Un[v]);
+						const double* f = fx + XROW[v] * T::CELLS;
+						Un[v] = __fma_rn(__dsub_rn(f[ri], f[r_east]), cx, Un[v]);
 					}
 				}
 				if (YACT) {
@@ -686,7 +694,7 @@ __device__ __forceinline__ void tile_step(const Step_Params& P, double* const sm
 					for (int v = 0; v < 8; v++) {
 						if (YROW[v] >= 0) {
 							const double* f = fy + YROW[v] * T::CELLS + ri;
-							Un[v] = __fma_rn(__dsub_rn(f[0], f[T::W]), cy, Un[v]);
+							Un[v] = __fma_rn(__dsub_rn(f[0], f[pitch]), cy, Un[v]);
 						}
 					}
 				}
@@ -738,9 +746,9 @@ __global__ void __launch_bounds__(TX * TY, Tile_Kind::resident_of(SOLVER, TY, ZA
 		__syncthreads();
 		const bool first = w.y == 0 and w.z == 0 and w.w == 0;
 		const double dt = begin_step(sp, &s_dt, first, &s_stop);
-		const int tiles_x = (sp.L.n[0] + TX - 1) / TX;
+		const int tiles_x = (sp.L.n[0] + sp.tw - 1) / sp.tw;
 		if (s_stop) {
-			tile_hold<TY, false>(sp, w.y % tiles_x, w.y / tiles_x, w.z);
+			tile_hold<false>(sp, w.y % tiles_x, w.y / tiles_x, w.z);
 			continue;
 		}
 		double s0 = 0.0, s1 = 0.0, s2 = 0.0;
@@ -866,7 +874,7 @@ __global__ void __launch_bounds__(TX * TY, Tile_Kind::resident_of(SOLVER, TY, ZA
 	const bool first_block = blockIdx.x == 0 and blockIdx.y == 0 and blockIdx.z == 0;
 	const double dt = begin_step(P, &s_dt, first_block, &s_stop);
 	if (s_stop) {
-		if (blockIdx.z < gridDim.z - P.boundary) tile_hold<TY, false>(P, blockIdx.x, blockIdx.y, blockIdx.z);
+		if (blockIdx.z < gridDim.z - P.boundary) tile_hold<false>(P, blockIdx.x, blockIdx.y, blockIdx.z);
 		return;
 	}
 	double s0 = 0.0, s1 = 0.0, s2 = 0.0;
@@ -875,7 +883,7 @@ __global__ void __launch_bounds__(TX * TY, Tile_Kind::resident_of(SOLVER, TY, ZA
 	if ((int)blockIdx.z >= chunks) {
 		double smax[3] = {0.0, 0.0, 0.0};
 		const long long block = (blockIdx.z - chunks) * (long long)gridDim.x * gridDim.y + blockIdx.y * gridDim.x + blockIdx.x;
-		boundary_faces<SOLVER, false>(P, block * (TX * TY) + threadIdx.y * TX + threadIdx.x,
+		boundary_faces<SOLVER, false>(P, block * (TX * TY) + threadIdx.x,
 		                              P.boundary * (long long)gridDim.x * gridDim.y * (TX * TY), smax, zero);
 		flush_speeds(P, smax, zero);
 		return;
@@ -963,9 +971,7 @@ __global__ void fill_ghosts_kernel(const Step_Params P, double* state, const Gho
 			} else if (kind == PAMHD_BC_COPY) {
 				s[d] = side ? P.L.n[d] - 1 : 0;
 				const long long o = P.L.offset(s[0], s[1], s[2]);
-				double W[8];
-				for (int v = 0; v < 8; v++) W[v] = state[v * P.L.var + o];
-				copy_state(W, P.gas, U);
+				for (int v = 0; v < 8; v++) U[v] = state[v * P.L.var + o];
 			} else {
 				for (int v = 0; v < 8; v++) U[v] = side ? V.hi[d][v] : V.lo[d][v];
 			}
@@ -1066,9 +1072,9 @@ __global__ void __launch_bounds__(TX * TY, Tile_Kind::resident_of(SOLVER, TY, ZA
 		if (w.w == 0) {
 			const bool first = w.y == 0 and w.z == 0;
 			const double dt = begin_step(sp, &s_dt, first, &s_stop);
-			const int tiles_x = (sp.L.n[0] + TX - 1) / TX;
+			const int tiles_x = (sp.L.n[0] + sp.tw - 1) / sp.tw;
 			if (s_stop) {
-				tile_hold<TY, true>(sp, w.y % tiles_x, w.y / tiles_x, w.z);
+				tile_hold<true>(sp, w.y % tiles_x, w.y / tiles_x, w.z);
 			} else {
 				tile_step<SOLVER, TY, ZACT, true>(sp, smem, bar, dt, w.y % tiles_x, w.y / tiles_x, w.z, smax[0], smax[1],
 				                            smax[2], zero);
@@ -1234,7 +1240,8 @@ static int status_of(const cudaError_t e)
 }
 
 /*
-The single-grid step's tile.  3-D grids: 32 x 8, two blocks of 256 threads
+The single-grid step's tile (its size; tile_shape() lays it out).  3-D
+grids: 32 x 8, two blocks of 256 threads
 per SM (a taller tile solves fewer halo faces and records per cell).  2-D
 grids: 32 x 4, four blocks of 128 threads per SM: the same 16 warps in
 blocks that wait for fewer others, and twice the blocks on small grids
@@ -1268,9 +1275,9 @@ int launch_step(const Step_Params& P, const int solver, cudaStream_t stream)
 	                 : (nz + P.kchunk - 1) / P.kchunk;
 	if (chunks < 1) return PAMHD_OK;  // no planes between the first and the last
 	return with_kind(step_tile(solver, P.active[1] != 0, P.active[2] != 0), [&](auto solver_, auto rows, auto zact) {
-		const dim3 grid((P.L.n[0] + TX - 1) / TX, (P.L.n[1] + rows() - 1) / rows(), chunks + P.boundary);
+		const dim3 grid((P.L.n[0] + P.tw - 1) / P.tw, (P.L.n[1] + P.th - 1) / P.th, chunks + P.boundary);
 		step_kernel<solver_(), rows(), zact()>
-			<<<grid, dim3(TX, rows()), tile_bytes<solver_(), rows(), zact()>(), stream>>>(P);
+			<<<grid, TX * rows(), tile_bytes<solver_(), rows(), zact()>(), stream>>>(P);
 		return status_of(cudaGetLastError());
 	});
 }
@@ -1319,7 +1326,7 @@ int launch_batch_run(const Step_Params* even, const Step_Params* odd, const int4
 	return with_kind(kind, [&](auto solver, auto rows, auto zact) {
 		cudaLaunchConfig_t c = {};
 		c.gridDim = dim3(grid);
-		c.blockDim = dim3(TX, rows());
+		c.blockDim = TX * rows();
 		c.dynamicSmemBytes = tile_bytes<solver(), rows(), zact()>();
 		c.stream = stream;
 		cudaLaunchAttribute a[1];
@@ -1338,7 +1345,7 @@ int launch_batch_step(const Step_Params* boxes, const int4* items, const int nit
 {
 	return with_kind(kind, [&](auto solver, auto rows, auto zact) {
 		batch_step_kernel<solver(), rows(), zact()>
-			<<<grid, dim3(TX, rows()), tile_bytes<solver(), rows(), zact()>(), stream>>>(boxes, items, nitems, phase);
+			<<<grid, TX * rows(), tile_bytes<solver(), rows(), zact()>(), stream>>>(boxes, items, nitems, phase);
 		return status_of(cudaGetLastError());
 	});
 }
@@ -1368,7 +1375,7 @@ int boundary_layers(const Step_Params& P, const int solver)
 	}
 	// about a face per thread
 	const int rows = step_tile(solver, P.active[1] != 0, P.active[2] != 0).rows;
-	const long long layer = (long long)((P.L.n[0] + TX - 1) / TX) * ((P.L.n[1] + rows - 1) / rows) * TX * rows;
+	const long long layer = (long long)((P.L.n[0] + P.tw - 1) / P.tw) * ((P.L.n[1] + P.th - 1) / P.th) * TX * rows;
 	return int(min(1024LL, (faces + layer - 1) / layer));
 }
 

@@ -42,11 +42,14 @@ def pair(port, n, solver, lengths, gamma, mu0, cfl, bc_lo=(0, 0, 0), bc_hi=(0, 0
 # ---------------------------------------------------------------- solver level
 
 @pytest.mark.parametrize("bc", ["periodic", "copy"])
-@pytest.mark.parametrize("n", [(33, 9, 2), (70, 17, 37), (31, 40, 3), (64, 8, 19)])
+@pytest.mark.parametrize("n", [(33, 9, 2), (70, 17, 37), (31, 40, 3), (64, 8, 19), (100, 20, 5), (36, 36, 7),
+                               (17, 45, 6)])
 def test_short_z_chunks_match_oracle(port, n, bc):
     """Small 3-D grids, whose blocks take a few planes each (the last chunk of 37 planes a single
-    one) and whose tiles end one cell short of, at and one cell past 32 columns and 8 rows; on open
-    sides the step's own blocks solve the ghost-ghost faces.  Per step, the bar of this file."""
+    one) and whose tiles end one cell short of, at and one cell past 32 columns and 8 rows, or have
+    other shapes (25 x 10, 18 x 12 and 17 x 15 columns on the last three), with threads that own no
+    cell; on open sides the step's own blocks solve the ghost-ghost faces.  Per step, the bar of this
+    file."""
     kinds = ((pg.BC_COPY,) * 3 if bc == "copy" else (pg.BC_PERIODIC,) * 3,) * 2
     L = (0.1, 0.12, 0.09)
     U = states.smooth_3d((n[2], n[1], n[0]), np.random.default_rng(3))
