@@ -248,6 +248,9 @@ int pamhd_gpu_create(const pamhd_cfg* cfg, pamhd_ctx** out)
 	if (prepare_step_kernels(step_tile(internal.solver, internal.n[1] > 1, internal.n[2] > 1)) != PAMHD_OK) {
 		return fail(PAMHD_ERR_CUDA);
 	}
+	if (line_run_fits(x->base, internal.solver) and prepare_line_run(internal.solver) != PAMHD_OK) {
+		return fail(PAMHD_ERR_CUDA);
+	}
 	if (reset_run_state(*x) != PAMHD_OK) return fail(PAMHD_ERR_CUDA);
 	if (cudaStreamSynchronize(x->stream) != cudaSuccess) return fail(PAMHD_ERR_CUDA);
 	*out = x;
@@ -367,6 +370,18 @@ int pamhd_gpu_steps(pamhd_ctx* x, const int32_t nsteps, const double t_end)
 	PAMHD_TRY(check(cudaSetDevice(x->device)));
 	PAMHD_TRY(set_control(*x, -1.0, t_end));
 	int left = nsteps;
+	if (line_run_fits(x->base, x->cfg.solver)) {
+		// one launch, of a few milliseconds at most
+		while (left > 1) {
+			const int steps = std::min(left, 2048);
+			Step_Params P = params_for(*x, x->steps, x->cur);
+			P.out = x->state[x->cur ^ (steps & 1)];
+			PAMHD_TRY(launch_line_run(P, x->state[x->cur ^ (steps & 1) ^ 1], steps, x->cfg.solver, x->stream));
+			x->cur ^= steps & 1;
+			x->steps += steps;
+			left -= steps;
+		}
+	}
 	while (left > 0 and x->steps % GRAPH_STEPS != 0) {
 		PAMHD_TRY(issue_step(*x));
 		left--;

@@ -136,6 +136,10 @@ struct Tile_Kind {
 
 // launchers (step_kernels.cu)
 int launch_step(const Step_Params& P, int solver, cudaStream_t stream);
+// nsteps steps of a small 1-D grid in one launch; P.out: the buffer of the last step, other: the other
+bool line_run_fits(const Step_Params& P, int solver);
+int prepare_line_run(int solver);
+int launch_line_run(const Step_Params& P, double* other, int nsteps, int solver, cudaStream_t stream);
 // block layers for the ghost-ghost faces of a grid with non-periodic sides (Step_Params::boundary)
 int boundary_layers(const Step_Params& P, int solver);
 int launch_scatter(const double* packed, double* var_base, const Layout& L, cudaStream_t stream);

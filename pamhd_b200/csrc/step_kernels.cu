@@ -24,6 +24,7 @@ step_kernel<SOLVER, TY, ZACT> - one launch = one whole step (the reference's
 Only the redundant halo faces of each tile (with 32 x 8 columns, 1/32 + 1/8
 of the x/y faces) and one z plane per chunk are solved twice.
 */
+#include <cooperative_groups.h>
 #include <cuda_runtime.h>
 
 #include <type_traits>
@@ -1100,6 +1101,243 @@ __global__ void __launch_bounds__(TX * TY, Tile_Kind::resident_of(SOLVER, TY, ZA
 	}
 }
 
+// ------------------------------------------------------------------ a 1-D grid's steps in one launch
+
+/*
+nsteps steps of a small 1-D grid in one launch of one thread-block cluster:
+a thread per cell, its state in registers from the first step to the last.
+A step is bound by latency (one face's solve, some 2 us with the barrier),
+where a launch per step spends most of its time starting up, reading the
+state and the last step's speeds back and draining: 1000 cells HLLD took
+7.1 us per step as graph-replayed launches and take 3.0 us here.
+
+Per step every thread derives its cell's record into shared memory (two
+buffers alternate), the tile's end cells also into the neighbouring block's
+halo (distributed shared memory), and one cluster barrier makes them, and
+the blocks' speed maxima of the step before, visible; then a thread solves
+its cell's -x face (one thread more the last +x face) and, after a block
+barrier, updates its cell.  The arithmetic is the step kernel's, bit for
+bit.  A step after a failing one is not taken (see stopped_before).
+*/
+template <int SOLVER> struct Line { static constexpr int THREADS = SOLVER == PAMHD_ROE_ATHENA ? 256 : 512; };
+constexpr int LINE_REC = 11;   // rho, mom xyz, E, B xyz, 1/rho, total pressure, cf x
+constexpr int LINE_BLOCKS = 8;
+
+struct Line_Slot {
+	double smax;
+	int zero;
+	int fail;
+};
+
+static size_t line_bytes(const int threads)
+{
+	return (size_t(2 * LINE_REC) * (threads + 2) + size_t(8) * (threads + 1)) * sizeof(double) + size_t(2) * (threads + 2);
+}
+
+template <int SOLVER>
+__global__ void __launch_bounds__(Line<SOLVER>::THREADS) line_run_kernel(const Step_Params P, double* const other,
+                                                                        const int nsteps, const int cells)
+{
+	namespace cg = cooperative_groups;
+	extern __shared__ __align__(16) double smem[];
+	__shared__ Line_Slot slots[2][LINE_BLOCKS];
+	__shared__ double warp_speed[Line<SOLVER>::THREADS / 32];
+	__shared__ int warp_zero[Line<SOLVER>::THREADS / 32];
+	__shared__ int block_fail;
+	const cg::cluster_group cluster = cg::this_cluster();
+	const int rank = cluster.block_rank(), blocks = cluster.num_blocks(), T = blockDim.x, t = threadIdx.x;
+	const int n = P.L.n[0], C = T + 2;
+	const int mine = min(cells, n - rank * cells), last_mine = n - (blocks - 1) * cells;
+	const int i = rank * cells + t;
+	const bool own = t < mine;
+	double* const flux = smem + 2 * LINE_REC * C;
+	uint8_t* const bad = reinterpret_cast<uint8_t*>(flux + 8 * (T + 1));
+
+	// a record at position pos of buffer b in block `to`
+	const auto put = [&](const int to, const int b, const int pos, const double U[8], const Derived& d) {
+		double* const r = cluster.map_shared_rank(smem, to) + b * LINE_REC * C + pos;
+		#pragma unroll
+		for (int v = 0; v < 8; v++) r[v * C] = U[v];
+		r[8 * C] = d.rinv;
+		r[9 * C] = d.pt;
+		r[10 * C] = d.cf[0];
+		cluster.map_shared_rank(bad, to)[b * C + pos] = uint8_t(d.bad);
+	};
+	const auto side = [&](const int b, const int pos) {
+		const double* const r = smem + b * LINE_REC * C + pos;
+		Side s;
+		s.rho = r[0];
+		s.m0 = r[C]; s.m1 = r[2 * C]; s.m2 = r[3 * C];
+		s.E = r[4 * C];
+		s.b0 = r[5 * C]; s.b1 = r[6 * C]; s.b2 = r[7 * C];
+		s.rinv = r[8 * C];
+		s.pt = r[9 * C];
+		s.p = 0.0;  // not read without a background field
+		s.cf = r[10 * C];
+		s.v0 = s.m0 * s.rinv;
+		s.v1 = s.m1 * s.rinv;
+		s.v2 = s.m2 * s.rinv;
+		s.bad = bad[b * C + pos];
+		return s;
+	};
+	const auto load = [&](const int cell, double U[8]) {
+		const long long off = P.L.offset(cell, 0, 0);
+		#pragma unroll
+		for (int v = 0; v < 8; v++) U[v] = P.in[v * P.L.var + off];
+	};
+
+	double U[8] = {};
+	if (own) load(i, U);
+	// constant ghosts
+	if (t == 0) {
+		double G[8];
+		if (rank == 0 and not P.periodic[0] and P.bc_lo[0] == PAMHD_BC_VALUE) {
+			load(-1, G);
+			const Derived d = derive<true, false, false>(G[0], G[1], G[2], G[3], G[4], G[5], G[6], G[7], P.gas);
+			put(rank, 0, 0, G, d);
+			put(rank, 1, 0, G, d);
+		}
+		if (rank == blocks - 1 and not P.periodic[0] and P.bc_hi[0] == PAMHD_BC_VALUE) {
+			load(n, G);
+			const Derived d = derive<true, false, false>(G[0], G[1], G[2], G[3], G[4], G[5], G[6], G[7], P.gas);
+			put(rank, 0, mine + 1, G, d);
+			put(rank, 1, mine + 1, G, d);
+		}
+		block_fail = 0;
+	}
+	double time = P.clock[P.phase].t, dt = P.clock[P.phase].dt;
+	long long steps = P.clock[P.phase].steps;
+	const double max_dt = P.control->max_dt, t_end = P.control->t_end;
+	double smax = __longlong_as_double((long long)P.red[P.phase].smax[0]);
+	bool zero = P.red[P.phase].zero != 0u, stop = stopped_before(P);
+	cluster.sync();   // every block runs; its flags are set
+
+	int s = 0;
+	for (; s < nsteps; s++) {
+		const int b = s & 1;
+		if (own) {
+			const Derived d = derive<true, false, false>(U[0], U[1], U[2], U[3], U[4], U[5], U[6], U[7], P.gas);
+			put(rank, b, t + 1, U, d);
+			if (t == 0) {
+				if (rank > 0) put(rank - 1, b, cells + 1, U, d);
+				else if (P.periodic[0]) put(blocks - 1, b, last_mine + 1, U, d);
+				else if (P.bc_lo[0] == PAMHD_BC_COPY) put(rank, b, 0, U, d);
+			}
+			if (t == mine - 1) {
+				if (rank < blocks - 1) put(rank + 1, b, 0, U, d);
+				else if (P.periodic[0]) put(0, b, 0, U, d);
+				else if (P.bc_hi[0] == PAMHD_BC_COPY) put(rank, b, mine + 1, U, d);
+			}
+		}
+		cluster.sync();
+		if (s > 0) {
+			smax = 0.0;
+			zero = stop = false;
+			for (int r = 0; r < blocks; r++) {
+				const Line_Slot& o = slots[b][r];
+				smax = larger(o.smax, smax);
+				zero = zero or o.zero != 0;
+				stop = stop or o.fail != 0;
+			}
+		}
+		if (stop) break;   // the same in every thread of the cluster
+		// the step's dt (step_dt with one active dimension)
+		double smallest = 0.0;
+		if (not zero and smax > 0.0) smallest = fmin(1.7976931348623157e308, (P.cfl * P.len[0]) / smax);
+		const double cap = max_dt >= 0.0 ? max_dt : t_end - time;
+		dt = cap <= smallest ? cap : smallest;
+		const double cx = dt * P.inv_len[0];
+
+		double speed = 0.0;
+		bool no = false;
+		if (t <= mine) {
+			const Side L = side(b, t), R = side(b, t + 1);
+			double F[8];
+			uint32_t flag = 0;
+			const auto pick = [&](const bool left) { return side(b, left ? t : t + 1); };
+			speed = solve_face<SOLVER>(L, R, P.gas, F, flag, pick);
+			no = no_speed(speed);
+			if (flag != 0) {
+				block_fail = 1;
+				int c = i - 1;
+				if (P.periodic[0] and c < 0) c += n;
+				atomicOr(&P.status->flags, flag);
+				atomicMin(&P.status->first, (((unsigned long long)(c + P.ext[0]) * 4ull + 1ull) << 8) | flag);
+				P.status->fail_step = (unsigned int)(steps + 1);
+			}
+			#pragma unroll
+			for (int v = 0; v < 8; v++) {
+				if (v != 5 or SOLVER == PAMHD_RUSANOV) flux[v * (T + 1) + t] = F[v];
+			}
+		}
+		speed = warp_max(larger(speed, 0.0));
+		no = __any_sync(0xffffffffu, no);
+		if ((t & 31) == 0) {
+			warp_speed[t >> 5] = speed;
+			warp_zero[t >> 5] = no ? 1 : 0;
+		}
+		__syncthreads();
+		if (own) {
+			#pragma unroll
+			for (int v = 0; v < 8; v++) {
+				if (v != 5 or SOLVER == PAMHD_RUSANOV) {
+					const double* const f = flux + v * (T + 1) + t;
+					U[v] = __fma_rn(__dsub_rn(f[0], f[1]), cx, U[v]);
+				}
+			}
+		}
+		if (t < blocks) {
+			Line_Slot o{0.0, 0, block_fail};
+			for (int w = 0; w < (T + 31) / 32; w++) {
+				o.smax = larger(warp_speed[w], o.smax);
+				o.zero |= warp_zero[w];
+			}
+			cluster.map_shared_rank(&slots[b ^ 1][rank], t)[0] = o;
+		}
+		if (rank == 0 and t == 0 and P.dt_hist != nullptr) P.dt_hist[steps % P.hist_len] = dt;
+		time += dt;
+		steps++;
+	}
+	cluster.sync();   // the last step's maxima; no block leaves while another writes to it
+	if (rank == 0 and t == 0) {
+		if (s > 0 and s == nsteps) {
+			smax = 0.0;
+			zero = false;
+			for (int r = 0; r < blocks; r++) {
+				smax = larger(slots[s & 1][r].smax, smax);
+				zero = zero or slots[s & 1][r].zero != 0;
+			}
+		}
+		const int end = (P.phase + nsteps) % 3;
+		Clock& c = P.clock[end];
+		c.t = time;
+		c.dt = s < nsteps ? 0.0 : dt;   // held steps have none
+		c.steps = steps;
+		Speed_Max& r = P.red[end];
+		r.smax[0] = smax > 0.0 ? (unsigned long long)__double_as_longlong(smax) : 0ull;
+		r.smax[1] = r.smax[2] = 0ull;
+		r.zero = zero ? 1u : 0u;
+		Speed_Max& next = P.red[(end + 1) % 3];
+		next.smax[0] = next.smax[1] = next.smax[2] = 0ull;
+		next.zero = 0u;
+	}
+	if (own) {
+		// a grid that stopped holds the failing step's result in both state buffers
+		for (int k = 0; k < (s < nsteps ? 2 : 1); k++) {
+			double* const out = k == 0 ? P.out : other;
+			store_cell(out, P.L, i, 0, 0, U);
+			if (i == 0) {
+				if (P.periodic[0]) store_cell(out, P.L, n, 0, 0, U);
+				else if (P.bc_lo[0] == PAMHD_BC_COPY) store_cell(out, P.L, -1, 0, 0, U);
+			}
+			if (i == n - 1) {
+				if (P.periodic[0]) store_cell(out, P.L, -1, 0, 0, U);
+				else if (P.bc_hi[0] == PAMHD_BC_COPY) store_cell(out, P.L, n, 0, 0, U);
+			}
+		}
+	}
+}
+
 // ------------------------------------------------------------------ solver-level entry
 
 __device__ __forceinline__ Side face_side(const double* s, const double* bg, const bool use_bg, const Gas& g)
@@ -1279,6 +1517,62 @@ int launch_step(const Step_Params& P, const int solver, cudaStream_t stream)
 		step_kernel<solver_(), rows(), zact()>
 			<<<grid, TX * rows(), tile_bytes<solver_(), rows(), zact()>(), stream>>>(P);
 		return status_of(cudaGetLastError());
+	});
+}
+
+// calls body with the solver as an integral constant
+template <class Body> static int with_solver(const int solver, const Body& body)
+{
+	switch (solver) {
+	case PAMHD_RUSANOV: return body(Const<PAMHD_RUSANOV>{});
+	case PAMHD_HLL_ATHENA: return body(Const<PAMHD_HLL_ATHENA>{});
+	case PAMHD_HLLD_ATHENA: return body(Const<PAMHD_HLLD_ATHENA>{});
+	case PAMHD_ROE_ATHENA: return body(Const<PAMHD_ROE_ATHENA>{});
+	default: return PAMHD_ERR_ARGUMENT;
+	}
+}
+
+/*
+Whether a grid's steps run as line_run_kernel: 1-D, cells enough for one per
+thread of eight blocks (a thread more per block for the last face), and no
+side whose state changes with time.
+*/
+bool line_run_fits(const Step_Params& P, const int solver)
+{
+	const int most = LINE_BLOCKS * ((solver == PAMHD_ROE_ATHENA ? 256 : 512) - 1);
+	return P.active[0] and not P.active[1] and not P.active[2] and P.L.n[0] <= most and P.inflow == nullptr
+		and P.forced_dt < 0.0;
+}
+
+int prepare_line_run(const int solver)
+{
+	return with_solver(solver, [](auto s) {
+		return status_of(cudaFuncSetAttribute(line_run_kernel<s()>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+		                                      int(line_bytes(Line<s()>::THREADS))));
+	});
+}
+
+int launch_line_run(const Step_Params& P, double* other, const int nsteps, const int solver, cudaStream_t stream)
+{
+	// 1, 2, 4 or 8 blocks of up to 127 cells (four warps, one per scheduler), then 8 larger ones
+	const int n = P.L.n[0];
+	int blocks = 1;
+	while (blocks < LINE_BLOCKS and n > 127 * blocks) blocks *= 2;
+	const int cells = (n + blocks - 1) / blocks;
+	return with_solver(solver, [&](auto s) {
+		cudaLaunchConfig_t c = {};
+		c.gridDim = dim3(blocks);
+		c.blockDim = dim3((cells + 1 + 31) / 32 * 32);
+		c.dynamicSmemBytes = line_bytes(int(c.blockDim.x));
+		c.stream = stream;
+		cudaLaunchAttribute a[1];
+		a[0].id = cudaLaunchAttributeClusterDimension;
+		a[0].val.clusterDim.x = c.gridDim.x;
+		a[0].val.clusterDim.y = 1;
+		a[0].val.clusterDim.z = 1;
+		c.attrs = a;
+		c.numAttrs = 1;
+		return status_of(cudaLaunchKernelEx(&c, line_run_kernel<s()>, P, other, nsteps, cells));
 	});
 }
 

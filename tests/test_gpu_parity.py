@@ -41,6 +41,59 @@ def pair(port, n, solver, lengths, gamma, mu0, cfl, bc_lo=(0, 0, 0), bc_hi=(0, 0
 
 # ---------------------------------------------------------------- solver level
 
+@pytest.mark.parametrize("bc", ["periodic", "copy", "value"])
+@pytest.mark.parametrize("solver", ["rusanov", "hll_athena", "hlld_athena", "roe_athena"])
+@pytest.mark.parametrize("n", [2, 31, 127, 128, 255, 1000, 1017, 2040, 2041, 4088, 4089])
+def test_line_run_equals_single_steps(n, solver, bc):
+    """A 1-D grid's steps in one launch (up to 4088 cells, 2040 with Roe) against the same steps made
+    one by one: state, every dt and the clock bit for bit, after an odd and an even number of steps;
+    n at the edges of one, two, four and eight blocks and just past the largest."""
+    kind = {"periodic": pg.BC_PERIODIC, "copy": pg.BC_COPY, "value": pg.BC_VALUE}[bc]
+    U = states.smooth_3d((1, 1, n), np.random.default_rng(n))
+    cfg = pg.Config(n=(n, 1, 1), solver=po.SOLVERS[solver], cell_length=(1.0 / n, 1.0, 1.0), time_step_factor=0.4,
+                    bc_lo=(kind, 0, 0), bc_hi=(kind, 0, 0), value_lo=[U[:, 0, 0, 0], None, None],
+                    value_hi=[U[:, 0, 0, -1], None, None])
+    a, b = pg.Context(cfg), pg.Context(cfg)
+    for g in (a, b):
+        g.set_state(U)
+    for count in (5, 8, 2):
+        a.steps(count, 1e300)
+        for _ in range(count):
+            b.step(1e300)
+        np.testing.assert_array_equal(a.get_state(), b.get_state())
+        assert a.time() == b.time()
+        np.testing.assert_array_equal(a.dt_history(20), b.dt_history(20))
+    a.sync()
+
+
+def test_line_run_stops_at_a_failure():
+    """A 1-D run that loses positivity (a timestep factor of 3, far beyond stability): the one-launch
+    steps stop at the step, cell and flag of the steps made one by one and hold that step's result,
+    in both state buffers."""
+    n = 300
+    U = states.smooth_3d((1, 1, n), np.random.default_rng(1))
+    cfg = pg.Config(n=(n, 1, 1), solver=pg.HLLD, cell_length=(1.0 / n, 1.0, 1.0), time_step_factor=3.0)
+    a, b = pg.Context(cfg), pg.Context(cfg)
+    for g in (a, b):
+        g.set_state(U)
+    failed = None
+    for s in range(80):
+        try:
+            b.step(1e300)
+        except pg.PhysicsError as e:
+            failed = (e.flags, e.cell, e.direction)
+            break
+    assert failed is not None and s > 0
+    held = b.get_state()
+    for count in (s + 1, 3, 2):   # the failing step last, then held steps
+        a.steps(count, 1e300)
+        with pytest.raises(pg.PhysicsError) as e:
+            a.sync()
+        assert (e.value.flags, e.value.cell, e.value.direction) == failed
+        np.testing.assert_array_equal(a.get_state(), held)
+    assert a.time()[:2] == b.time()[:2]
+
+
 @pytest.mark.parametrize("bc", ["periodic", "copy"])
 @pytest.mark.parametrize("n", [(33, 9, 2), (70, 17, 37), (31, 40, 3), (64, 8, 19), (100, 20, 5), (36, 36, 7),
                                (17, 45, 6)])
