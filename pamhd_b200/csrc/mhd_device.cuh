@@ -9,9 +9,10 @@ the MHD primitives they use (mhd/common.hpp), written for the GPU:
     magnetic pressure and the fast magnetosonic speed along each axis) are
     computed once per cell and shared by the six faces of the cell.  The
     reference recomputes them in every solver call.
-  - Divisions by the same denominator are done once as a reciprocal, and
-    the compiler contracts a*b+c into FMA.  Results therefore differ from
-    the reference by round-off (the parity tests hold them to 1e-12).
+  - Divisions by the same denominator are done once as a reciprocal,
+    products added are fused multiply-adds, and HLLD and Roe are rearranged
+    (see flux_hlld, flux_roe).  Results therefore differ from the reference
+    by round-off (the parity tests hold them to 1e-12).
   - Branches (supersonic upwinding, HLLD degeneracy thresholds, region
     selection, Roe's positivity check) are the reference's, with its
     epsilon thresholds.
@@ -455,9 +456,9 @@ state keeps the outer B_t and v_t, also (v_n - S_M) B_t in the field.
 That is some 60 operations less per face, and the double-star state needs
 only the velocity step across its Alfven wave: v** = v* + dv,
 B** = B* +- sqrt(mu0 rho*) sign(B_x) dv, dv = 0 where there is no such
-wave.  The step is bound by the latency of these FP64 chains: with this
-form, the third-order reciprocals and the fast speed of derive() a 256^3
-step went from 2.14 to 1.73 ms, a 150 x 99 x 67 step from 180 to 148 us.
+wave.  The step is bound by the latency of these FP64 chains: this form, the
+third-order reciprocals and the fast speed of derive() took a 256^3 step
+from 2.14 to 1.73 ms, a 150 x 99 x 67 step from 180 to 148 us.
 
 The side the flux is taken from comes from pick(left): a caller that holds
 the sides' records in shared memory reads that side again instead of

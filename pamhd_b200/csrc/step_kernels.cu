@@ -171,39 +171,46 @@ __device__ __forceinline__ Split_Barrier split_barrier(unsigned long long* const
 	return Split_Barrier{uint32_t(__cvta_generic_to_shared(word)), 0u};
 }
 
-// block-wide start of a step: every block computes dt; block 0 advances the clock ring.  *s_stop:
-// the grid stopped in an earlier step (dt 0, the clock held)
+/*
+The start of a step, by one thread of the block: the step's dt to *s_dt and
+whether the grid stopped in an earlier step to *s_stop (dt 0, the clock
+held); the first block's thread advances the clock ring.
+*/
+__device__ __forceinline__ void find_dt(const Step_Params& P, double* s_dt, const bool first_block, int* s_stop)
+{
+	const bool stop = stopped_before(P);
+	const double dt = stop ? 0.0 : step_dt(P);
+	*s_dt = dt;
+	*s_stop = stop ? 1 : 0;
+	if (first_block) {
+		Clock c;
+		c.t = __ldcg(&P.clock[P.phase].t);
+		c.steps = __ldcg(&P.clock[P.phase].steps);
+		Clock& next = P.clock[(P.phase + 1) % 3];
+		next.t = c.t + dt;
+		next.dt = dt;
+		next.steps = stop ? c.steps : c.steps + 1;
+		if (P.dt_hist != nullptr and not stop) P.dt_hist[c.steps % P.hist_len] = dt;
+		Speed_Max& z = P.red[(P.phase + 2) % 3];
+		z.smax[0] = z.smax[1] = z.smax[2] = 0ull;
+		z.zero = 0u;
+		if (stop) {
+			// no face is solved: the failing step's maxima stay the latest
+			const Speed_Max& r = P.red[P.phase];
+			Speed_Max& o = P.red[(P.phase + 1) % 3];
+			o.smax[0] = __ldcg(&r.smax[0]);
+			o.smax[1] = __ldcg(&r.smax[1]);
+			o.smax[2] = __ldcg(&r.smax[2]);
+			o.zero = __ldcg(&r.zero);
+		}
+	}
+}
+
+// the same for the whole block, which knows both when it returns
 __device__ __forceinline__ double begin_step(const Step_Params& P, double* s_dt, const bool first_block,
                                              int* s_stop)
 {
-	if (threadIdx.x == 0 and threadIdx.y == 0) {
-		const bool stop = stopped_before(P);
-		const double dt = stop ? 0.0 : step_dt(P);
-		*s_dt = dt;
-		*s_stop = stop ? 1 : 0;
-		if (first_block) {
-			Clock c;
-			c.t = __ldcg(&P.clock[P.phase].t);
-			c.steps = __ldcg(&P.clock[P.phase].steps);
-			Clock& next = P.clock[(P.phase + 1) % 3];
-			next.t = c.t + dt;
-			next.dt = dt;
-			next.steps = stop ? c.steps : c.steps + 1;
-			if (P.dt_hist != nullptr and not stop) P.dt_hist[c.steps % P.hist_len] = dt;
-			Speed_Max& z = P.red[(P.phase + 2) % 3];
-			z.smax[0] = z.smax[1] = z.smax[2] = 0ull;
-			z.zero = 0u;
-			if (stop) {
-				// no face is solved: the failing step's maxima stay the latest
-				const Speed_Max& r = P.red[P.phase];
-				Speed_Max& o = P.red[(P.phase + 1) % 3];
-				o.smax[0] = __ldcg(&r.smax[0]);
-				o.smax[1] = __ldcg(&r.smax[1]);
-				o.smax[2] = __ldcg(&r.smax[2]);
-				o.zero = __ldcg(&r.zero);
-			}
-		}
-	}
+	if (threadIdx.x == 0) find_dt(P, s_dt, first_block, s_stop);
 	__syncthreads();
 	return *s_dt;
 }
@@ -326,13 +333,14 @@ CO: loads at L2 (ld.global.cg) instead of through the read-only cache, for a
 persistent launch whose later steps read what other blocks wrote (the
 non-coherent L1 could hold a line of the same buffer from two steps before).
 */
-template <bool CX, bool CY, bool CZ, bool CO>
+template <bool CX, bool CY, bool CZ, bool CO, class Meanwhile>
 __device__ __forceinline__ double load_record(const Step_Params& P, double* rec, uint8_t* bad, const int cells,
-                                              const int ri, const long long off)
+                                              const int ri, const long long off, const Meanwhile& meanwhile)
 {
 	double U[8];
 	#pragma unroll
 	for (int v = 0; v < 8; v++) U[v] = CO ? __ldcg(P.in + v * P.L.var + off) : __ldg(P.in + v * P.L.var + off);
+	meanwhile();   // while the loads are on their way
 	const Derived d = derive<CX, CY, CZ>(U[0], U[1], U[2], U[3], U[4], U[5], U[6], U[7], P.gas);
 	#pragma unroll
 	for (int v = 0; v < 8; v++) rec[v * cells + ri] = U[v];
@@ -463,6 +471,13 @@ __device__ __forceinline__ double solve_xy(const Step_Params& P, const double* r
 
 // ------------------------------------------------------------------ the step
 
+// a step's dt and stop found within tile_step (shared memory); first: this block advances the clock
+struct Late_Start {
+	double dt;
+	int stop;
+	int first;
+};
+
 // the planes [kb, ke) of block row bz: a z chunk, or with kpart 1 the first (bz 0) or the last
 // (bz 1) plane alone, or with kpart 2 a chunk of the planes between them
 __device__ __forceinline__ void tile_planes(const Step_Params& P, const int bz, int& kb, int& ke)
@@ -516,12 +531,17 @@ pass in (b) two thirds of a plane's work to catch up in: with one barrier
 before and one after (b) warps spent 18 % of their time at the two, and a
 256^3 HLLD step took 1.73 ms; split, 1.56 ms.
 A grid without z faces (ZACT false) has one plane and nothing to overlap:
-one record slot and two block barriers.
+one record slot and two block barriers.  There a block finds the step's dt
+late: thread 0 while its first loads are under way, the block behind its
+first barrier, instead of before the loads (512^2 HLLD 33.1 -> 32.0 us per
+step; the 3-D tiles, which start once per 16 planes, lost 1.6 % that way and
+Roe's 4 % to registers).
 */
-template <int SOLVER, int TY, bool ZACT, bool CO = false>
+template <int SOLVER, int TY, bool ZACT, bool CO = false, bool LATE = false>
 __device__ __forceinline__ void tile_step(const Step_Params& P, double* const smem, Split_Barrier& bar,
-                                          const double dt, const int bx, const int by, const int bz,
-                                          double& s0, double& s1, double& s2, bool& zero)
+                                          double dt, const int bx, const int by, const int bz,
+                                          double& s0, double& s1, double& s2, bool& zero,
+                                          Late_Start* const late = nullptr)
 {
 	constexpr int NF = Flux_Rows<SOLVER>::N;
 	using T = Tile<TY, ZACT, NF>;
@@ -559,7 +579,7 @@ __device__ __forceinline__ void tile_step(const Step_Params& P, double* const sm
 	const int ri = at(ty, tx);
 	const int r_east = ZACT and tx == tw - 1 ? right_of_row(ty) : ri + 1;
 	// the flux terms are dt F / dx: dt / dx once per axis and cell
-	const double cx = dt * P.inv_len[0], cy = dt * P.inv_len[1], cz = dt * P.inv_len[2];
+	double cx = dt * P.inv_len[0], cy = dt * P.inv_len[1], cz = dt * P.inv_len[2];
 
 	// this thread's halo cell of planes with x / y faces, if any: first the rows below and above the
 	// tile, then the columns left and right of it
@@ -590,9 +610,13 @@ __device__ __forceinline__ void tile_step(const Step_Params& P, double* const sm
 		double* const rec = rec_base + slot * T::REC;
 		uint8_t* const bad = bad_base + slot * T::CELLS;
 		double cfz = 0.0;
-		if (stage) cfz = load_record<true, YACT, ZACT, CO>(P, rec, bad, T::CELLS, ri, col + k * P.L.plane);
+		if (stage) {
+			cfz = load_record<true, YACT, ZACT, CO>(P, rec, bad, T::CELLS, ri, col + k * P.L.plane, [&]() {
+				if (LATE and t == 0) find_dt(P, &late->dt, late->first, &late->stop);
+			});
+		}
 		if (k >= kb and k < ke and hri >= 0) {
-			load_record<true, YACT, false, CO>(P, rec, bad, T::CELLS, hri, hoff + k * P.L.plane);
+			load_record<true, YACT, false, CO>(P, rec, bad, T::CELLS, hri, hoff + k * P.L.plane, []() {});
 		}
 		return cfz;
 	};
@@ -644,6 +668,15 @@ __device__ __forceinline__ void tile_step(const Step_Params& P, double* const sm
 
 		if (inner) {
 			__syncthreads();
+			if (LATE) {
+				if (late->stop) {
+					tile_hold<CO>(P, bx, by, bz);
+					return;
+				}
+				dt = late->dt;
+				cx = dt * P.inv_len[0];
+				cy = dt * P.inv_len[1];
+			}
 			// (b) x and y faces, all through one call site
 			#pragma unroll 1
 			for (int pass = 0; pass < (ZACT ? 3 : (YACT ? 4 : 1)); pass++) {
@@ -867,16 +900,22 @@ template <int SOLVER, int TY, bool ZACT>
 __global__ void __launch_bounds__(TX * TY, Tile_Kind::resident_of(SOLVER, TY, ZACT)) step_kernel(const Step_Params P)
 {
 	extern __shared__ __align__(16) double smem[];
-	__shared__ double s_dt;
-	__shared__ int s_stop;
+	constexpr bool LATE = not ZACT and SOLVER != PAMHD_ROE_ATHENA;
+	__shared__ Late_Start start;
 	__shared__ unsigned long long s_bar;
 	Split_Barrier bar = split_barrier(&s_bar);
-	if (threadIdx.x == 0 and threadIdx.y == 0) bar.init(TY);
 	const bool first_block = blockIdx.x == 0 and blockIdx.y == 0 and blockIdx.z == 0;
-	const double dt = begin_step(P, &s_dt, first_block, &s_stop);
-	if (s_stop) {
-		if (blockIdx.z < gridDim.z - P.boundary) tile_hold<false>(P, blockIdx.x, blockIdx.y, blockIdx.z);
-		return;
+	if (threadIdx.x == 0) {
+		bar.init(TY);
+		start.first = first_block ? 1 : 0;
+	}
+	double dt = 0.0;
+	if (not LATE or blockIdx.z >= gridDim.z - P.boundary) {
+		dt = begin_step(P, &start.dt, first_block, &start.stop);
+		if (start.stop) {
+			if (blockIdx.z < gridDim.z - P.boundary) tile_hold<false>(P, blockIdx.x, blockIdx.y, blockIdx.z);
+			return;
+		}
 	}
 	double s0 = 0.0, s1 = 0.0, s2 = 0.0;
 	bool zero = false;
@@ -889,7 +928,8 @@ __global__ void __launch_bounds__(TX * TY, Tile_Kind::resident_of(SOLVER, TY, ZA
 		flush_speeds(P, smax, zero);
 		return;
 	}
-	tile_step<SOLVER, TY, ZACT>(P, smem, bar, dt, blockIdx.x, blockIdx.y, blockIdx.z, s0, s1, s2, zero);
+	tile_step<SOLVER, TY, ZACT, false, LATE>(P, smem, bar, dt, blockIdx.x, blockIdx.y, blockIdx.z, s0, s1, s2, zero, &start);
+	if (LATE and start.stop) return;
 	double smax[3] = {s0, s1, s2};
 	flush_speeds(P, smax, zero);
 }
