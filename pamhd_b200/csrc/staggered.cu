@@ -95,11 +95,14 @@ __device__ __forceinline__ long long wrap_index(const Stag_Params& P, int i, int
 	return (long long)i + (long long)P.n[0] * ((long long)j + (long long)P.n[1] * k);
 }
 
+// (32-bit arithmetic: create keeps N at 2^31 at most)
 __device__ __forceinline__ void cell_coords(const Stag_Params& P, const long long c, int& i, int& j, int& k)
 {
-	i = int(c % P.n[0]);
-	j = int((c / P.n[0]) % P.n[1]);
-	k = int(c / ((long long)P.n[0] * P.n[1]));
+	const unsigned int u = (unsigned int)c, n0 = (unsigned int)P.n[0], n1 = (unsigned int)P.n[1];
+	const unsigned int q = u / n0, r = q / n1;
+	i = int(u - q * n0);
+	j = int(q - r * n1);
+	k = int(r);
 }
 
 __device__ __forceinline__ void record_failure(const Stag_Params& P, const uint32_t flag, const long long cell,

@@ -36,7 +36,7 @@ Layout: state 8 x N, flux slots 6 x 8 x N (each cell's -x, +x, -y, +y, -z,
 +z), the speed of every cell's -d face 3 x N, exponents and periods
 N int32, x fastest, no ghosts.  One host round trip per step for the plan
 (the host needs the substep count to launch the substeps).  Compiled without
-FMA contraction; the update follows the oracle's operation order.
+FMA contraction; the update sums the oracle's terms, x, then y, then z.
 */
 #include <cuda_runtime.h>
 
@@ -97,11 +97,14 @@ __device__ __forceinline__ long long wrap(const Sub_Params& P, int i, int j, int
 	return (long long)i + (long long)P.n[0] * ((long long)j + (long long)P.n[1] * k);
 }
 
+// (32-bit arithmetic: create keeps N at 2^30 at most; 64-bit quotients were most of the plan kernels)
 __device__ __forceinline__ void coords(const Sub_Params& P, const long long c, int& i, int& j, int& k)
 {
-	i = int(c % P.n[0]);
-	j = int((c / P.n[0]) % P.n[1]);
-	k = int(c / ((long long)P.n[0] * P.n[1]));
+	const unsigned int u = (unsigned int)c, n0 = (unsigned int)P.n[0], n1 = (unsigned int)P.n[1];
+	const unsigned int q = u / n0, r = q / n1;
+	i = int(u - q * n0);
+	j = int(q - r * n1);
+	k = int(r);
 }
 
 // calls body(neighbour) for the face and edge neighbours of cell (i, j, k) in the active dimensions
@@ -334,25 +337,12 @@ __global__ void __launch_bounds__(THREADS, 2) update_kernel(const Sub_Params P, 
 		double u[8];
 		#pragma unroll
 		for (int v = 0; v < 8; v++) u[v] = P.U[v * N + c];
-		#pragma unroll
-		for (int d = 0; d < 3; d++) {
-			if (P.active[d]) u[0] += (f(2 * d, 0) - f(2 * d + 1, 0)) / P.len[d];
-		}
+		// x, then y, then z, each length's inverse multiplied in (quotients were most of the arithmetic)
 		#pragma unroll
 		for (int d = 0; d < 3; d++) {
 			if (not P.active[d]) continue;
 			#pragma unroll
-			for (int e = 1; e <= 3; e++) u[e] = u[e] + P.inv_len[d] * (f(2 * d, e) + (-f(2 * d + 1, e)));
-		}
-		#pragma unroll
-		for (int d = 0; d < 3; d++) {
-			if (P.active[d]) u[4] += (f(2 * d, 4) - f(2 * d + 1, 4)) / P.len[d];
-		}
-		#pragma unroll
-		for (int d = 0; d < 3; d++) {
-			if (not P.active[d]) continue;
-			#pragma unroll
-			for (int e = 5; e <= 7; e++) u[e] = u[e] + P.inv_len[d] * (f(2 * d, e) + (-f(2 * d + 1, e)));
+			for (int v = 0; v < 8; v++) u[v] = __fma_rn(f(2 * d, v) - f(2 * d + 1, v), P.inv_len[d], u[v]);
 		}
 		#pragma unroll
 		for (int v = 0; v < 8; v++) P.U[v * N + c] = u[v];
