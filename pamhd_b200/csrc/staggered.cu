@@ -298,6 +298,12 @@ __global__ void __launch_bounds__(STX * STY, SOLVER == PAMHD_ROE_ATHENA ? 1 : 2)
 		} else if (hr >= 0) {
 			stage_cell<true, false, false, BG>(P, rec, bad, hr, hcol + kofs);
 		}
+		// the next plane's own cell on its way to L2 while this plane's faces are solved
+		if (own and k + 1 < ke) {
+			const double* const next = P.U + col + kofs + plane;
+			#pragma unroll
+			for (int v = 0; v < 8; v++) asm volatile("prefetch.global.L2 [%0];" :: "l"(next + v * P.N));
+		}
 		__syncthreads();
 		if (own) {
 			const long long c = col + kofs;
