@@ -96,6 +96,24 @@ struct Derived {
 	uint32_t bad;
 };
 
+#ifdef __CUDACC__
+// the hardware's estimates of 1/x and 1/sqrt(x), which take a subnormal x for zero (a host build of
+// these solvers brings its own)
+__device__ __forceinline__ double rcp_estimate(const double x)
+{
+	double r;
+	asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(x));
+	return r;
+}
+
+__device__ __forceinline__ double rsqrt_estimate(const double x)
+{
+	double r;
+	asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(x));
+	return r;
+}
+#endif
+
 /*
 Reciprocal of a non-zero normal double: one third-order step of the
 Householder family for f(r) = 1/r - x, r <- r (1 + e + e^2) with
@@ -107,8 +125,7 @@ Used where the operand is a normal, non-zero number by construction.
 */
 __device__ __forceinline__ double recip(const double x)
 {
-	double r;
-	asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(x));
+	const double r = rcp_estimate(x);
 	const double e = __fma_rn(-x, r, 1.0);
 	return __fma_rn(r, __fma_rn(e, e, e), r);
 }
@@ -129,9 +146,7 @@ estimate of PTX rsqrt.approx.ftz.f64.
 */
 __device__ __forceinline__ double rsqrt_nr(const double x)
 {
-	double r;
-	asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(x));
-	return rsqrt_step(x, r);
+	return rsqrt_step(x, rsqrt_estimate(x));
 }
 
 /*
@@ -142,9 +157,7 @@ high word), so that 0 gives 0.
 __device__ __forceinline__ double sqrt_nr(const double x)
 {
 	const double c = __hiloint2double(max(__double2hiint(x), 0x00100000), __double2loint(x));
-	double r;
-	asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(c));
-	return __dmul_rn(x, rsqrt_step(x, r));
+	return __dmul_rn(x, rsqrt_step(x, rsqrt_estimate(c)));
 }
 
 /*
@@ -566,7 +579,8 @@ __device__ __forceinline__ Rd mad(const Rd a, const Rd b, const Rd c) { return _
 
 /*
 alpha_f and alpha_s of Roe's eigensystem (B17-B29 of Stone et al.) for an
-exactly aligned average field (no transverse component).  The reference's
+aligned average field (the square of its transverse component below the
+smallest normal number).  The reference's
 numerators a^2 - c_s^2 and c_f^2 - a^2 are then round-off, 0 or some 1e-16,
 whose root weighs in at 1e-8 where the transverse velocity or field jumps:
 its operations are repeated here one for one, each rounded on its own
@@ -712,11 +726,19 @@ __device__ __forceinline__ double flux_roe(const Side& L, const Side& R, const G
 		const Rd large = big * iroot, small = a2ct2 * recip(big) * iroot;
 		const bool slow_field = tdif < 0.0;
 		const Rd one = 1.0, none = 0.0;
-		const bool has_bt = btsq > 0.0;
 		Rd af = sqrt_nr(slow_field ? large : small), as = sqrt_nr(slow_field ? small : large);
-		if (not has_bt) aligned_alphas(L, R, g, af.v, as.v);
-		const Rd ibt = rsqrt_nr(has_bt ? btsq : one), bt = btsq * ibt;
-		const Rd bet2 = has_bt ? b2 * ibt : one, bet3 = has_bt ? b3 * ibt : none;
+		const Rd ibt = rsqrt_nr(btsq);
+		Rd bt = btsq * ibt, bet2 = b2 * ibt, bet3 = b3 * ibt;
+		if (not is_positive_normal(btsq)) {
+			// no field, or one whose square is subnormal, which the estimate of the root takes for 0:
+			// its direction from the field times 2^600
+			aligned_alphas(L, R, g, af.v, as.v);
+			const Rd s2 = b2 * 0x1p600, s3 = b3 * 0x1p600;
+			const double s = __dsqrt_rn(mad(s3, s3, s2 * s2));
+			bt = s * 0x1p-600;
+			bet2 = btsq > 0.0 ? __ddiv_rn(s2, s) : 1.0;
+			bet3 = btsq > 0.0 ? __ddiv_rn(s3, s) : 0.0;
+		}
 		const Rd iys = rsqrt_nr(ystar), sys = ystar * iys;
 		const Rd sg = bxi > 0.0 ? one : -one;
 		const Rd qf = cf * af * sg, qs = cs * as * sg;

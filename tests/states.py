@@ -44,6 +44,17 @@ def nearby_face_states(n, rng, gamma=GAMMA_53, jump=0.05):
     return a, b
 
 
+def small_transverse_field_states(n, rng, low, high):
+    """Pairs of random states whose transverse field is 10^low to 10^high in size (uniform exponent)."""
+    a, b = random_face_states(n, rng, spread=0.3), random_face_states(n, rng, spread=0.3)
+    size = 10.0 ** rng.uniform(low, high, n)
+    for s in (a, b):
+        s[:, 4] -= 0.5 * (s[:, 6:8] ** 2).sum(1)
+        s[:, 6:8] = rng.normal(size=(n, 2)) * size[:, None]
+        s[:, 4] += 0.5 * (s[:, 6:8] ** 2).sum(1)
+    return a, b
+
+
 def edge_case_face_states(gamma=GAMMA_53):
     """Hand-made face problems covering the branches of the four solvers."""
     def st(rho, v, p, B):

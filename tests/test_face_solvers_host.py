@@ -1,0 +1,60 @@
+"""The face solvers of the GPU step (pamhd_b200/csrc/mhd_device.cuh), compiled for the host
+(tests/host/solvers_host.cpp), against the oracle's on states where rearranged arithmetic can go
+wrong (CPU only)."""
+import ctypes
+import os
+import subprocess
+
+import numpy as np
+import pytest
+
+from oracle import pyoracle as po
+import states
+
+HERE = os.path.dirname(os.path.abspath(__file__))
+SRC = os.path.join(HERE, "host", "solvers_host.cpp")
+LIB = os.path.join(HERE, "host", "_build", "libsolvers_host.so")
+D = ctypes.POINTER(ctypes.c_double)
+
+
+@pytest.fixture(scope="module")
+def host():
+    """face_flux(solver, neg, pos, mu0) -> flux, speed, flags of the host build."""
+    os.makedirs(os.path.dirname(LIB), exist_ok=True)
+    deps = [SRC, os.path.join(os.path.dirname(HERE), "pamhd_b200", "csrc", "mhd_device.cuh")]
+    if not os.path.exists(LIB) or any(os.path.getmtime(d) > os.path.getmtime(LIB) for d in deps):
+        subprocess.run(["g++", "-std=c++17", "-O2", "-ffp-contract=off", "-fPIC", "-shared", "-o", LIB, SRC],
+                       check=True)
+    L = ctypes.CDLL(LIB)
+    L.host_face_flux.argtypes = [ctypes.c_int32, ctypes.c_int64, D, D, ctypes.c_double, ctypes.c_double, D, D,
+                                 ctypes.POINTER(ctypes.c_uint32)]
+    L.host_face_flux.restype = None
+
+    def face_flux(solver, neg, pos, mu0=1.0):
+        neg, pos = np.ascontiguousarray(neg), np.ascontiguousarray(pos)
+        flux, speed, flags = np.zeros((len(neg), 8)), np.zeros(len(neg)), np.zeros(len(neg), np.uint32)
+        c = lambda a: a.ctypes.data_as(D)
+        L.host_face_flux(solver, len(neg), c(neg), c(pos), 5 / 3, mu0, c(flux), c(speed),
+                         flags.ctypes.data_as(ctypes.POINTER(ctypes.c_uint32)))
+        return flux, speed, flags
+
+    return face_flux
+
+
+@pytest.mark.parametrize("low,high", [(-165, -153), (-153, -3)])
+def test_roe_small_transverse_field(host, port, low, high):
+    """Roe faces whose transverse field is 1e-165 to 1e-3: its square is zero, subnormal (below some
+    1.5e-154) or normal.  The flux is finite wherever the oracle's is.  Except between 1e-163 and
+    1e-157, where that square keeps too few bits for the oracle's field direction to have length 1, the
+    flags are the oracle's and the flux is at most 1e-6 of the row away (the alphas of an almost aligned
+    field are a root of round-off, some 1e-8)."""
+    a, b = states.small_transverse_field_states(20000, np.random.default_rng(5), low, high)
+    fo, so, go = port.face_flux(po.SOLVERS["roe_athena"], a, b, None, 5 / 3, 1.0)
+    fh, sh, gh = host(po.SOLVERS["roe_athena"], a, b)
+    assert (go == 0).sum() > 10000 and np.isfinite(fo).all()
+    assert np.isfinite(fh).all()
+    size = np.maximum(np.abs(a[:, 6:8]).max(1), np.abs(b[:, 6:8]).max(1))
+    clear = (size < 1e-163) | (size > 1e-157)
+    assert np.array_equal(gh[clear], go[clear])
+    ok = clear & (go == 0)
+    assert (np.abs(fh[ok] - fo[ok]) / np.abs(fo[ok]).max(axis=1, keepdims=True)).max() <= 1e-6

@@ -148,6 +148,36 @@ def test_roe_aligned_faces_match_oracle(port, normal):
     assert (np.abs(fg[ok] - fo[ok]) / np.abs(fo[ok]).max(axis=1, keepdims=True)).max() <= STEP_TOL
 
 
+def test_roe_small_transverse_field():
+    """Roe faces whose transverse field's square is zero, subnormal or a small normal number: finite."""
+    a, b = states.small_transverse_field_states(4000, np.random.default_rng(5), -165, -150)
+    flux, _, _ = pg.face_flux(po.SOLVERS["roe_athena"], a, b, None, 5 / 3, 1.0)
+    assert np.isfinite(flux).all()
+
+
+def test_roe_field_tail_matches_oracle(port):
+    """A narrow transverse field on 1000 periodic cells, 320 Roe steps: its tail falls by a factor per
+    cell and reaches 1e-154 (whose square is subnormal) at step 239.  Bar: STEP_TOL per step."""
+    n, steps = 1000, 320
+    x = (np.arange(n) + 0.5) / n
+    U = np.zeros((8, 1, 1, n))
+    U[0] = 1.0
+    U[5] = 0.75
+    U[6] = np.where(np.abs(x - 0.5) < 0.03, 0.2, 0.0)
+    U[4] = 1.0 / (5 / 3 - 1) + 0.5 * (U[5:] ** 2).sum(0)
+    gpu, ora = pair(port, (n, 1, 1), po.SOLVERS["roe_athena"], (1 / n, 1.0, 1.0), 5 / 3, 1.0, 0.4)
+    gpu.set_state(U)
+    ora.set_state(U)
+    gpu.steps(steps, 1e300)
+    gpu.sync()
+    for s in range(steps):
+        _, flag, _, _ = ora.step(0.0 if s == 0 else 1e300)
+        assert flag == 0
+    small = np.abs(ora.get_state()[6])
+    assert ((small > 1e-162) & (small < 1.5e-154)).any()
+    assert field_err(gpu.get_state(), ora.get_state()) <= steps * STEP_TOL
+
+
 @pytest.mark.parametrize("solver", list(po.SOLVERS))
 def test_face_flux_matches_oracle(port, solver):
     rng = np.random.default_rng(11)
