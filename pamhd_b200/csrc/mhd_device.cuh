@@ -578,16 +578,43 @@ __device__ __forceinline__ Rd operator-(const Rd a) { return -a.v; }
 __device__ __forceinline__ Rd mad(const Rd a, const Rd b, const Rd c) { return __fma_rn(a.v, b.v, c.v); }
 
 /*
-alpha_f and alpha_s of Roe's eigensystem (B17-B29 of Stone et al.) for an
-aligned average field (the square of its transverse component below the
-smallest normal number).  The reference's
-numerators a^2 - c_s^2 and c_f^2 - a^2 are then round-off, 0 or some 1e-16,
-whose root weighs in at 1e-8 where the transverse velocity or field jumps:
-its operations are repeated here one for one, each rounded on its own
-(mhd/roe_athena.hpp:56-559), so that such faces agree with it too.
+Correctly rounded reciprocals, quotients and roots of normal numbers by
+Markstein's final step (IBM J. Res. Dev. 34, 1990): a result y within an ulp
+is corrected by its remainder, which a fused multiply-add gives exactly,
+times the (rounded) reciprocal.  Straight code where the IEEE functions are
+calls; only a divisor whose mantissa is all ones can miss the last bit.
 */
-__device__ __forceinline__ void aligned_alphas(const Side& L, const Side& R, const Gas& g, double& alpha_f,
-                                               double& alpha_s)
+__device__ __forceinline__ double recip_rn(const double x)
+{
+	const double r = recip(x);
+	return __fma_rn(__fma_rn(-x, r, 1.0), r, r);
+}
+
+// a / x, with r = recip_rn(x)
+__device__ __forceinline__ double quotient_rn(const double a, const double x, const double r)
+{
+	const double q = __dmul_rn(a, r);
+	return __fma_rn(__fma_rn(-q, x, a), r, q);
+}
+
+// 0 gives 0
+__device__ __forceinline__ double sqrt_rn(const double x)
+{
+	const double r = rsqrt_nr(fmax(x, DBL_MIN_NORMAL)), s = __dmul_rn(x, r);
+	return __fma_rn(__fma_rn(-s, s, x), __dmul_rn(0.5, r), s);
+}
+
+/*
+alpha_f and alpha_s of Roe's eigensystem (B17-B29 of Stone et al.) for an
+almost aligned average field (a small transverse component).  One of the
+reference's numerators a^2 - c_s^2 and c_f^2 - a^2 is then all or partly
+round-off, some 1e-16, whose root weighs in at up to 1e-8 where the
+transverse velocity or field jumps: its operations are repeated here one for
+one, each rounded on its own (mhd/roe_athena.hpp:56-559), so that such faces
+agree with it too.
+*/
+__device__ __forceinline__ void near_aligned_alphas(const Side& L, const Side& R, const Gas& g, double& alpha_f,
+                                                    double& alpha_s)
 {
 	const auto mul = [](const double a, const double b) { return __dmul_rn(a, b); };
 	const auto add = [](const double a, const double b) { return __dadd_rn(a, b); };
@@ -595,25 +622,36 @@ __device__ __forceinline__ void aligned_alphas(const Side& L, const Side& R, con
 	const auto sq3 = [&](const double a, const double b, const double c) {
 		return add(add(mul(a, a), mul(b, b)), mul(c, c));
 	};
-	const double gm1 = g.gamma - 1.0, gm2 = g.gamma - 2.0, ism = g.inv_sqrt_mu0;
-	const double bx = mul(mul(0.5, add(L.b0, R.b0)), ism);
-	const auto enthalpy = [&](const Side& s, const double by, const double bz) {
-		const double p = mul(gm1, sub(sub(s.E, mul(mul(0.5, s.rinv), sq3(s.m0, s.m1, s.m2))),
-		                              mul(0.5, sq3(s.b0, s.b1, s.b2))));
-		return add(add(s.E, p), mul(0.5, sq3(bx, by, bz)));
+	const double gm1 = g.gamma - 1.0, gm2 = g.gamma - 2.0;
+	const auto field = [&](const double b) { return quotient_rn(b, g.sqrt_mu0, g.inv_sqrt_mu0); };
+	const double bx = mul(0.5, field(add(L.b0, R.b0))), bx2 = mul(bx, bx);
+	const double byl = field(L.b1), bzl = field(L.b2), byr = field(R.b1), bzr = field(R.b2);
+	const double il = recip_rn(L.rho), ir = recip_rn(R.rho);
+	const double sl = sqrt_rn(L.rho), sr = sqrt_rn(R.rho), sum = add(sl, sr);
+	const double isd = recip_rn(sum), rho = mul(sl, sr), di = recip_rn(rho);
+	const auto enthalpy = [&](const Side& s, const double i, const double by, const double bz, const double root) {
+		const double p = mul(sub(sub(s.E, mul(mul(0.5, i), sq3(s.m0, s.m1, s.m2))),
+		                         mul(0.5, sq3(s.b0, s.b1, s.b2))), gm1);
+		const double H = add(add(s.E, p), mul(0.5, add(add(bx2, mul(by, by)), mul(bz, bz))));
+		return quotient_rn(H, root, recip_rn(root));
 	};
-	const double byl = mul(L.b1, ism), bzl = mul(L.b2, ism), byr = mul(R.b1, ism), bzr = mul(R.b2, ism);
-	const double sl = __dsqrt_rn(L.rho), sr = __dsqrt_rn(R.rho);
-	const double isd = __drcp_rn(add(sl, sr)), rho = mul(sl, sr);
-	const double v0 = mul(add(mul(sl, L.v0), mul(sr, R.v0)), isd), v1 = mul(add(mul(sl, L.v1), mul(sr, R.v1)), isd);
-	const double v2 = mul(add(mul(sl, L.v2), mul(sr, R.v2)), isd);
-	const double h = mul(add(__ddiv_rn(enthalpy(L, byl, bzl), sl), __ddiv_rn(enthalpy(R, byr, bzr), sr)), isd);
-	const double dy = sub(byl, byr), dz = sub(bzl, bzr);
-	const double x = mul(mul(0.5, add(mul(dy, dy), mul(dz, dz))), mul(isd, isd));
-	const double va2 = mul(mul(bx, bx), __drcp_rn(rho));
-	const double a2 = fmax(sub(mul(gm1, sub(sub(h, va2), mul(0.5, sq3(v0, v1, v2)))), mul(gm2, x)), DBL_EPS);
-	const double cf2 = mul(0.5, add(add(va2, a2), fabs(sub(va2, a2))));
-	const double cs2 = __ddiv_rn(mul(a2, va2), cf2);
+	const double h = mul(add(enthalpy(L, il, byl, bzl, sl), enthalpy(R, ir, byr, bzr, sr)), isd);
+	const auto mean = [&](const double l, const double r) {
+		return mul(add(mul(sl, mul(l, il)), mul(sr, mul(r, ir))), isd);
+	};
+	const double vsq = sq3(mean(L.m0, R.m0), mean(L.m1, R.m1), mean(L.m2, R.m2));
+	const double by = mul(add(mul(sr, byl), mul(sl, byr)), isd), bz = mul(add(mul(sr, bzl), mul(sl, bzr)), isd);
+	const double dy = sub(byl, byr), dz = sub(bzl, bzr), sum2 = mul(sum, sum);
+	const double x = quotient_rn(mul(0.5, add(mul(dy, dy), mul(dz, dz))), sum2, recip_rn(sum2));
+	const double y = quotient_rn(mul(0.5, add(L.rho, R.rho)), rho, di);
+	const double btsq = add(mul(by, by), mul(bz, bz));
+	const double ct2 = mul(mul(sub(gm1, mul(gm2, y)), btsq), di), va2 = mul(bx2, di);
+	const double hp = sub(h, add(va2, mul(btsq, di)));
+	const double a2 = fmax(sub(mul(gm1, sub(hp, mul(0.5, vsq))), mul(gm2, x)), DBL_EPS);
+	const double vat2 = add(va2, ct2), tdif = sub(vat2, a2);
+	const double root = sqrt_rn(add(mul(tdif, tdif), mul(mul(4.0, a2), ct2)));
+	const double cf2 = mul(0.5, add(add(vat2, a2), root));
+	const double cs2 = quotient_rn(mul(a2, va2), cf2, recip_rn(cf2));
 	const double q = sub(cf2, cs2), f = sub(a2, cs2), s = sub(cf2, a2);
 	alpha_f = 1.0;
 	alpha_s = 0.0;
@@ -622,9 +660,9 @@ __device__ __forceinline__ void aligned_alphas(const Side& L, const Side& R, con
 		alpha_f = 0.0;
 		alpha_s = 1.0;
 	} else if (s > 0.0) {
-		const double iq = __drcp_rn(q);
-		alpha_f = __dsqrt_rn(mul(f, iq));
-		alpha_s = __dsqrt_rn(mul(s, iq));
+		const double iq = recip_rn(q);
+		alpha_f = sqrt_rn(quotient_rn(f, q, iq));
+		alpha_s = sqrt_rn(quotient_rn(s, q, iq));
 	}
 }
 
@@ -649,7 +687,8 @@ alpha_f^2 = (a^2 - c_s^2) / (c_f^2 - c_s^2) and alpha_s^2 = (c_f^2 - a^2) /
 roots: with q = c_f^2 - c_s^2 its discriminant's root and
 t = v_A^2 - a^2 (v_A with the starred transverse field), the larger of the
 two numerators is (q + |t|) / 2 and the smaller a^2 c_t^2 over that, so
-that nothing cancels.
+that nothing cancels; where the reference's own cancellation shows, in an
+almost aligned field, they are the reference's (near_aligned_alphas).
 */
 __device__ __forceinline__ double flux_roe(const Side& L, const Side& R, const Gas& g, double F[8],
                                            uint32_t& flag)
@@ -729,10 +768,12 @@ __device__ __forceinline__ double flux_roe(const Side& L, const Side& R, const G
 		Rd af = sqrt_nr(slow_field ? large : small), as = sqrt_nr(slow_field ? small : large);
 		const Rd ibt = rsqrt_nr(btsq);
 		Rd bt = btsq * ibt, bet2 = b2 * ibt, bet3 = b3 * ibt;
+		// below 1e-5 the reference's round-off in the smaller alpha weighs more than some 2e-13 of the flux
+		// (1e5 random faces; 6e-13 at 1e-6).  NaN, where the root is 0, too
+		if (not (small > 1e-5)) near_aligned_alphas(L, R, g, af.v, as.v);
 		if (not is_positive_normal(btsq)) {
 			// no field, or one whose square is subnormal, which the estimate of the root takes for 0:
 			// its direction from the field times 2^600
-			aligned_alphas(L, R, g, af.v, as.v);
 			const Rd s2 = b2 * 0x1p600, s3 = b3 * 0x1p600;
 			const double s = __dsqrt_rn(mad(s3, s3, s2 * s2));
 			bt = s * 0x1p-600;

@@ -46,8 +46,8 @@ def test_roe_small_transverse_field(host, port, low, high):
     """Roe faces whose transverse field is 1e-165 to 1e-3: its square is zero, subnormal (below some
     1.5e-154) or normal.  The flux is finite wherever the oracle's is.  Except between 1e-163 and
     1e-157, where that square keeps too few bits for the oracle's field direction to have length 1, the
-    flags are the oracle's and the flux is at most 1e-6 of the row away (the alphas of an almost aligned
-    field are a root of round-off, some 1e-8)."""
+    flags are the oracle's and the flux is at most 1e-6 of the row away (alphas that are a root of
+    round-off, some 1e-8)."""
     a, b = states.small_transverse_field_states(20000, np.random.default_rng(5), low, high)
     fo, so, go = port.face_flux(po.SOLVERS["roe_athena"], a, b, None, 5 / 3, 1.0)
     fh, sh, gh = host(po.SOLVERS["roe_athena"], a, b)
@@ -58,3 +58,16 @@ def test_roe_small_transverse_field(host, port, low, high):
     assert np.array_equal(gh[clear], go[clear])
     ok = clear & (go == 0)
     assert (np.abs(fh[ok] - fo[ok]) / np.abs(fo[ok]).max(axis=1, keepdims=True)).max() <= 1e-6
+
+
+@pytest.mark.parametrize("exponent", [-400, -14, -12, -10, -8, -6, -5, -4, -3, -2, -1])
+def test_roe_almost_aligned_field_matches_oracle(host, port, exponent):
+    """Roe faces with a transverse field of size 10^exponent (0 at -400): the smaller of the reference's
+    alphas is a root of round-off below some 1e-8, partly so up to 1e-3.  Bar: 1e-12 of the flux row."""
+    a, b = states.small_transverse_field_states(20000, np.random.default_rng(4), exponent, exponent)
+    fo, so, go = port.face_flux(po.SOLVERS["roe_athena"], a, b, None, 5 / 3, 1.0)
+    fh, sh, gh = host(po.SOLVERS["roe_athena"], a, b)
+    assert np.array_equal(gh, go)
+    ok = go == 0
+    assert ok.sum() > 10000
+    assert (np.abs(fh[ok] - fo[ok]) / np.abs(fo[ok]).max(axis=1, keepdims=True)).max() <= 1e-12

@@ -155,6 +155,19 @@ def test_roe_small_transverse_field():
     assert np.isfinite(flux).all()
 
 
+@pytest.mark.parametrize("exponent", [-400, -14, -10, -6, -4, -2])
+def test_roe_almost_aligned_faces_match_oracle(port, exponent):
+    """Roe faces with a transverse field of size 10^exponent (0 at -400), where the smaller of the
+    reference's alphas is all or partly a root of round-off.  Bar: the face bar."""
+    a, b = states.small_transverse_field_states(4000, np.random.default_rng(4), exponent, exponent)
+    fo, so, go = port.face_flux(po.SOLVERS["roe_athena"], a, b, None, 5 / 3, 1.0)
+    fg, sg, gg = pg.face_flux(po.SOLVERS["roe_athena"], a, b, None, 5 / 3, 1.0)
+    assert np.array_equal(gg, go)
+    ok = go == 0
+    assert ok.sum() > 1000
+    assert (np.abs(fg[ok] - fo[ok]) / np.abs(fo[ok]).max(axis=1, keepdims=True)).max() <= STEP_TOL
+
+
 def test_roe_field_tail_matches_oracle(port):
     """A narrow transverse field on 1000 periodic cells, 320 Roe steps: its tail falls by a factor per
     cell and reaches 1e-154 (whose square is subnormal) at step 239.  Bar: STEP_TOL per step."""
