@@ -371,8 +371,7 @@ __device__ __forceinline__ double flux_rusanov(const Side& L, const Side& R, con
 HLL with Davis wave-speed estimates, mhd/hll_athena.hpp:65-275:
 S_L = min(u_L, u_R) - max c_f, S_R = max(u_L, u_R) + max c_f,
 bm = min(S_L, 0), bp = max(S_R, 0); a degenerate fan (bp - bm not a
-positive normal number) gives zero flux and zero speed.  The flux as
-bp / (bp - bm) (F_L - bm U_L) - bm / (bp - bm) (F_R - bp U_R).
+positive normal number) gives zero flux and zero speed.
 */
 template <bool BG>
 __device__ __forceinline__ double flux_hll(const Side& L, const Side& R, const Gas& g, double F[8],
@@ -400,11 +399,14 @@ __device__ __forceinline__ double flux_hll(const Side& L, const Side& R, const G
 	}
 	const double UL[8] = {L.rho, L.m0, L.m1, L.m2, L.E, L.b0, L.b1, L.b2};
 	const double UR[8] = {R.rho, R.m0, R.m1, R.m2, R.E, R.b0, R.b1, R.b2};
-	const double iw = recip(width);
-	const double wl = A::mul(bp, iw), wr = A::mul(-bm, iw);
+	// as a mean and a difference, in which both sides round alike: equal states at rest give exactly
+	// their pressure, mirrored faces mirrored fluxes (weights on the sides, two operations less per
+	// row, leave a mass flux of up to 1e-9 of the row between equal states at rest)
+	const double w = A::mul(A::mul(0.5, A::add(bp, bm)), recip(width));
 	#pragma unroll
 	for (int v = 0; v < 8; v++) {
-		F[v] = v == 5 ? 0.0 : A::fma(wl, A::fma(-bm, UL[v], FL[v]), A::mul(wr, A::fma(-bp, UR[v], FR[v])));
+		const double a = A::fma(-bm, UL[v], FL[v]), b = A::fma(-bp, UR[v], FR[v]);
+		F[v] = v == 5 ? 0.0 : A::fma(A::sub(a, b), w, A::mul(0.5, A::add(a, b)));
 	}
 	return larger(bp, -bm);
 }

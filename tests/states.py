@@ -44,6 +44,20 @@ def nearby_face_states(n, rng, gamma=GAMMA_53, jump=0.05):
     return a, b
 
 
+def states_at_rest(n, rng, mu0=4e-7 * np.pi, gamma=GAMMA_53):
+    """Random states of zero velocity in SI units: some 1e-20 kg/m^3, 1e-9 Pa, 1e-8 T."""
+    s = np.zeros((n, 8))
+    s[:, 0] = 1e-20 * rng.uniform(0.1, 3.0, n)
+    s[:, 5:8] = 1e-8 * rng.normal(size=(n, 3))
+    s[:, 4] = 1e-9 * rng.uniform(0.05, 2.0, n) / (gamma - 1) + 0.5 / mu0 * (s[:, 5:8] ** 2).sum(1)
+    return s
+
+
+# the signs a face's state and its flux take when the face is mirrored along its normal
+MIRROR_STATE = np.array([1, -1, 1, 1, 1, -1, 1, 1.0])
+MIRROR_FLUX = np.array([-1, 1, -1, -1, -1, 1, -1, -1.0])
+
+
 def small_transverse_field_states(n, rng, low, high):
     """Pairs of random states whose transverse field is 10^low to 10^high in size (uniform exponent)."""
     a, b = random_face_states(n, rng, spread=0.3), random_face_states(n, rng, spread=0.3)

@@ -71,3 +71,23 @@ def test_roe_almost_aligned_field_matches_oracle(host, port, exponent):
     ok = go == 0
     assert ok.sum() > 10000
     assert (np.abs(fh[ok] - fo[ok]) / np.abs(fo[ok]).max(axis=1, keepdims=True)).max() <= 1e-12
+
+
+def test_hll_equal_states_at_rest(host):
+    """HLL between equal states at rest, SI units: no mass, energy or field flux at all."""
+    mu0 = 4e-7 * np.pi
+    s = states.states_at_rest(2000, np.random.default_rng(6), mu0)
+    flux, speed, flags = host(po.SOLVERS["hll_athena"], s, s, mu0)
+    assert not flags.any() and (speed > 0).all()
+    assert np.array_equal(flux[:, [0, 4, 5, 6, 7]], np.zeros((len(s), 5)))
+
+
+@pytest.mark.parametrize("solver", ["rusanov", "hll_athena"])
+def test_mirrored_faces(host, solver):
+    """A face mirrored along its normal has the mirrored flux, bit for bit."""
+    rng = np.random.default_rng(7)
+    a, b = states.random_face_states(5000, rng), states.random_face_states(5000, rng)
+    f, s, g = host(po.SOLVERS[solver], a, b)
+    fm, sm, gm = host(po.SOLVERS[solver], b * states.MIRROR_STATE, a * states.MIRROR_STATE)
+    assert np.array_equal(g, gm) and np.array_equal(s, sm)
+    assert np.array_equal(fm, np.where(g[:, None] == 0, f * states.MIRROR_FLUX, 0.0))

@@ -148,6 +148,23 @@ def test_roe_aligned_faces_match_oracle(port, normal):
     assert (np.abs(fg[ok] - fo[ok]) / np.abs(fo[ok]).max(axis=1, keepdims=True)).max() <= STEP_TOL
 
 
+def test_hll_uniform_states_at_rest():
+    """HLL in SI units: no mass, energy or field flux between equal states at rest, and a uniform grid
+    at rest stays as it is, bit for bit."""
+    mu0 = 4e-7 * np.pi
+    s = states.states_at_rest(2000, np.random.default_rng(6), mu0)
+    flux, speed, flags = pg.face_flux(pg.HLL, s, s, None, 5 / 3, mu0)
+    assert not flags.any() and (speed > 0).all()
+    assert np.array_equal(flux[:, [0, 4, 5, 6, 7]], np.zeros((len(s), 5)))
+    U = np.tile(s[0].reshape(8, 1, 1, 1), (1, 9, 12, 40))
+    grid = pg.Context(pg.Config(n=(40, 12, 9), solver=pg.HLL, cell_length=(1e7,) * 3, vacuum_permeability=mu0,
+                                time_step_factor=0.4))
+    grid.set_state(U)
+    grid.steps(8, 1e300)
+    grid.sync()
+    np.testing.assert_array_equal(grid.get_state(), U)
+
+
 def test_roe_small_transverse_field():
     """Roe faces whose transverse field's square is zero, subnormal or a small normal number: finite."""
     a, b = states.small_transverse_field_states(4000, np.random.default_rng(5), -165, -150)
