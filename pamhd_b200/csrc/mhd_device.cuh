@@ -500,7 +500,7 @@ __device__ __forceinline__ double flux_hlld(const Side& L, const Side& R, const 
 	const double sdL = A::sub(s_neg, L.v0), sdR = A::sub(s_pos, R.v0);       // < 0 and > 0 here
 	const double rsdL = A::mul(L.rho, sdL), rsdR = A::mul(R.rho, sdR);
 	// eqn 38; the denominator is sdR rho_R - sdL rho_L > 0
-	const double s_mid = A::mul(A::add(A::sub(A::fma(sdR, R.m0, -A::mul(sdL, L.m0)), R.pt), L.pt),
+	const double s_mid = A::mul(A::add(A::sub(A::mul(sdR, R.m0), A::mul(sdL, L.m0)), A::sub(L.pt, R.pt)),
 	                            recip(A::sub(rsdR, rsdL)));
 	const double smL = A::sub(s_neg, s_mid), smR = A::sub(s_pos, s_mid);     // < 0 and > 0 for physical states
 	const double ismL = recip(smL), ismR = recip(smR);
@@ -511,8 +511,7 @@ __device__ __forceinline__ double flux_hlld(const Side& L, const Side& R, const 
 	// eqn 51
 	const double abx = A::mul(fabs(bx), g.inv_sqrt_mu0);
 	const double ssL = A::fma(-abx, irL, s_mid), ssR = A::fma(abx, irR, s_mid);
-	const double ptst = A::fma(rsdL, A::sub(s_mid, L.v0), L.pt);
-	const double thr = A::mul(DBL_EPS, ptst);
+	const double thr = A::mul(DBL_EPS, A::fma(rsdL, A::sub(s_mid, L.v0), L.pt));
 	// transverse star velocity and field of both sides, eqns 44-47
 	const Star_T tl = star_transverse(L, rsdL, sdL, smL, s_mid, bxm, bx2_mu, thr);
 	const Star_T tr = star_transverse(R, rsdR, sdR, smR, s_mid, bxm, bx2_mu, thr);
@@ -527,6 +526,9 @@ __device__ __forceinline__ double flux_hlld(const Side& L, const Side& R, const 
 	const Side S = pick(useL);
 	const Star_T ts = useL ? tl : tr;
 	const double ism = useL ? ismL : ismR, rs = useL ? rsL : rsR;
+	// the star total pressure, equal on both sides but for round-off, from the side the flux is taken
+	// from, so that a mirrored face has the mirrored flux
+	const double ptst = A::fma(useL ? rsdL : rsdR, A::sub(s_mid, S.v0), S.pt);
 
 	// the step across that side's Alfven wave, eqns 59-62 less the star state
 	const double inv_sum = recip(A::add(sqL, sqR));

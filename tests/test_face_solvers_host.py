@@ -82,7 +82,7 @@ def test_hll_equal_states_at_rest(host):
     assert np.array_equal(flux[:, [0, 4, 5, 6, 7]], np.zeros((len(s), 5)))
 
 
-@pytest.mark.parametrize("solver", ["rusanov", "hll_athena"])
+@pytest.mark.parametrize("solver", ["rusanov", "hll_athena", "hlld_athena"])
 def test_mirrored_faces(host, solver):
     """A face mirrored along its normal has the mirrored flux, bit for bit."""
     rng = np.random.default_rng(7)
