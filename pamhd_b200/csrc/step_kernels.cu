@@ -341,7 +341,7 @@ __device__ __forceinline__ double load_record(const Step_Params& P, double* rec,
 	#pragma unroll
 	for (int v = 0; v < 8; v++) U[v] = CO ? __ldcg(P.in + v * P.L.var + off) : __ldg(P.in + v * P.L.var + off);
 	meanwhile();   // while the loads are on their way
-	const Derived d = derive<CX, CY, CZ>(U[0], U[1], U[2], U[3], U[4], U[5], U[6], U[7], P.gas);
+	const Derived d = derive<CX, CY, CZ, false>(U[0], U[1], U[2], U[3], U[4], U[5], U[6], U[7], P.gas);
 	#pragma unroll
 	for (int v = 0; v < 8; v++) rec[v * cells + ri] = U[v];
 	rec[R_RINV * cells + ri] = d.rinv;
@@ -1247,13 +1247,13 @@ __global__ void __launch_bounds__(Line<SOLVER>::THREADS) line_run_kernel(const S
 		double G[8];
 		if (rank == 0 and not P.periodic[0] and P.bc_lo[0] == PAMHD_BC_VALUE) {
 			load(-1, G);
-			const Derived d = derive<true, false, false>(G[0], G[1], G[2], G[3], G[4], G[5], G[6], G[7], P.gas);
+			const Derived d = derive<true, false, false, false>(G[0], G[1], G[2], G[3], G[4], G[5], G[6], G[7], P.gas);
 			put(rank, 0, 0, G, d);
 			put(rank, 1, 0, G, d);
 		}
 		if (rank == blocks - 1 and not P.periodic[0] and P.bc_hi[0] == PAMHD_BC_VALUE) {
 			load(n, G);
-			const Derived d = derive<true, false, false>(G[0], G[1], G[2], G[3], G[4], G[5], G[6], G[7], P.gas);
+			const Derived d = derive<true, false, false, false>(G[0], G[1], G[2], G[3], G[4], G[5], G[6], G[7], P.gas);
 			put(rank, 0, mine + 1, G, d);
 			put(rank, 1, mine + 1, G, d);
 		}
@@ -1270,7 +1270,7 @@ __global__ void __launch_bounds__(Line<SOLVER>::THREADS) line_run_kernel(const S
 	for (; s < nsteps; s++) {
 		const int b = s & 1;
 		if (own) {
-			const Derived d = derive<true, false, false>(U[0], U[1], U[2], U[3], U[4], U[5], U[6], U[7], P.gas);
+			const Derived d = derive<true, false, false, false>(U[0], U[1], U[2], U[3], U[4], U[5], U[6], U[7], P.gas);
 			put(rank, b, t + 1, U, d);
 			if (t == 0) {
 				if (rank > 0) put(rank - 1, b, cells + 1, U, d);

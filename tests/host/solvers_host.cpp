@@ -93,3 +93,14 @@ extern "C" void host_face_flux(const int32_t solver, const int64_t n, const doub
 	default: solve<PAMHD_ROE_ATHENA>(n, neg, pos, g, flux, speed, flags); break;
 	}
 }
+
+// the correctly rounded helpers: 1 / x, a / x, sqrt(x)
+extern "C" void host_rounded(const int64_t n, const double* a, const double* x, double* inverse, double* quotient,
+                             double* root)
+{
+	for (int64_t i = 0; i < n; i++) {
+		inverse[i] = recip_rn(x[i]);
+		quotient[i] = quotient_rn(a[i], x[i], inverse[i]);
+		root[i] = sqrt_rn(x[i]);
+	}
+}

@@ -53,6 +53,15 @@ def states_at_rest(n, rng, mu0=4e-7 * np.pi, gamma=GAMMA_53):
     return s
 
 
+def unit_density_gas(n, rng):
+    """Random states of density 1 at rest without a field, and their sound speeds as IEEE arithmetic gives
+    them from the state."""
+    s = np.zeros((n, 8))
+    s[:, 0] = 1.0
+    s[:, 4] = 10.0 ** rng.uniform(-12, 12, n)
+    return s, np.sqrt(GAMMA_53 * (s[:, 4] * (GAMMA_53 - 1)))
+
+
 # the signs a face's state and its flux take when the face is mirrored along its normal
 MIRROR_STATE = np.array([1, -1, 1, 1, 1, -1, 1, 1.0])
 MIRROR_FLUX = np.array([-1, 1, -1, -1, -1, 1, -1, -1.0])

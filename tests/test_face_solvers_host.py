@@ -19,7 +19,7 @@ D = ctypes.POINTER(ctypes.c_double)
 
 @pytest.fixture(scope="module")
 def host():
-    """face_flux(solver, neg, pos, mu0) -> flux, speed, flags of the host build."""
+    """face_flux(solver, neg, pos, mu0) -> flux, speed, flags of the host build; .lib, the build."""
     os.makedirs(os.path.dirname(LIB), exist_ok=True)
     deps = [SRC, os.path.join(os.path.dirname(HERE), "pamhd_b200", "csrc", "mhd_device.cuh")]
     if not os.path.exists(LIB) or any(os.path.getmtime(d) > os.path.getmtime(LIB) for d in deps):
@@ -38,6 +38,7 @@ def host():
                          flags.ctypes.data_as(ctypes.POINTER(ctypes.c_uint32)))
         return flux, speed, flags
 
+    face_flux.lib = L
     return face_flux
 
 
@@ -91,3 +92,28 @@ def test_mirrored_faces(host, solver):
     fm, sm, gm = host(po.SOLVERS[solver], b * states.MIRROR_STATE, a * states.MIRROR_STATE)
     assert np.array_equal(g, gm) and np.array_equal(s, sm)
     assert np.array_equal(fm, np.where(g[:, None] == 0, f * states.MIRROR_FLUX, 0.0))
+
+
+def test_rounded_helpers(host):
+    """recip_rn, quotient_rn and sqrt_rn against IEEE division and square root, bit for bit."""
+    rng = np.random.default_rng(8)
+    n = 200000
+    x = rng.uniform(1.0, 2.0, n) * 2.0 ** rng.integers(-500, 500, n)
+    a = rng.uniform(-2.0, 2.0, n) * 2.0 ** rng.integers(-200, 200, n)
+    x[:3] = 1.0, 2.0 ** -700, 2.0 ** 1000
+    inverse, quotient, root = np.zeros(n), np.zeros(n), np.zeros(n)
+    host.lib.host_rounded(ctypes.c_int64(n), *(v.ctypes.data_as(D) for v in (a, x, inverse, quotient, root)))
+    assert np.array_equal(inverse, 1.0 / x)
+    assert np.array_equal(quotient, a / x)
+    assert np.array_equal(root, np.sqrt(x))
+    zero = np.zeros(1)
+    host.lib.host_rounded(ctypes.c_int64(1), *(v.ctypes.data_as(D) for v in (zero, zero, inverse, quotient, root)))
+    assert root[0] == 0.0
+
+
+def test_sound_speed_is_correctly_rounded(host):
+    """The speed of a face between equal states at rest without a field is the sound speed, whose root is
+    correctly rounded in the face fluxes (as in the staggered and local-time-stepping steps)."""
+    s, speed = states.unit_density_gas(5000, np.random.default_rng(9))
+    for solver in ("rusanov", "hll_athena", "hlld_athena", "roe_athena"):
+        assert np.array_equal(host(po.SOLVERS[solver], s, s)[1], speed), solver

@@ -165,6 +165,13 @@ def test_hll_uniform_states_at_rest():
     np.testing.assert_array_equal(grid.get_state(), U)
 
 
+@pytest.mark.parametrize("solver", list(po.SOLVERS))
+def test_sound_speed_is_correctly_rounded(solver):
+    """The face speed between equal states at rest without a field: the sound speed, correctly rounded."""
+    s, speed = states.unit_density_gas(5000, np.random.default_rng(9))
+    assert np.array_equal(pg.face_flux(po.SOLVERS[solver], s, s, None, 5 / 3, 1.0)[1], speed)
+
+
 def test_roe_small_transverse_field():
     """Roe faces whose transverse field's square is zero, subnormal or a small normal number: finite."""
     a, b = states.small_transverse_field_states(4000, np.random.default_rng(5), -165, -150)
