@@ -238,7 +238,7 @@ planes, 128 with 12, 129 with 8).
 */
 int default_work(pamhd_batch& b, const int sms)
 {
-	b.ty = step_tile(b.solver, b.yact, b.zact).rows;
+	b.ty = step_tile(b.solver, b.yact ? 2 : 1, b.zact).rows;
 	if (not b.zact) return build_work(b, 1);
 	const long long enough = 3LL * sms * b.kind(b.ty).resident() / 2;
 	for (const int planes: {64, 48, 32, 24, 16, 12}) {

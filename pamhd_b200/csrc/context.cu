@@ -209,8 +209,8 @@ int pamhd_gpu_create(const pamhd_cfg* cfg, pamhd_ctx** out)
 	PAMHD_TRY(validate(internal));
 	// the step's launch: rows of tiles along y and z chunks within a grid dimension's 65535 blocks
 	if (internal.n[1] > 1) {
-		const int rows = step_tile(internal.solver, true, internal.n[2] > 1).rows;
-		if ((internal.n[1] + rows - 1) / rows > 65535) return PAMHD_ERR_ARGUMENT;
+		const int rows = step_tile(internal.solver, internal.n[1], internal.n[2] > 1).rows;
+		if ((internal.n[1] + rows - 1) / rows > MAX_TILE_ROWS) return PAMHD_ERR_ARGUMENT;
 	}
 	if (internal.n[2] > 16 * 65535) return PAMHD_ERR_ARGUMENT;
 	pamhd_ctx* x = new (std::nothrow) pamhd_ctx;
@@ -245,7 +245,7 @@ int pamhd_gpu_create(const pamhd_cfg* cfg, pamhd_ctx** out)
 	}
 	set_params(*x);
 	// kernel attributes are set here, outside any stream capture
-	if (prepare_step_kernels(step_tile(internal.solver, internal.n[1] > 1, internal.n[2] > 1)) != PAMHD_OK) {
+	if (prepare_step_kernels(step_tile(internal.solver, internal.n[1], internal.n[2] > 1)) != PAMHD_OK) {
 		return fail(PAMHD_ERR_CUDA);
 	}
 	if (line_run_fits(x->base, internal.solver) and prepare_line_run(internal.solver) != PAMHD_OK) {

@@ -137,7 +137,7 @@ inline void tile_shape(const Tile_Kind& kind, const int nx, const int ny, int& t
 	double least = 1e300;
 	for (int w = 16; w <= 64; w++) {
 		for (int h = 2; h * w <= threads and w + h <= threads / 2; h++) {
-			if (w * (h + 2) + 2 * h > Tile_Kind::records_of(kind.rows) or (ny + h - 1) / h > 65535) continue;
+			if (w * (h + 2) + 2 * h > Tile_Kind::records_of(kind.rows) or (ny + h - 1) / h > MAX_TILE_ROWS) continue;
 			const double tiles = double((nx + w - 1) / w) * ((ny + h - 1) / h);
 			const int warps = (w * h + 31) / 32, spare = threads - w * h;
 			const int extra = std::max(0, w + h - 2 * spare);
@@ -214,7 +214,7 @@ inline bool grid_params(const pamhd_cfg& c, const Layout& L, Step_Params& P, con
 		const bool own_side = c.bc_lo[d] != PAMHD_BC_EXTERNAL or c.bc_hi[d] != PAMHD_BC_EXTERNAL;
 		if (P.active[d] and not P.periodic[d] and own_side and active_count > 1) needs_boundary_speeds = true;
 	}
-	const Tile_Kind kind = step_tile(c.solver, P.active[1], P.active[2]);
+	const Tile_Kind kind = step_tile(c.solver, c.n[1], P.active[2]);
 	tile_shape(kind, c.n[0], c.n[1], P.tw, P.th);
 	const long long tiles = (long long)((c.n[0] + P.tw - 1) / P.tw) * ((c.n[1] + P.th - 1) / P.th);
 	P.kchunk = planes_per_block(tiles, c.n[2], kind.resident());

@@ -151,7 +151,8 @@ int launch_face_flux(int solver, long long n, const double* neg, const double* p
                      const Gas& gas, double* flux, double* speed, uint32_t* flags, cudaStream_t stream);
 int launch_totals(const double* state, const Layout& L, double volume, double* partial, int nblocks,
                   cudaStream_t stream);
-Tile_Kind step_tile(int solver, bool yact, bool zact);
+constexpr int MAX_TILE_ROWS = 65535;   // of a launch: tiles along y are its grid's y dimension
+Tile_Kind step_tile(int solver, int ny, bool zact);
 int batch_tile_rows();
 int prepare_batch_kernels(const Tile_Kind& kind);
 int batch_blocks_per_sm(const Tile_Kind& kind, int* blocks);

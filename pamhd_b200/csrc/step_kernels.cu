@@ -1538,13 +1538,15 @@ per SM (a taller tile solves fewer halo faces and records per cell).  2-D
 grids: 32 x 4, four blocks of 128 threads per SM: the same 16 warps in
 blocks that wait for fewer others, and twice the blocks on small grids
 (HLLD against 32 x 8 tiles: 257 x 180 cells 10.1 us per step, was 11.2;
-512^2 33.8, was 34.4; 1024^2 118, was 128).  Roe's solver needs more
+512^2 33.8, was 34.4; 1024^2 118, was 128), but for grids with more rows than
+a launch has 32 x 4 tiles for.  Roe's solver needs more
 registers than either leaves, so it keeps 32 x 4 tiles at three blocks per
 SM (at four, 512^2 took 72 us instead of 66).
 */
-Tile_Kind step_tile(const int solver, const bool yact, const bool zact)
+Tile_Kind step_tile(const int solver, const int ny, const bool zact)
 {
-	return Tile_Kind{solver, not yact ? 1 : (solver == PAMHD_ROE_ATHENA or not zact ? TY_3D : TY_WIDE), zact};
+	const bool small = solver == PAMHD_ROE_ATHENA or (not zact and ny <= TY_3D * MAX_TILE_ROWS);
+	return Tile_Kind{solver, ny <= 1 ? 1 : (small ? TY_3D : TY_WIDE), zact};
 }
 
 int prepare_step_kernels(const Tile_Kind& kind)
@@ -1566,7 +1568,7 @@ int launch_step(const Step_Params& P, const int solver, cudaStream_t stream)
 	                 : P.kpart == 2 ? (nz - 2 + P.kchunk - 1) / P.kchunk
 	                 : (nz + P.kchunk - 1) / P.kchunk;
 	if (chunks < 1) return PAMHD_OK;  // no planes between the first and the last
-	return with_kind(step_tile(solver, P.active[1] != 0, P.active[2] != 0), [&](auto solver_, auto rows, auto zact) {
+	return with_kind(step_tile(solver, P.L.n[1], P.active[2] != 0), [&](auto solver_, auto rows, auto zact) {
 		const dim3 grid((P.L.n[0] + P.tw - 1) / P.tw, (P.L.n[1] + P.th - 1) / P.th, chunks + P.boundary);
 		step_kernel<solver_(), rows(), zact()>
 			<<<grid, TX * rows(), tile_bytes<solver_(), rows(), zact()>(), stream>>>(P);
@@ -1722,7 +1724,7 @@ int boundary_layers(const Step_Params& P, const int solver)
 		}
 	}
 	// about a face per thread
-	const int rows = step_tile(solver, P.active[1] != 0, P.active[2] != 0).rows;
+	const int rows = step_tile(solver, P.L.n[1], P.active[2] != 0).rows;
 	const long long layer = (long long)((P.L.n[0] + P.tw - 1) / P.tw) * ((P.L.n[1] + P.th - 1) / P.th) * TX * rows;
 	return int(min(1024LL, (faces + layer - 1) / layer));
 }

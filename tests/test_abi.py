@@ -63,6 +63,8 @@ def test_cfg_layout_matches_oracle():
     dict(bc_lo=(0, 0, 0), bc_hi=(1, 0, 0)),  # periodic on one side only
     dict(n=(2, 8 * 65535 + 1, 1)),           # more rows of 32 x 8 tiles than a launch can have
     dict(n=(2, 4 * 65535 + 1, 1), solver=4),  # Roe's 32 x 4 tiles
+    dict(n=(2, 8 * 65535 + 1, 2)),
+    dict(n=(2, 4 * 65535 + 1, 2), solver=4),
 ])
 def test_create_rejects_invalid_config(lib, change):
     kw = dict(n=(8, 8, 8), solver=pg.HLLD, cell_length=(0.1, 0.1, 0.1))
@@ -77,6 +79,20 @@ def test_null_arguments_rejected(lib):
     assert lib.pamhd_gpu_create(None, None) == pg.ERR_ARGUMENT
     assert lib.pamhd_gpu_step(None, 0.0, None, None) == pg.ERR_ARGUMENT
     assert lib.pamhd_gpu_destroy(None) == pg.OK
+
+
+@pytest.mark.parametrize("n,solver", [
+    ((2, 4 * 65535, 1), 4), ((2, 4 * 65535, 2), 4),
+    *[((2, ny, nz), s) for s in (0, 2, 3) for ny, nz in ((4 * 65535 + 1, 1), (300000, 1), (8 * 65535, 1), (8 * 65535, 2))],
+])
+def test_documented_rows_pass_the_checks(lib, n, solver):
+    """Up to 524,280 cells (262,140 with Roe) along the second dimension are accepted, in 2-D and 3-D."""
+    cfg = pg.Config(n=n, solver=solver, cell_length=(0.1, 0.1, 0.1)).to_c()
+    h = ctypes.c_void_p()
+    rc = lib.pamhd_gpu_create(ctypes.byref(cfg), ctypes.byref(h))
+    assert rc != pg.ERR_ARGUMENT
+    if h.value:
+        lib.pamhd_gpu_destroy(h)
 
 
 @pytest.mark.parametrize("n", [(1, 8, 8), (8, 1, 8), (1, 8, 1), (1, 1, 8)])

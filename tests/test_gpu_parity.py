@@ -119,6 +119,25 @@ def test_short_z_chunks_match_oracle(port, n, bc):
         assert field_err(gpu.get_state(), ora.get_state()) <= STEP_TOL, s
 
 
+@pytest.mark.parametrize("ny,solver", [(4 * 65535, "hlld_athena"), (4 * 65535 + 1, "hlld_athena"),
+                                       (300000, "rusanov"), (300000, "hll_athena"), (8 * 65535, "hlld_athena")])
+def test_many_rows_match_oracle(port, ny, solver):
+    """2-D grids of as many rows as a launch has 32 x 4 tiles for, one more (then 32 x 8 tiles), and the
+    most accepted, with COPY sides along y, whose ghost-ghost faces are solved.  Per step, the bar of
+    this file."""
+    n, kinds = (2, ny, 1), (0, pg.BC_COPY, 0)
+    U = states.smooth_3d((1, ny, 2), np.random.default_rng(3))
+    gpu, ora = pair(port, n, po.SOLVERS[solver], (0.5, 1.0 / ny, 1.0), states.GAMMA_53, 1.0, 0.4, kinds, kinds)
+    gpu.set_state(U)
+    ora.set_state(U)
+    for s in range(3):
+        dg = gpu.step(0.0 if s == 0 else 1.0)
+        do, flag, _, _ = ora.step(0.0 if s == 0 else 1.0)
+        assert flag == 0
+        assert abs(dg - do) <= 1e-13 * max(do, 1e-300), s
+        assert field_err(gpu.get_state(), ora.get_state()) <= STEP_TOL, s
+
+
 @pytest.mark.parametrize("normal", ["field", "none"])
 def test_roe_aligned_faces_match_oracle(port, normal):
     """Faces without a transverse field in the Roe average (no transverse field at all, or opposite
