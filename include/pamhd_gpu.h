@@ -258,8 +258,21 @@ next step, so that every slab takes the grid's dt
 */
 int pamhd_gpu_speed_slot(pamhd_ctx* ctx, void** slot);
 
-/* Waits for the context's stream; returns PAMHD_ERR_PHYSICS if a face failed. */
+/*
+Waits for the context's stream; returns PAMHD_ERR_PHYSICS if a face failed,
+PAMHD_ERR_TIMEOUT if a wait gave up (pamhd_gpu_set_wait_limit).
+*/
 int pamhd_gpu_sync(pamhd_ctx* ctx);
+
+/*
+Polls the barrier between the warps of a block makes in the 3-D steps before
+it gives up (>= 0; 0: no wait at all; default and most: 2^20, which only a
+fault could exhaust, since every warp arrives).  When it does, the status
+gets PAMHD_FLAG_TIMEOUT, pamhd_gpu_step and pamhd_gpu_sync return
+PAMHD_ERR_TIMEOUT, and later steps leave the grid as it is; the state is
+then mid-step (set it again).
+*/
+int pamhd_gpu_set_wait_limit(pamhd_ctx* ctx, int64_t polls);
 
 /* Simulation time, number of steps taken and the last dt (synchronises). */
 int pamhd_gpu_time(pamhd_ctx* ctx, double* time, int64_t* steps, double* last_dt);
@@ -409,7 +422,12 @@ equal pamhd_gpu_batch_steps bit for bit.  Does not wait for the GPU.
 */
 int pamhd_gpu_batch_run(pamhd_batch* batch, int32_t nsteps, double t_end);
 
-/* Polls a wait of pamhd_gpu_batch_run makes before it gives up (>= 0; 0: no wait at all). */
+/*
+Polls a wait of pamhd_gpu_batch_run makes before it gives up (>= 0; 0: no
+wait at all), and, up to its default of 2^20, a barrier between the warps of
+a block there and in pamhd_gpu_batch_steps: a box whose barrier gives up
+gets PAMHD_FLAG_TIMEOUT and holds its later steps.
+*/
 int pamhd_gpu_batch_set_wait_limit(pamhd_batch* batch, int64_t polls);
 
 /*

@@ -260,6 +260,12 @@ class Context:
         self._check(fn(self.h, dim, side, len(times), times.ctypes.data_as(_DP), states.ctypes.data_as(_DP)),
                     "pamhd_gpu_set_inflow")
 
+    def set_wait_limit(self, polls: int):
+        """Polls the barrier between a block's warps makes before it gives up (pamhd_gpu_set_wait_limit)."""
+        fn = self.L.pamhd_gpu_set_wait_limit
+        fn.argtypes = [ctypes.c_void_p, ctypes.c_int64]
+        self._check(fn(self.h, int(polls)), "pamhd_gpu_set_wait_limit")
+
     def save_dc(self, path: str, step: int, time: float, proton_mass: float = 1.0, start=(0.0, 0.0, 0.0)):
         """Writes the current state as a reference .dc file (pamhd_dc_write)."""
         c = self.cfg
@@ -907,7 +913,8 @@ class Batch:
         self._check(fn(self.h, int(n), float(t_end)), "pamhd_gpu_batch_run")
 
     def set_wait_limit(self, polls: int):
-        """Polls a wait of the persistent run makes before it gives up (pamhd_gpu_batch_set_wait_limit)."""
+        """Polls a wait of the persistent run, or a barrier between a block's warps, makes before it
+        gives up (pamhd_gpu_batch_set_wait_limit)."""
         fn = self.L.pamhd_gpu_batch_set_wait_limit
         fn.argtypes = [ctypes.c_void_p, ctypes.c_int64]
         self._check(fn(self.h, int(polls)), "pamhd_gpu_batch_set_wait_limit")

@@ -477,7 +477,7 @@ int pamhd_gpu_adjoint(pamhd_ctx* x, const int32_t nsteps, const int32_t every, c
 		Status s;
 		PAMHD_TRY(check(cudaMemcpyAsync(&s, x->status, sizeof s, cudaMemcpyDeviceToHost, x->stream)));
 		PAMHD_TRY(check(cudaStreamSynchronize(x->stream)));
-		if (s.flags != 0) return PAMHD_ERR_PHYSICS;
+		PAMHD_TRY(status_code(s));
 		for (int n = 0; n < nsteps; n++) dts[n] = hist[(x->steps - nsteps + n) % x->hist_len];
 	}
 	if (dt_out != nullptr) std::copy(dts.begin(), dts.end(), dt_out);

@@ -273,7 +273,8 @@ int issue_step(pamhd_batch& b)
 		PAMHD_TRY(launch_batch_boundary_speeds(b.d_params[b.cur], b.nboxes, b.largest_plane, phase, b.solver,
 		                                       b.stream));
 	}
-	PAMHD_TRY(launch_batch_step(b.d_params[b.cur], b.d_items, b.nitems, phase, b.grid, b.kind(b.ty), b.stream));
+	PAMHD_TRY(launch_batch_step(b.d_params[b.cur], b.d_items, b.nitems, phase,
+	                            int(std::min<long long>(b.wait_limit, BARRIER_POLLS)), b.grid, b.kind(b.ty), b.stream));
 	b.cur ^= 1;
 	b.steps++;
 	return PAMHD_OK;
@@ -636,10 +637,14 @@ int pamhd_gpu_batch_set_wait_limit(pamhd_batch* b, const int64_t polls)
 {
 	if (b == nullptr or polls < 0) return PAMHD_ERR_ARGUMENT;
 	b->wait_limit = polls;
-	// the limit is a launch argument: a graph captured with the old one is captured again
+	// the limit is a launch argument: graphs captured with the old one are captured again
+	PAMHD_TRY(check(cudaSetDevice(b->device)));
+	PAMHD_TRY(check(cudaStreamSynchronize(b->stream)));
+	if (b->graph != nullptr) {
+		cudaGraphExecDestroy(b->graph);
+		b->graph = nullptr;
+	}
 	if (b->run_graph != nullptr) {
-		PAMHD_TRY(check(cudaSetDevice(b->device)));
-		PAMHD_TRY(check(cudaStreamSynchronize(b->stream)));
 		cudaGraphExecDestroy(b->run_graph);
 		b->run_graph = nullptr;
 		b->run_key = -1;
@@ -818,9 +823,7 @@ int pamhd_gpu_batch_sync(pamhd_batch* b)
 	for (const auto& x: s) {
 		if (x.flags & PAMHD_FLAG_TIMEOUT) return PAMHD_ERR_TIMEOUT;
 	}
-	for (const auto& x: s) {
-		if (x.flags != 0) return PAMHD_ERR_PHYSICS;
-	}
+	for (const auto& x: s) PAMHD_TRY(status_code(x));
 	return PAMHD_OK;
 }
 

@@ -149,6 +149,13 @@ int fill_ghosts(pamhd_ctx& x)
 	return launch_fill_ghosts_values(P, x.state[1], lo, hi, x.stream);
 }
 
+// after a change of the parameters that captured steps hold
+void drop_graph(pamhd_ctx& x)
+{
+	if (x.graph != nullptr) cudaGraphExecDestroy(x.graph);
+	x.graph = nullptr;
+}
+
 int capture_graph(pamhd_ctx& x)
 {
 	if (x.graph != nullptr) return PAMHD_OK;
@@ -360,7 +367,7 @@ int pamhd_gpu_step(pamhd_ctx* x, const double max_dt, double* dt_taken, double* 
 			max_signal[x->map.perm[a]] = v;
 		}
 	}
-	return s.flags != 0 ? PAMHD_ERR_PHYSICS : PAMHD_OK;
+	return status_code(s);
 }
 
 int pamhd_gpu_steps(pamhd_ctx* x, const int32_t nsteps, const double t_end)
@@ -461,11 +468,7 @@ int pamhd_gpu_set_inflow(pamhd_ctx* x, const int32_t user_dim, const int32_t sid
 	const Inflow_Table table{dev, dev + nt, count};
 	PAMHD_TRY(check(cudaMemcpy(x->inflow_tables + 2 * dim + side, &table, sizeof table, cudaMemcpyHostToDevice)));
 	x->base.inflow = x->inflow_tables;
-	// the captured steps hold the old parameters
-	if (x->graph != nullptr) {
-		cudaGraphExecDestroy(x->graph);
-		x->graph = nullptr;
-	}
+	drop_graph(*x);
 	// the current state's ghosts take the value of the current time
 	if (x->loaded) {
 		Clock c;
@@ -476,6 +479,16 @@ int pamhd_gpu_set_inflow(pamhd_ctx* x, const int32_t user_dim, const int32_t sid
 		PAMHD_TRY(launch_fill_ghosts_values(x->base, x->state[x->cur], lo, hi, x->stream));
 		PAMHD_TRY(check(cudaStreamSynchronize(x->stream)));
 	}
+	return PAMHD_OK;
+}
+
+int pamhd_gpu_set_wait_limit(pamhd_ctx* x, const int64_t polls)
+{
+	if (x == nullptr or polls < 0) return PAMHD_ERR_ARGUMENT;
+	PAMHD_TRY(check(cudaSetDevice(x->device)));
+	PAMHD_TRY(check(cudaStreamSynchronize(x->stream)));
+	x->base.barrier_polls = int(std::min<int64_t>(polls, BARRIER_POLLS));
+	drop_graph(*x);
 	return PAMHD_OK;
 }
 
@@ -515,7 +528,7 @@ int pamhd_gpu_sync(pamhd_ctx* x)
 	PAMHD_TRY(check(cudaSetDevice(x->device)));
 	Status s;
 	PAMHD_TRY(read_status(*x, s));
-	return s.flags != 0 ? PAMHD_ERR_PHYSICS : PAMHD_OK;
+	return status_code(s);
 }
 
 int pamhd_gpu_time(pamhd_ctx* x, double* time, int64_t* steps, double* last_dt)

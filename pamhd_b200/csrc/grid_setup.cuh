@@ -214,6 +214,7 @@ inline bool grid_params(const pamhd_cfg& c, const Layout& L, Step_Params& P, con
 		const bool own_side = c.bc_lo[d] != PAMHD_BC_EXTERNAL or c.bc_hi[d] != PAMHD_BC_EXTERNAL;
 		if (P.active[d] and not P.periodic[d] and own_side and active_count > 1) needs_boundary_speeds = true;
 	}
+	P.barrier_polls = BARRIER_POLLS;
 	const Tile_Kind kind = step_tile(c.solver, c.n[1], P.active[2]);
 	tile_shape(kind, c.n[0], c.n[1], P.tw, P.th);
 	const long long tiles = (long long)((c.n[0] + P.tw - 1) / P.tw) * ((c.n[1] + P.th - 1) / P.th);

@@ -56,6 +56,13 @@ struct Status {
 	unsigned long long first;
 };
 
+// what a call returns for it
+inline int status_code(const Status& s)
+{
+	if (s.flags & PAMHD_FLAG_TIMEOUT) return PAMHD_ERR_TIMEOUT;
+	return s.flags != 0 ? PAMHD_ERR_PHYSICS : PAMHD_OK;
+}
+
 // limits read by the step kernel from device memory (so graphs need no re-capture)
 struct Control {
 	double max_dt;   // >= 0: cap of dt; < 0: cap is t_end - t
@@ -109,6 +116,7 @@ struct Step_Params {
 	double forced_dt;    // >= 0: the step's dt (a prescribed schedule); < 0: the CFL rule
 	int kpart;           // z planes a launch computes: 0 all, 1 the first and last only, 2 the others
 	int boundary;        // block layers of the step's launch that solve ghost-ghost faces (0: none)
+	int barrier_polls;   // polls a block's split barrier makes before it gives up
 	const Inflow_Table* inflow;  // [3][2] by dimension and side (lo, hi) in device memory, or nullptr
 };
 
@@ -156,7 +164,7 @@ Tile_Kind step_tile(int solver, int ny, bool zact);
 int batch_tile_rows();
 int prepare_batch_kernels(const Tile_Kind& kind);
 int batch_blocks_per_sm(const Tile_Kind& kind, int* blocks);
-int launch_batch_step(const Step_Params* boxes, const int4* items, int nitems, int phase, int grid,
+int launch_batch_step(const Step_Params* boxes, const int4* items, int nitems, int phase, int barrier_polls, int grid,
                       const Tile_Kind& kind, cudaStream_t stream);
 int launch_batch_boundary_speeds(const Step_Params* boxes, int nboxes, int largest, int phase, int solver,
                                  cudaStream_t stream);
@@ -167,6 +175,8 @@ int launch_batch_run(const Step_Params* boxes_even, const Step_Params* boxes_odd
                      const int* box_items, unsigned int* done, int nboxes, long long step0, int nsteps,
                      Run_Sync* sync, long long wait_limit, int grid, const Tile_Kind& kind,
                      cudaStream_t stream);
+// polls of a block's split barrier where the caller set no limit (its warps all arrive: never reached)
+constexpr int BARRIER_POLLS = 1 << 20;
 constexpr int BOUNDARY_CHUNK = 4096;  // ghost-ghost faces per boundary work item of the persistent run
 
 } // namespace pamhd_b200

@@ -148,20 +148,24 @@ struct Split_Barrier {
 		}
 	}
 
-	// false (with PAMHD_FLAG_TIMEOUT raised) when the other warps did not arrive within the poll limit
-	__device__ __forceinline__ bool wait(Status* status)
+	// false when the other warps did not arrive within the poll limit.  The step has then failed: it is
+	// dated, as a failing face's (record_failure), so that the grid or box holds its later steps.  The
+	// warp goes on to the block's next barrier, which it reaches like the others: this use is then
+	// complete, and the phase in step again
+	__device__ __forceinline__ bool wait(const Step_Params& P)
 	{
 		const uint32_t parity = phase & 1u;
 		phase++;
 		#pragma unroll 1
-		for (int poll = 0; poll < (1 << 20); poll++) {
+		for (int poll = 0; poll < P.barrier_polls; poll++) {
 			uint32_t done;
 			asm volatile("{\n\t.reg .pred p;\n\t"
 			             "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
 			             "selp.u32 %0, 1, 0, p;\n\t}" : "=r"(done) : "r"(addr), "r"(parity) : "memory");
 			if (done) return true;
 		}
-		atomicOr(&status->flags, (unsigned int)PAMHD_FLAG_TIMEOUT);
+		atomicOr(&P.status->flags, (unsigned int)PAMHD_FLAG_TIMEOUT);
+		P.status->fail_step = (unsigned int)(__ldcg(&P.clock[P.phase].steps) + 1);
 		return false;
 	}
 };
@@ -716,8 +720,9 @@ __device__ __forceinline__ void tile_step(const Step_Params& P, double* const sm
 		}
 		// (d) the own cell: U += (F- - F+) dt/dx, then y, then z (solve.hpp:1551-1587)
 		if (inner) {
-			if (ZACT and not bar.wait(P.status)) return;
-			if (own) {
+			// without the other warps' fluxes (a wait that gave up) the cell stays unwritten
+			const bool arrived = not ZACT or bar.wait(P);
+			if (own and arrived) {
 				// the flux row of each xyz variable in the x and the y face frames; -1: the normal
 				// field component, whose flux is zero unless the solver keeps an eighth row
 				constexpr int XROW[8] = {0, 1, 2, 3, 4, NF == 8 ? 7 : -1, 5, 6};
@@ -768,7 +773,8 @@ The block holding a box's first item advances that box's clock.
 template <int SOLVER, int TY, bool ZACT>
 __global__ void __launch_bounds__(TX * TY, Tile_Kind::resident_of(SOLVER, TY, ZACT)) batch_step_kernel(const Step_Params* __restrict__ boxes,
                                                                   const int4* __restrict__ items,
-                                                                  const int nitems, const int phase)
+                                                                  const int nitems, const int phase,
+                                                                  const int barrier_polls)
 {
 	extern __shared__ __align__(16) double smem[];
 	__shared__ Step_Params sp;
@@ -784,6 +790,7 @@ __global__ void __launch_bounds__(TX * TY, Tile_Kind::resident_of(SOLVER, TY, ZA
 		if (tid == 0) {
 			sp = boxes[w.x];
 			sp.phase = phase;
+			sp.barrier_polls = barrier_polls;
 		}
 		__syncthreads();
 		const bool first = w.y == 0 and w.z == 0 and w.w == 0;
@@ -1119,6 +1126,7 @@ __global__ void __launch_bounds__(TX * TY, Tile_Kind::resident_of(SOLVER, TY, ZA
 			s_go = go;
 			sp = boxes[w.x];
 			sp.phase = int((step0 + s) % 3);
+			sp.barrier_polls = int(min(wait_limit, (long long)BARRIER_POLLS));
 		}
 		__syncthreads();
 		if (not s_go) return;
@@ -1691,11 +1699,11 @@ int launch_batch_run(const Step_Params* even, const Step_Params* odd, const int4
 }
 
 int launch_batch_step(const Step_Params* boxes, const int4* items, const int nitems, const int phase,
-                      const int grid, const Tile_Kind& kind, cudaStream_t stream)
+                      const int barrier_polls, const int grid, const Tile_Kind& kind, cudaStream_t stream)
 {
 	return with_kind(kind, [&](auto solver, auto rows, auto zact) {
 		batch_step_kernel<solver(), rows(), zact()>
-			<<<grid, TX * rows(), tile_bytes<solver(), rows(), zact()>(), stream>>>(boxes, items, nitems, phase);
+			<<<grid, TX * rows(), tile_bytes<solver(), rows(), zact()>(), stream>>>(boxes, items, nitems, phase, barrier_polls);
 		return status_of(cudaGetLastError());
 	});
 }

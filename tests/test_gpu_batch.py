@@ -363,3 +363,38 @@ def test_persistent_run_wait_timeout_is_reported():
     ref.sync()
     for i in range(len(cfgs)):
         np.testing.assert_array_equal(batch.get_state(i), ref.get_state(i))
+
+
+@pytest.mark.parametrize("persistent", [False, True])
+def test_block_barrier_timeout_holds_the_boxes(persistent):
+    """Block barriers that give up (a limit of 0 polls): every box is flagged with PAMHD_FLAG_TIMEOUT in
+    its first step and, in the launches per step, holds its clock from there; usable again after
+    set_state."""
+    cfgs, U0s = small_ensemble()
+    batch, ref = pg.Batch(cfgs), pg.Batch(cfgs)
+    run = (lambda b, n: b.run(n)) if persistent else (lambda b, n: b.steps(n))
+    for i, U in enumerate(U0s):
+        batch.set_state(i, U)
+    batch.steps(7)   # a captured graph holds the old limit
+    batch.sync()
+    batch.set_wait_limit(0)
+    for i, U in enumerate(U0s):
+        batch.set_state(i, U)
+    run(batch, 7)
+    with pytest.raises(pg.PamhdError) as e:
+        batch.sync()
+    assert e.value.code == pg.ERR_TIMEOUT
+    for i, c in enumerate(cfgs):
+        assert c.n[2] > 1 and batch.status(i)[0] & pg.FLAG_TIMEOUT
+        if not persistent:
+            assert batch.time(i)[1] == 1
+    batch.set_wait_limit(10_000_000)
+    for i, U in enumerate(U0s):
+        batch.set_state(i, U)
+        ref.set_state(i, U)
+    run(batch, 7)
+    run(ref, 7)
+    batch.sync()
+    ref.sync()
+    for i in range(len(cfgs)):
+        np.testing.assert_array_equal(batch.get_state(i), ref.get_state(i))

@@ -119,6 +119,44 @@ def test_short_z_chunks_match_oracle(port, n, bc):
         assert field_err(gpu.get_state(), ora.get_state()) <= STEP_TOL, s
 
 
+@pytest.mark.parametrize("solver", list(po.SOLVERS))
+def test_block_barrier_timeout_is_reported(solver):
+    """A block barrier that gives up (a limit of 0 polls) ends in PAMHD_ERR_TIMEOUT and
+    PAMHD_FLAG_TIMEOUT, in a single step and in replayed ones; later steps hold the grid and its clock;
+    after set_state with the limit restored the grid steps as a new one."""
+    n = (40, 21, 33)
+    U = states.smooth_3d(n[::-1], np.random.default_rng(2))
+    cfg = pg.Config(n=n, solver=po.SOLVERS[solver], cell_length=(0.1, 0.12, 0.09), time_step_factor=0.4)
+    a, b = pg.Context(cfg), pg.Context(cfg)
+    a.set_state(U)
+    a.steps(13, 1e300)   # a captured graph holds the old limit
+    a.sync()
+    a.set_wait_limit(0)
+    with pytest.raises(pg.PamhdError) as e:
+        a.step(1.0)
+    assert e.value.code == pg.ERR_TIMEOUT
+    assert a.status()[0] & pg.FLAG_TIMEOUT
+    held, clock = a.get_state(), a.time()[:2]
+    a.steps(13, 1e300)
+    with pytest.raises(pg.PamhdError) as e:
+        a.sync()
+    assert e.value.code == pg.ERR_TIMEOUT
+    np.testing.assert_array_equal(a.get_state(), held)
+    assert a.time()[:2] == clock
+    a.set_state(U)
+    a.steps(13, 1e300)   # fails in its first step
+    with pytest.raises(pg.PamhdError) as e:
+        a.sync()
+    assert e.value.code == pg.ERR_TIMEOUT and a.time()[1] == 1
+    a.set_wait_limit(1 << 20)
+    for g in (a, b):
+        g.set_state(U)
+        g.steps(13, 1e300)
+        g.sync()
+    np.testing.assert_array_equal(a.get_state(), b.get_state())
+    assert a.time() == b.time()
+
+
 @pytest.mark.parametrize("ny,solver", [(4 * 65535, "hlld_athena"), (4 * 65535 + 1, "hlld_athena"),
                                        (300000, "rusanov"), (300000, "hll_athena"), (8 * 65535, "hlld_athena")])
 def test_many_rows_match_oracle(port, ny, solver):
