@@ -96,6 +96,10 @@ struct Derived {
 	uint32_t bad;
 };
 
+// in Derived::bad, alone: round-off decides whether the reference takes the cell's fast speed
+// (reference_wave), and derive was told to leave that to the caller
+constexpr uint32_t OPEN_WAVE = 1u << 7;
+
 #ifdef __CUDACC__
 // the hardware's estimates of 1/x and 1/sqrt(x), which take a subnormal x for zero (a host build of
 // these solvers brings its own)
@@ -192,6 +196,32 @@ __device__ __forceinline__ double sqrt_rn(const double x)
 }
 
 /*
+Whether get_fast_magnetosonic_speed (mhd/common.hpp:418-491) takes a cell, in
+the frame of the face: the argument of its inner root,
+a^4 + v_A^4 + 2 a^2 v_A^2 (1 - 2 cos^2), cancels to round-off, of either
+sign, where the sound and Alfven speeds are equal and the field is along the
+normal.  Its operations one for one, each rounded on its own.
+*/
+__device__ __forceinline__ bool reference_wave(
+	const double rho, const double m0, const double m1, const double m2, const double E,
+	const double b0, const double b1, const double b2, const Gas& g
+) {
+	const auto mul = [](const double x, const double y) { return __dmul_rn(x, y); };
+	const auto add = [](const double x, const double y) { return __dadd_rn(x, y); };
+	const auto sub = [](const double x, const double y) { return __dsub_rn(x, y); };
+	const double i = recip_rn(rho);
+	const double bsq = add(add(mul(b0, b0), mul(b1, b1)), mul(b2, b2));
+	const double kinetic = mul(mul(0.5, i), add(add(mul(m0, m0), mul(m1, m1)), mul(m2, m2)));
+	const double p = mul(sub(sub(E, kinetic), mul(mul(0.5, g.inv_mu0), bsq)), g.gamma - 1.0);
+	const double sound = sqrt_rn(quotient_rn(mul(g.gamma, p), rho, i)), b = sqrt_rn(bsq);
+	const double mass = sqrt_rn(mul(g.mu0, rho));
+	const double alfven = quotient_rn(b, mass, recip_rn(mass)), cosine = quotient_rn(b0, b, recip_rn(b));
+	const double s2 = mul(sound, sound), a2 = mul(alfven, alfven);
+	const double part = sub(1.0, mul(2.0, mul(cosine, cosine)));
+	return is_positive_normal(add(add(mul(s2, s2), mul(a2, a2)), mul(mul(mul(2.0, s2), a2), part)));
+}
+
+/*
 Every operation below is an explicitly rounded intrinsic, so that every
 inlined copy of this function computes the same bits for the same cell
 (the halo of one tile is the interior of the next).
@@ -199,11 +229,16 @@ inlined copy of this function computes the same bits for the same cell
 The fast speed: c_f^2 = (a^2 + v_A^2 + root) / 2 with
 root^2 = (a^2 + v_A^2)^2 - 4 a^2 v_A,n^2, written as
 (a^2 - v_A^2)^2 + 4 a^2 v_A,t^2 (v_A,t from the field across the axis):
-no division by B^2 and no cancellation.  ROUNDED: both roots correctly
-rounded, three operations more each; without it the speed's error is 8 %
-larger (rms; the cell-centred steps' records).
+no division by B^2 and no cancellation.
+
+RECORD: for the cell-centred steps' records.  Without it both roots are
+correctly rounded, three operations more each (with it the speed's error is
+8 % larger, rms), and a cell whose wave speed round-off decides is judged
+here, for the axes asked for; with it that is left open (OPEN_WAVE) and the
+speeds are given: the judgement, though it is hardly ever made, took 1.8 %
+of a 256^3 step here.
 */
-template <bool NEED_X, bool NEED_Y, bool NEED_Z, bool ROUNDED = true>
+template <bool NEED_X, bool NEED_Y, bool NEED_Z, bool RECORD = false>
 __device__ __forceinline__ Derived derive(
 	const double rho, const double mx, const double my, const double mz,
 	const double E, const double bx, const double by, const double bz, const Gas& g
@@ -227,7 +262,7 @@ __device__ __forceinline__ Derived derive(
 		d.bad = PAMHD_FLAG_PRESSURE;
 	}
 	const double cs2 = __dmul_rn(__dmul_rn(g.gamma, d.p), d.rinv);
-	const auto root = [](const double x) { return ROUNDED ? sqrt_rn(x) : sqrt_nr(x); };
+	const auto root = [](const double x) { return RECORD ? sqrt_nr(x) : sqrt_rn(x); };
 	const bool need[3] = {NEED_X, NEED_Y, NEED_Z};
 	if (b2 > 0.0) {
 		const double im = __dmul_rn(g.inv_mu0, d.rinv);
@@ -235,7 +270,12 @@ __device__ __forceinline__ Derived derive(
 		const double sum2 = __dadd_rn(cs2, va2), diff2 = __dsub_rn(cs2, va2);
 		const double base = __dmul_rn(diff2, diff2);
 		const double cross = __dmul_rn(__dmul_rn(4.0, cs2), im);
-		bool wave_ok = is_positive_normal(sum2) and is_finite(b2);
+		const bool sum_ok = is_positive_normal(sum2) and is_finite(b2);
+		bool wave_ok = sum_ok;
+		// the high word of some 2^-40 (a^2 + v_A^2)^2 (twice a logarithm, in integers): where the root's
+		// argument is smaller, round-off decides whether the reference takes the cell
+		const int low = int(2u * ((unsigned int)__double2hiint(sum2) - (0x1ff80000u + (20u << 20))));
+		bool open[3] = {false, false, false};
 		#pragma unroll
 		for (int a = 0; a < 3; a++) {
 			if (not need[a]) {
@@ -243,17 +283,40 @@ __device__ __forceinline__ Derived derive(
 				continue;
 			}
 			const double to_sqrt = __fma_rn(cross, __dadd_rn(bb[(a + 1) % 3], bb[(a + 2) % 3]), base);
+			open[a] = __double2hiint(to_sqrt) < low;
 			wave_ok = wave_ok and is_positive_normal(to_sqrt);
 			d.cf[a] = root(__dmul_rn(0.5, __dadd_rn(sum2, root(to_sqrt))));
 		}
-		if (d.bad == 0 and not wave_ok) d.bad = PAMHD_FLAG_WAVE_SPEED;
+		const bool undecided = (open[0] or open[1] or open[2]) and sum_ok;
+		if (d.bad == 0) d.bad = undecided ? OPEN_WAVE : (wave_ok ? 0u : (uint32_t)PAMHD_FLAG_WAVE_SPEED);
+		if (not RECORD and d.bad == OPEN_WAVE) {
+			d.bad = 0;
+			#pragma unroll 1
+			for (int a = 0; a < 3; a++) {
+				const auto turn = [a](const double x, const double y, const double z) { return a == 0 ? x : (a == 1 ? y : z); };
+				if ((a == 0 ? open[0] : (a == 1 ? open[1] : open[2]))
+					and not reference_wave(rho, turn(mx, my, mz), turn(my, mz, mx), turn(mz, mx, my), E,
+					                       turn(bx, by, bz), turn(by, bz, bx), turn(bz, bx, by), g)) {
+					d.bad = PAMHD_FLAG_WAVE_SPEED;
+				}
+			}
+		}
 	} else {
 		d.cf[0] = d.cf[1] = d.cf[2] = root(cs2);
 		if (d.bad == 0 and not is_finite(b2)) d.bad = PAMHD_FLAG_WAVE_SPEED;
 	}
 	// a refused cell: no face of it counts, its speeds stay numbers
-	if (d.bad != 0) d.cf[0] = d.cf[1] = d.cf[2] = 0.0;
+	if (d.bad != 0 and d.bad != OPEN_WAVE) d.cf[0] = d.cf[1] = d.cf[2] = 0.0;
 	return d;
+}
+
+// in the frame of faces normal to axis a (known at run time): cf[0] is the fast speed along it
+__device__ __forceinline__ Derived derive_along(const int a, const double U[8], const Gas& g)
+{
+	const auto turn = [a](const double x, const double y, const double z) { return a == 0 ? x : (a == 1 ? y : z); };
+	return derive<true, false, false>(
+		U[0], turn(U[1], U[2], U[3]), turn(U[2], U[3], U[1]), turn(U[3], U[1], U[2]), U[4],
+		turn(U[5], U[6], U[7]), turn(U[6], U[7], U[5]), turn(U[7], U[5], U[6]), g);
 }
 
 // one cell seen from a face, rotated into the face frame

@@ -237,7 +237,8 @@ __device__ void record_failure(const Step_Params& P, const uint32_t flag, const 
 	P.status->fail_step = (unsigned int)(__ldcg(&P.clock[P.phase].steps) + 1);
 }
 
-__device__ __forceinline__ void flush_speeds(const Step_Params& P, double smax[3], bool zero)
+// folds a block's speeds into the step's reduction; returns whether any of its threads has `open` set
+__device__ __forceinline__ bool flush_speeds(const Step_Params& P, double smax[3], bool zero, bool open = false)
 {
 	__shared__ double part[3][32];
 	__shared__ int part_zero[32];
@@ -245,7 +246,7 @@ __device__ __forceinline__ void flush_speeds(const Step_Params& P, double smax[3
 	const int warp = tid >> 5, lane = tid & 31, warps = (blockDim.x * blockDim.y + 31) >> 5;
 	#pragma unroll
 	for (int d = 0; d < 3; d++) smax[d] = warp_max(smax[d]);
-	const int z = __any_sync(0xffffffffu, zero);
+	const int z = (__any_sync(0xffffffffu, zero) ? 1 : 0) | (__any_sync(0xffffffffu, open) ? 2 : 0);
 	if (lane == 0) {
 		part[0][warp] = smax[0];
 		part[1][warp] = smax[1];
@@ -253,9 +254,10 @@ __device__ __forceinline__ void flush_speeds(const Step_Params& P, double smax[3
 		part_zero[warp] = z;
 	}
 	__syncthreads();
+	int any = 0;
+	for (int w = 0; w < warps; w++) any |= part_zero[w];
 	if (tid == 0) {
 		Speed_Max& r = P.red[(P.phase + 1) % 3];
-		int any_zero = 0;
 		#pragma unroll
 		for (int d = 0; d < 3; d++) {
 			double m = 0.0;
@@ -264,9 +266,9 @@ __device__ __forceinline__ void flush_speeds(const Step_Params& P, double smax[3
 				atomicMax(&r.smax[d], (unsigned long long)__double_as_longlong(m));
 			}
 		}
-		for (int w = 0; w < warps; w++) any_zero |= part_zero[w];
-		if (any_zero) atomicOr(&r.zero, 1u);
+		if ((any & 1) != 0) atomicOr(&r.zero, 1u);
 	}
+	return (any & 2) != 0;
 }
 
 __device__ __forceinline__ void store_cell(double* out, const Layout& L, const int i, const int j,
@@ -336,23 +338,27 @@ Read a cell from HBM, derive its per-cell quantities into a record slot.
 CO: loads at L2 (ld.global.cg) instead of through the read-only cache, for a
 persistent launch whose later steps read what other blocks wrote (the
 non-coherent L1 could hold a line of the same buffer from two steps before).
+A cell whose wave speed round-off decides is taken for now, and open set
+(settle_tile).
 */
 template <bool CX, bool CY, bool CZ, bool CO, class Meanwhile>
 __device__ __forceinline__ double load_record(const Step_Params& P, double* rec, uint8_t* bad, const int cells,
-                                              const int ri, const long long off, const Meanwhile& meanwhile)
+                                              const int ri, const long long off, bool& open,
+                                              const Meanwhile& meanwhile)
 {
 	double U[8];
 	#pragma unroll
 	for (int v = 0; v < 8; v++) U[v] = CO ? __ldcg(P.in + v * P.L.var + off) : __ldg(P.in + v * P.L.var + off);
 	meanwhile();   // while the loads are on their way
-	const Derived d = derive<CX, CY, CZ, false>(U[0], U[1], U[2], U[3], U[4], U[5], U[6], U[7], P.gas);
+	const Derived d = derive<CX, CY, CZ, true>(U[0], U[1], U[2], U[3], U[4], U[5], U[6], U[7], P.gas);
 	#pragma unroll
 	for (int v = 0; v < 8; v++) rec[v * cells + ri] = U[v];
 	rec[R_RINV * cells + ri] = d.rinv;
 	rec[R_PT * cells + ri] = d.pt;
 	if (CX) rec[(R_CF + 0) * cells + ri] = d.cf[0];
 	if (CY) rec[(R_CF + 1) * cells + ri] = d.cf[1];
-	bad[ri] = uint8_t(d.bad);
+	bad[ri] = uint8_t(d.bad & ~OPEN_WAVE);
+	open = open or d.bad == OPEN_WAVE;
 	// the fast speed along z, for the caller's z faces
 	return CZ ? d.cf[2] : 0.0;
 }
@@ -515,6 +521,47 @@ __device__ void tile_hold(const Step_Params& P, const int bx, const int by, cons
 }
 
 /*
+Judges the cells of a tile whose wave speed round-off decides, as the
+reference judges them at each face they have: along its normal, and the face
+is named by the cell before it.  An own cell has two faces along each axis; a
+ghost of a side that is not periodic has one, along the side's axis.  By
+blocks that met such a cell, after their planes (in the planes' loop the
+judgement took 1.4 % of a 256^3 step, unused: registers and code).
+*/
+__device__ void settle_tile(const Step_Params& P, const int bx, const int by, const int bz)
+{
+	int kb, ke;
+	tile_planes(P, bz, kb, ke);
+	const int ty = threadIdx.x / P.tw, tx = threadIdx.x - ty * P.tw;
+	const int gx = bx * P.tw + tx, gy = by * P.th + ty;
+	if (ty >= P.th or gx >= P.L.n[0] or gy >= P.L.n[1]) return;
+	// axis a, of the cell at (i, j, k): whether the reference refuses it
+	const auto refused = [&](const int a, const int i, const int j, const int k) {
+		const long long off = P.L.offset(i, j, k);
+		double U[8];
+		#pragma unroll
+		for (int v = 0; v < 8; v++) U[v] = __ldcg(P.in + v * P.L.var + off);
+		return derive_along(a, U, P.gas).bad == PAMHD_FLAG_WAVE_SPEED;
+	};
+	#pragma unroll 1
+	for (int k = kb; k < ke; k++) {
+		#pragma unroll 1
+		for (int a = 0; a < 3; a++) {
+			if (not P.active[a]) continue;
+			const int di = a == 0 ? 1 : 0, dj = a == 1 ? 1 : 0, dk = a == 2 ? 1 : 0;
+			const int at = a == 0 ? gx : (a == 1 ? gy : k);
+			const bool own = refused(a, gx, gy, k);
+			if (own or (not P.periodic[a] and at == 0 and refused(a, gx - di, gy - dj, k - dk))) {
+				record_failure(P, PAMHD_FLAG_WAVE_SPEED, gx - di, gy - dj, k - dk, a + 1);
+			}
+			if (own or (not P.periodic[a] and at == P.L.n[a] - 1 and refused(a, gx + di, gy + dj, k + dk))) {
+				record_failure(P, PAMHD_FLAG_WAVE_SPEED, gx, gy, k, a + 1);
+			}
+		}
+	}
+}
+
+/*
 One work item of a step: the tile (bx, by) of tw x th columns over the z
 chunk bz, marched plane by plane; the face speeds are folded into
 s0, s1, s2 and zero (flushed by the caller).  Shared by the single-grid
@@ -544,7 +591,7 @@ Roe's 4 % to registers).
 template <int SOLVER, int TY, bool ZACT, bool CO = false, bool LATE = false>
 __device__ __forceinline__ void tile_step(const Step_Params& P, double* const smem, Split_Barrier& bar,
                                           double dt, const int bx, const int by, const int bz,
-                                          double& s0, double& s1, double& s2, bool& zero,
+                                          double& s0, double& s1, double& s2, bool& zero, bool& open,
                                           Late_Start* const late = nullptr)
 {
 	constexpr int NF = Flux_Rows<SOLVER>::N;
@@ -615,7 +662,7 @@ __device__ __forceinline__ void tile_step(const Step_Params& P, double* const sm
 		uint8_t* const bad = bad_base + slot * T::CELLS;
 		double cfz = 0.0;
 		if (stage) {
-			cfz = load_record<true, YACT, ZACT, CO>(P, rec, bad, T::CELLS, ri, col + k * P.L.plane, [&]() {
+			cfz = load_record<true, YACT, ZACT, CO>(P, rec, bad, T::CELLS, ri, col + k * P.L.plane, open, [&]() {
 				if (LATE and t == 0) find_dt(P, &late->dt, late->first, &late->stop);
 				// the plane after this one on its way to L2, a plane's time before its loads: they waited
 				// for DRAM a seventh of the warps' time (256^3 HLLD 1.46 -> 1.41 ms per step; copying it
@@ -628,7 +675,7 @@ __device__ __forceinline__ void tile_step(const Step_Params& P, double* const sm
 			});
 		}
 		if (k >= kb and k < ke and hri >= 0) {
-			load_record<true, YACT, false, CO>(P, rec, bad, T::CELLS, hri, hoff + k * P.L.plane, []() {});
+			load_record<true, YACT, false, CO>(P, rec, bad, T::CELLS, hri, hoff + k * P.L.plane, open, []() {});
 		}
 		return cfz;
 	};
@@ -801,10 +848,10 @@ __global__ void __launch_bounds__(TX * TY, Tile_Kind::resident_of(SOLVER, TY, ZA
 			continue;
 		}
 		double s0 = 0.0, s1 = 0.0, s2 = 0.0;
-		bool zero = false;
-		tile_step<SOLVER, TY, ZACT>(sp, smem, bar, dt, w.y % tiles_x, w.y / tiles_x, w.z, s0, s1, s2, zero);
+		bool zero = false, open = false;
+		tile_step<SOLVER, TY, ZACT>(sp, smem, bar, dt, w.y % tiles_x, w.y / tiles_x, w.z, s0, s1, s2, zero, open);
 		double smax[3] = {s0, s1, s2};
-		flush_speeds(sp, smax, zero);
+		if (flush_speeds(sp, smax, zero, open)) settle_tile(sp, w.y % tiles_x, w.y / tiles_x, w.z);
 	}
 }
 
@@ -855,8 +902,7 @@ __device__ __forceinline__ void boundary_face(const Step_Params& P, const int d,
 		UA[v] = CO ? __ldcg(P.in + v * P.L.var + oa) : P.in[v * P.L.var + oa];
 		UB[v] = CO ? __ldcg(P.in + v * P.L.var + ob) : P.in[v * P.L.var + ob];
 	}
-	const Derived da = derive<true, true, true>(UA[0], UA[1], UA[2], UA[3], UA[4], UA[5], UA[6], UA[7], P.gas);
-	const Derived db = derive<true, true, true>(UB[0], UB[1], UB[2], UB[3], UB[4], UB[5], UB[6], UB[7], P.gas);
+	const Derived da = derive_along(e, UA, P.gas), db = derive_along(e, UB, P.gas);
 	Side L, R;
 	auto fill = [e](Side& s, const double U[8], const Derived& dd) {
 		s.rho = U[0];
@@ -869,7 +915,7 @@ __device__ __forceinline__ void boundary_face(const Step_Params& P, const int d,
 		s.v0 = s.m0 * s.rinv; s.v1 = s.m1 * s.rinv; s.v2 = s.m2 * s.rinv;
 		s.p = dd.p;
 		s.pt = dd.pt;
-		s.cf = dd.cf[e];
+		s.cf = dd.cf[0];
 		s.bad = dd.bad;
 	};
 	fill(L, UA, da);
@@ -943,10 +989,11 @@ __global__ void __launch_bounds__(TX * TY, Tile_Kind::resident_of(SOLVER, TY, ZA
 		flush_speeds(P, smax, zero);
 		return;
 	}
-	tile_step<SOLVER, TY, ZACT, false, LATE>(P, smem, bar, dt, blockIdx.x, blockIdx.y, blockIdx.z, s0, s1, s2, zero, &start);
+	bool open = false;
+	tile_step<SOLVER, TY, ZACT, false, LATE>(P, smem, bar, dt, blockIdx.x, blockIdx.y, blockIdx.z, s0, s1, s2, zero, open, &start);
 	if (LATE and start.stop) return;
 	double smax[3] = {s0, s1, s2};
-	flush_speeds(P, smax, zero);
+	if (flush_speeds(P, smax, zero, open)) settle_tile(P, blockIdx.x, blockIdx.y, blockIdx.z);
 }
 
 // the ghost-ghost faces of every box of a batch, blockIdx.y the box
@@ -1131,7 +1178,7 @@ __global__ void __launch_bounds__(TX * TY, Tile_Kind::resident_of(SOLVER, TY, ZA
 		__syncthreads();
 		if (not s_go) return;
 		double smax[3] = {0.0, 0.0, 0.0};
-		bool zero = false;
+		bool zero = false, open = false;
 		if (w.w == 0) {
 			const bool first = w.y == 0 and w.z == 0;
 			const double dt = begin_step(sp, &s_dt, first, &s_stop);
@@ -1140,7 +1187,7 @@ __global__ void __launch_bounds__(TX * TY, Tile_Kind::resident_of(SOLVER, TY, ZA
 				tile_hold<true>(sp, w.y % tiles_x, w.y / tiles_x, w.z);
 			} else {
 				tile_step<SOLVER, TY, ZACT, true>(sp, smem, bar, dt, w.y % tiles_x, w.y / tiles_x, w.z, smax[0], smax[1],
-				                            smax[2], zero);
+				                            smax[2], zero, open);
 			}
 		} else if (not stopped_before(sp)) {
 			// ghost-ghost faces: combination w.y, faces [w.z BOUNDARY_CHUNK, (w.z + 1) BOUNDARY_CHUNK)
@@ -1155,7 +1202,10 @@ __global__ void __launch_bounds__(TX * TY, Tile_Kind::resident_of(SOLVER, TY, ZA
 				}
 			}
 		}
-		flush_speeds(sp, smax, zero);
+		if (flush_speeds(sp, smax, zero, open)) {
+			const int tiles_x = (sp.L.n[0] + sp.tw - 1) / sp.tw;
+			settle_tile(sp, w.y % tiles_x, w.y / tiles_x, w.z);
+		}
 		// publish the item's writes (every thread's), then count it done
 		__threadfence();
 		__syncthreads();
@@ -1248,6 +1298,13 @@ __global__ void __launch_bounds__(Line<SOLVER>::THREADS) line_run_kernel(const S
 		for (int v = 0; v < 8; v++) U[v] = P.in[v * P.L.var + off];
 	};
 
+	// a wave speed that round-off decides
+	const auto settle = [&](Derived& d, const double U[8]) {
+		if (d.bad == OPEN_WAVE) {
+			d.bad = reference_wave(U[0], U[1], U[2], U[3], U[4], U[5], U[6], U[7], P.gas) ? 0u : (uint32_t)PAMHD_FLAG_WAVE_SPEED;
+		}
+	};
+
 	double U[8] = {};
 	if (own) load(i, U);
 	// constant ghosts
@@ -1255,13 +1312,15 @@ __global__ void __launch_bounds__(Line<SOLVER>::THREADS) line_run_kernel(const S
 		double G[8];
 		if (rank == 0 and not P.periodic[0] and P.bc_lo[0] == PAMHD_BC_VALUE) {
 			load(-1, G);
-			const Derived d = derive<true, false, false, false>(G[0], G[1], G[2], G[3], G[4], G[5], G[6], G[7], P.gas);
+			Derived d = derive<true, false, false, true>(G[0], G[1], G[2], G[3], G[4], G[5], G[6], G[7], P.gas);
+			settle(d, G);
 			put(rank, 0, 0, G, d);
 			put(rank, 1, 0, G, d);
 		}
 		if (rank == blocks - 1 and not P.periodic[0] and P.bc_hi[0] == PAMHD_BC_VALUE) {
 			load(n, G);
-			const Derived d = derive<true, false, false, false>(G[0], G[1], G[2], G[3], G[4], G[5], G[6], G[7], P.gas);
+			Derived d = derive<true, false, false, true>(G[0], G[1], G[2], G[3], G[4], G[5], G[6], G[7], P.gas);
+			settle(d, G);
 			put(rank, 0, mine + 1, G, d);
 			put(rank, 1, mine + 1, G, d);
 		}
@@ -1278,7 +1337,8 @@ __global__ void __launch_bounds__(Line<SOLVER>::THREADS) line_run_kernel(const S
 	for (; s < nsteps; s++) {
 		const int b = s & 1;
 		if (own) {
-			const Derived d = derive<true, false, false, false>(U[0], U[1], U[2], U[3], U[4], U[5], U[6], U[7], P.gas);
+			Derived d = derive<true, false, false, true>(U[0], U[1], U[2], U[3], U[4], U[5], U[6], U[7], P.gas);
+			settle(d, U);
 			put(rank, b, t + 1, U, d);
 			if (t == 0) {
 				if (rank > 0) put(rank - 1, b, cells + 1, U, d);

@@ -272,10 +272,12 @@ __device__ __forceinline__ void plus_face(const Sub_Params& P, const long long c
 	#pragma unroll
 	for (int v = 0; v < 8; v++) Uu[v] = P.U[v * P.N + up];
 	const Derived du = derive<A == 0, A == 1, A == 2>(Uu[0], Uu[1], Uu[2], Uu[3], Uu[4], Uu[5], Uu[6], Uu[7], P.gas);
-	const Side L = side_of<A>(Uc, dc), R = side_of<A>(Uu, du);
+	// a refused fast speed, of this axis or another
+	const Derived dl = dc.bad == PAMHD_FLAG_WAVE_SPEED
+		? derive<A == 0, A == 1, A == 2>(Uc[0], Uc[1], Uc[2], Uc[3], Uc[4], Uc[5], Uc[6], Uc[7], P.gas) : dc;
+	const Side L = side_of<A>(Uc, dl), R = side_of<A>(Uu, du);
 	double G[8];
 	uint32_t flag = 0;
-	// HLLD in explicitly rounded arithmetic, as in the cell-centred step
 	const double s = solve_face<SOLVER>(L, R, P.gas, G, flag);
 	if (flag != 0) {
 		atomicOr(&P.status->flags, flag);

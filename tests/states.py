@@ -53,6 +53,22 @@ def states_at_rest(n, rng, mu0=4e-7 * np.pi, gamma=GAMMA_53):
     return s
 
 
+def equal_speed_states(n, rng, gamma=GAMMA_53, mu0=1.0):
+    """Random states whose sound and Alfven speeds are equal to a few units in the last place, the field
+    along the face normal or up to 1e-6 of it across."""
+    s = np.zeros((n, 8))
+    rho, p = rng.uniform(0.1, 3.0, n), rng.uniform(0.05, 2.0, n)
+    v = rng.normal(0.0, 0.5, (3, n))
+    b0 = np.sqrt(gamma * p * mu0) * (1 + 2.0 ** -52 * rng.integers(-4, 5, n))
+    across = np.where(rng.random(n) < 0.5, 0.0, 10.0 ** rng.uniform(-20, -6, n))
+    B = b0 * np.array([rng.choice([-1.0, 1.0], n), across, 0.5 * across])
+    s[:, 0] = rho
+    s[:, 1:4] = (v * rho).T
+    s[:, 4] = p / (gamma - 1) + 0.5 * rho * (v ** 2).sum(0) + 0.5 / mu0 * (B ** 2).sum(0)
+    s[:, 5:8] = B.T
+    return s
+
+
 def unit_density_gas(n, rng):
     """Random states of density 1 at rest without a field, and their sound speeds as IEEE arithmetic gives
     them from the state."""

@@ -117,3 +117,15 @@ def test_sound_speed_is_correctly_rounded(host):
     s, speed = states.unit_density_gas(5000, np.random.default_rng(9))
     for solver in ("rusanov", "hll_athena", "hlld_athena", "roe_athena"):
         assert np.array_equal(host(po.SOLVERS[solver], s, s)[1], speed), solver
+
+
+@pytest.mark.parametrize("mu0", [1.0, 4e-7 * np.pi])
+def test_equal_wave_speeds_are_refused_like_the_oracle(host, port, mu0):
+    """Cells whose sound and Alfven speeds are equal to rounding, the field along the face normal: the
+    reference's fast speed is the root of round-off, of either sign or zero, and it refuses the cell
+    unless that is positive.  The same flags as the oracle."""
+    s = states.equal_speed_states(5000, np.random.default_rng(10), mu0=mu0)
+    for solver in ("rusanov", "hll_athena", "hlld_athena", "roe_athena"):
+        go = port.face_flux(po.SOLVERS[solver], s, s, None, 5 / 3, mu0)[2]
+        assert (go == 0).sum() > 500 and (go != 0).sum() > 500
+        assert np.array_equal(host(po.SOLVERS[solver], s, s, mu0)[2], go), solver

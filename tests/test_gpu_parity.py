@@ -223,6 +223,61 @@ def test_hll_uniform_states_at_rest():
 
 
 @pytest.mark.parametrize("solver", list(po.SOLVERS))
+def test_equal_wave_speeds_are_refused_like_the_oracle(port, solver):
+    """Cells whose sound and Alfven speeds are equal to rounding, the field along the face normal, which
+    the reference takes or refuses by the sign of its round-off: the oracle's flags, face by face."""
+    s = states.equal_speed_states(5000, np.random.default_rng(10))
+    go = port.face_flux(po.SOLVERS[solver], s, s, None, 5 / 3, 1.0)[2]
+    assert np.array_equal(pg.face_flux(po.SOLVERS[solver], s, s, None, 5 / 3, 1.0)[2], go)
+
+
+@pytest.mark.parametrize("solver", list(po.SOLVERS))
+@pytest.mark.parametrize("n", [(9, 1, 1), (9, 6, 1), (7, 6, 5), (34, 9, 3)])
+def test_a_cell_of_equal_wave_speeds_is_refused_like_the_oracle(port, n, solver):
+    """One such cell in a grid at rest, at its corners, on its sides and inside, the field along each
+    axis, the sides periodic, COPY or (the cell a ghost state) VALUE: the step takes or refuses it as the
+    oracle, with its flag and at its face; in one step, in a run of two and in an ensemble."""
+    rng = np.random.default_rng(10)
+    cells = states.equal_speed_states(48, rng)
+    cells[:, 4] -= 0.5 * (cells[:, 1:4] ** 2).sum(1) / cells[:, 0]
+    cells[:, 1:4] = 0.0
+    refused = 0
+    for i, U in enumerate(cells):
+        axis = i % sum(m > 1 for m in n)
+        U[5:] = np.roll(U[5:], axis)
+        around = U.copy()
+        around[4] *= 1.1   # another sound speed
+        grid = np.tile(around.reshape(8, 1, 1, 1), (1,) + n[::-1])
+        value = i % 3 == 2
+        at = [(0, m // 2, m - 1)[rng.integers(3)] for m in n]
+        if not value:
+            grid[:, at[2], at[1], at[0]] = U
+        lo, hi, vlo, vhi = [0] * 3, [0] * 3, [None] * 3, [None] * 3
+        if i % 3 > 0:
+            lo = hi = [pg.BC_COPY if m > 1 else 0 for m in n]
+        if value:
+            lo = list(lo)
+            lo[axis], vlo[axis] = pg.BC_VALUE, U
+        gpu, ora = pair(port, n, po.SOLVERS[solver], (0.1, 0.1, 0.1), 5 / 3, 1.0, 0.4, lo, hi, vlo, vhi)
+        ora.set_state(grid)
+        _, flag, cell, direction = ora.step(0.0)
+        refused += flag != 0
+        batch = pg.Batch([gpu.cfg])
+        batch.set_state(0, grid)
+        for run in (lambda: gpu.step(0.0), lambda: (gpu.steps(2, 0.0), gpu.sync()),
+                    lambda: (batch.steps(1, 0.0), batch.sync()), lambda: (batch.run(1, 0.0), batch.sync())):
+            gpu.set_state(grid)
+            batch.set_state(0, grid)
+            if flag == 0:
+                run()
+                continue
+            with pytest.raises(pg.PhysicsError) as e:
+                run()
+            assert (e.value.flags, tuple(e.value.cell), e.value.direction) == (flag, tuple(cell), direction), i
+    assert 0 < refused < len(cells)
+
+
+@pytest.mark.parametrize("solver", list(po.SOLVERS))
 def test_sound_speed_is_correctly_rounded(solver):
     """The face speed between equal states at rest without a field: the sound speed, correctly rounded."""
     s, speed = states.unit_density_gas(5000, np.random.default_rng(9))
