@@ -69,6 +69,24 @@ def test_zero_exponents_are_the_plain_step():
     assert np.array_equal(out, a.get_state())
 
 
+def test_flat_grid_does_not_judge_the_inactive_axis(port):
+    """2-D cells whose sound and Alfven speeds are equal to rounding with the field along z, which has no
+    faces: the reference refuses such a cell at a z face only, so the step is taken, as the oracle's."""
+    s = states.equal_speed_states(64, np.random.default_rng(10))
+    refused = port.face_flux(po.HLLD, s, s, None, 5 / 3, 1.0)[2] != 0
+    assert 10 < refused.sum()
+    for U in s[refused][:10]:
+        for v in (1, 5):
+            U[v:v + 3] = np.roll(U[v:v + 3], 2)   # the frame of a face normal to z
+        grid = np.tile(U.reshape(8, 1, 1, 1), (1, 1, 4, 5))
+        gpu = pg.SubstepContext(pg.Config(n=(5, 4, 1), solver=pg.HLLD, cell_length=(0.1,) * 3, time_step_factor=0.4))
+        ora = port.substep_grid(po.make_cfg((5, 4, 1), po.HLLD, (0.1,) * 3, states.GAMMA_53, 1.0, 0.4))
+        for g in (gpu, ora):
+            g.set_state(grid)
+        assert ora.step(0.0)[3] == 0
+        gpu.step(0.0)
+
+
 def test_failure_is_reported():
     shape, n, L = (4, 4, 4), (4, 4, 4), (0.1, 0.1, 0.1)
     U = states.smooth_3d(shape, np.random.default_rng(4))
