@@ -1,6 +1,6 @@
 /*
-Host build of the face solvers (pamhd_b200/csrc/mhd_device.cuh) for the CPU
-tests: the same source the GPU kernels inline, compiled by g++ with the
+Host build of the face solvers (pamhd_b200/csrc/mhd_device.cuh) and of the
+step's tile shapes (grid_setup.cuh) for the CPU tests: the same source the GPU kernels inline, compiled by g++ with the
 device intrinsics it uses written out as the IEEE operations they are, and
 stand-ins for the two hardware estimates: 20 good bits, a subnormal operand
 taken for zero (the .ftz of the instructions).  Test infrastructure; not
@@ -11,10 +11,15 @@ part of the library.
 #include <cstdint>
 #include <cstring>
 
+#define __host__
 #define __device__
 #define __forceinline__ inline
 
 using std::max;
+
+// of the CUDA runtime, in declarations only
+typedef struct CUstream_st* cudaStream_t;
+struct int4;
 
 static inline double __fma_rn(const double a, const double b, const double c) { return std::fma(a, b, c); }
 static inline double __dmul_rn(const double a, const double b) { return a * b; }
@@ -55,7 +60,7 @@ static inline double rsqrt_estimate(const double x) { return short_of(1.0 / std:
 
 } // namespace pamhd_b200
 
-#include "../../pamhd_b200/csrc/mhd_device.cuh"
+#include "../../pamhd_b200/csrc/grid_setup.cuh"
 
 using namespace pamhd_b200;
 
@@ -103,4 +108,13 @@ extern "C" void host_rounded(const int64_t n, const double* a, const double* x, 
 		quotient[i] = quotient_rn(a[i], x[i], inverse[i]);
 		root[i] = sqrt_rn(x[i]);
 	}
+}
+
+// columns along x and y of the tiles of a step with 32 x rows threads and z faces, and its z planes per block
+extern "C" void host_tile_shape(const int32_t solver, const int32_t rows, const int32_t n[3], int32_t shape[3])
+{
+	const Tile_Kind kind{solver, rows, true};
+	tile_shape(kind, n[0], n[1], shape[0], shape[1]);
+	const long long tiles = (long long)((n[0] + shape[0] - 1) / shape[0]) * ((n[1] + shape[1] - 1) / shape[1]);
+	shape[2] = planes_per_block(tiles, n[2], kind.resident());
 }

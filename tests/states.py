@@ -53,6 +53,22 @@ def states_at_rest(n, rng, mu0=4e-7 * np.pi, gamma=GAMMA_53):
     return s
 
 
+# small 3-D grids and the tiles their steps take (columns along x and y, z planes per block; Rusanov, HLL
+# and HLLD): 32 x 8 columns one column short of, at and one past the grid's ends in x and y, with a last
+# block of one plane where the others take two, and other shapes, with threads that own no cell
+SHORT_GRIDS = {
+    (31, 40, 3): (32, 8, 1),
+    (64, 8, 19): (32, 8, 1),
+    (257, 145, 7): (32, 8, 2),
+    (33, 9, 2): (17, 9, 1),
+    (70, 17, 37): (24, 9, 2),
+    (100, 20, 5): (25, 10, 1),
+    (36, 36, 7): (18, 12, 1),
+    (17, 45, 6): (17, 15, 1),
+    (70, 50, 61): (24, 10, 7),
+}
+
+
 def equal_speed_states(n, rng, gamma=GAMMA_53, mu0=1.0):
     """Random states whose sound and Alfven speeds are equal to a few units in the last place, the field
     along the face normal or up to 1e-6 of it across."""

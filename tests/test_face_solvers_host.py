@@ -1,6 +1,6 @@
 """The face solvers of the GPU step (pamhd_b200/csrc/mhd_device.cuh), compiled for the host
 (tests/host/solvers_host.cpp), against the oracle's on states where rearranged arithmetic can go
-wrong (CPU only)."""
+wrong, and the tile shapes of the step (CPU only)."""
 import ctypes
 import os
 import subprocess
@@ -21,7 +21,8 @@ D = ctypes.POINTER(ctypes.c_double)
 def host():
     """face_flux(solver, neg, pos, mu0) -> flux, speed, flags of the host build; .lib, the build."""
     os.makedirs(os.path.dirname(LIB), exist_ok=True)
-    deps = [SRC, os.path.join(os.path.dirname(HERE), "pamhd_b200", "csrc", "mhd_device.cuh")]
+    csrc = os.path.join(os.path.dirname(HERE), "pamhd_b200", "csrc")
+    deps = [SRC] + [os.path.join(csrc, f) for f in ("mhd_device.cuh", "step.cuh", "grid_setup.cuh")]
     if not os.path.exists(LIB) or any(os.path.getmtime(d) > os.path.getmtime(LIB) for d in deps):
         subprocess.run(["g++", "-std=c++17", "-O2", "-ffp-contract=off", "-fPIC", "-shared", "-o", LIB, SRC],
                        check=True)
@@ -129,3 +130,12 @@ def test_equal_wave_speeds_are_refused_like_the_oracle(host, port, mu0):
         go = port.face_flux(po.SOLVERS[solver], s, s, None, 5 / 3, mu0)[2]
         assert (go == 0).sum() > 500 and (go != 0).sum() > 500
         assert np.array_equal(host(po.SOLVERS[solver], s, s, mu0)[2], go), solver
+
+
+def test_short_grids_have_the_tiles_they_are_named_for(host):
+    """The grids of the GPU test of short z chunks and shaped tiles take the tiles listed with them."""
+    I3 = ctypes.c_int32 * 3
+    for n, tiles in states.SHORT_GRIDS.items():
+        shape = I3()
+        host.lib.host_tile_shape(po.SOLVERS["hlld_athena"], 8, I3(*n), shape)
+        assert tuple(shape) == tiles, n

@@ -95,20 +95,16 @@ def test_line_run_stops_at_a_failure():
 
 
 @pytest.mark.parametrize("bc", ["periodic", "copy"])
-@pytest.mark.parametrize("n", [(33, 9, 2), (70, 17, 37), (31, 40, 3), (64, 8, 19), (100, 20, 5), (36, 36, 7),
-                               (17, 45, 6)])
-def test_short_z_chunks_match_oracle(port, n, bc):
-    """Small 3-D grids, whose blocks take a few planes each (the last chunk of 37 planes a single
-    one) and whose tiles end one cell short of, at and one cell past 32 columns and 8 rows, or have
-    other shapes (25 x 10, 18 x 12 and 17 x 15 columns on the last three), with threads that own no
-    cell; on open sides the step's own blocks solve the ghost-ghost faces.  Per step, the bar of this
-    file."""
+@pytest.mark.parametrize("solver", list(po.SOLVERS))
+@pytest.mark.parametrize("n", list(states.SHORT_GRIDS))
+def test_short_z_chunks_match_oracle(port, n, solver, bc):
+    """Small 3-D grids, whose blocks take a few planes each, in tiles of 32 x 8 and of other columns (the
+    sizes and what they are for: states.SHORT_GRIDS; Roe's tiles, of half as many threads, are others);
+    on open sides the step's own blocks solve the ghost-ghost faces.  Per step, the bar of this file."""
     kinds = ((pg.BC_COPY,) * 3 if bc == "copy" else (pg.BC_PERIODIC,) * 3,) * 2
     L = (0.1, 0.12, 0.09)
     U = states.smooth_3d((n[2], n[1], n[0]), np.random.default_rng(3))
-    gpu = pg.Context(pg.Config(n=n, solver=pg.HLLD, cell_length=L, time_step_factor=0.4, bc_lo=kinds[0],
-                               bc_hi=kinds[1]))
-    ora = port.grid(po.make_cfg(n, pg.HLLD, L, states.GAMMA_53, 1.0, 0.4, *kinds), threads=4)
+    gpu, ora = pair(port, n, po.SOLVERS[solver], L, states.GAMMA_53, 1.0, 0.4, *kinds)
     gpu.set_state(U)
     ora.set_state(U)
     for s in range(4):
