@@ -26,7 +26,9 @@ OBJ = os.path.join(PKG, "_build")
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 FLAGS = ["-O3", "-std=c++17", "-lineinfo", "-Xcompiler", "-fPIC", "-Xcompiler", "-O3",
          "-I", os.path.join(ROOT, "include")]
-# per-file flags: these steps round their updates as the CPU oracle does
+# per-file flags, no contraction: the two-population step has the CPU oracle's bits; the staggered and
+# local-time-stepping steps say themselves where they fuse (their updates' sums; the oracle's expressions
+# elsewhere round as they do there)
 FILE_FLAGS = {"staggered.cu": ["-fmad=false"], "npop.cu": ["-fmad=false"], "substep.cu": ["-fmad=false"]}
 
 

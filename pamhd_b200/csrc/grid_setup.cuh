@@ -158,9 +158,10 @@ step.  A block of kc planes takes about kc + 1 plane times (the planes
 before and after the chunk, and the block's start and end); 148 SMs run
 `resident` blocks each, and a wave with fewer blocks per SM is shorter,
 since the blocks of an SM share its FP64 pipe: two side by side take 1.6
-times as long as one alone.  Grids of many waves keep the 16 planes of
-before (256^3: 4096 blocks); smaller ones get shorter chunks that fill the
-SMs, e.g. 96 x 64 x 50 cells 240 blocks of 5 planes instead of 72 of 17.
+times as long as one alone.  Grids of many waves get long chunks, which
+repeat fewer planes (256^3: 2048 blocks of 32; 384^3: 576 of all 384),
+smaller ones short chunks that fill the SMs, e.g. 96 x 64 x 50 cells 240
+blocks of 5 planes instead of 72 of 17.
 */
 inline int planes_per_block(const long long tiles, const int nz, const int resident)
 {

@@ -752,9 +752,9 @@ each pair's strengths are a sum and a difference of two shared
 projections, and its contribution to the flux takes the sum and the
 difference of the pair's weights.  No 7 x 7 matrix is formed, and no
 product with one of its zeros computed; every root and quotient comes from
-the reciprocal steps above.  Bound by FP64 work (3026 flops per 2-D
-cell-update as dense matrices with IEEE roots and quotients): a 512^2 step
-went from 107 to 65 us.
+the reciprocal steps above.  Bound by FP64 work (1798 flops per 2-D
+cell-update, 3026 as dense matrices with IEEE roots and quotients): a 512^2
+step went from 107 to 65 us (67 with the almost aligned faces' alphas).
 
 alpha_f^2 = (a^2 - c_s^2) / (c_f^2 - c_s^2) and alpha_s^2 = (c_f^2 - a^2) /
 (c_f^2 - c_s^2), whose numerators cancel, are taken from the quadratic's

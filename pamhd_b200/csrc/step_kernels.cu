@@ -585,7 +585,7 @@ A grid without z faces (ZACT false) has one plane and nothing to overlap:
 one record slot and two block barriers.  There a block finds the step's dt
 late: thread 0 while its first loads are under way, the block behind its
 first barrier, instead of before the loads (512^2 HLLD 33.1 -> 32.0 us per
-step; the 3-D tiles, which start once per 16 planes, lost 1.6 % that way and
+step; the 3-D tiles, which start once per chunk of planes, lost 1.6 % that way and
 Roe's 4 % to registers).
 */
 template <int SOLVER, int TY, bool ZACT, bool CO = false, bool LATE = false>

@@ -1,7 +1,7 @@
 """Local time stepping on the GPU (pamhd_gpu_substep_*, through the C ABI) against the CPU oracle
 (oracle/substep.hpp): periods, substep counts and step lengths, and the state after every step
-within 1e-12 of each field's largest magnitude (the cell-centred bar: the face solves round
-differently, the updates follow the oracle's order)."""
+within 1e-12 of each field's largest magnitude (the cell-centred bar: the face solves and the
+updates, the oracle's terms in its order, round differently)."""
 import numpy as np
 import pytest
 
