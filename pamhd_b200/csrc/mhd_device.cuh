@@ -33,7 +33,6 @@ mhd/common.hpp:612).  Flux order: rho, mom x/y/z, E, B x/y/z.
 namespace pamhd_b200 {
 
 constexpr double DBL_EPS = 2.220446049250313080847e-16;  // numeric_limits<double>::epsilon()
-constexpr double DBL_MIN_NORMAL = 2.2250738585072013831e-308;
 
 /*
 Checks on the high word (sign, exponent, top of the mantissa): one or two
